@@ -201,6 +201,27 @@ size_t partial_bytes(const fa_fwd_params* p, int splits, size_t* lse_off) {
     return o_bytes + ((rows * sizeof(float) + 255) & ~static_cast<size_t>(255));
 }
 
+void fill_decode_args(const fa_fwd_params* p, const FwdArgs& a, DecodeArgs* d) {
+    std::memset(d, 0, sizeof(*d));
+    d->q = p->q; d->o = p->o; d->lse = p->lse;
+    d->alibi_slopes = p->alibi_slopes; d->status = p->status;
+    d->heads = p->heads; d->kv_group = a.kv_group; d->seqlen_q = p->seqlen_q; d->seqlen_k = p->seqlen_k;
+    d->head_dim = p->head_dim; d->tc = a.tc; d->tiles_per_split = a.tiles_per_split; d->scale_log2 = a.scale_log2;
+    d->is_causal = a.is_causal; d->window_left = a.window_left; d->window_right = a.window_right;
+    d->q_pos0 = a.q_pos0; d->k_pos0 = a.k_pos0; d->o_is_fp32 = a.o_is_fp32; d->drop = a.drop;
+}
+
+// Partial results per unit that a launch with num_splits = 0 keeps in the workspace (1 = none).
+int planned_parts(const fa_fwd_params* p, int splits, int sms) {
+    if (p->seqlen_q > 8 || p->accum_o != nullptr) return splits;
+    FwdArgs a;
+    DecodeArgs d;
+    fill_args(p, splits, &a);
+    fill_decode_args(p, a, &d);
+    plan_decode(&d, p->batch * p->heads, splits, false, sms);
+    return d.merge ? 1 : d.parts;
+}
+
 // head_dim that is not a multiple of 8: Q/K/V are copied to a pitch of d8 = ceil8(head_dim)
 // elements (zero columns), the kernels run on the padded problem, O is copied back.
 struct PadPlan {
@@ -270,17 +291,20 @@ int fa_fwd_resolve_splits(const fa_fwd_params* p) {
 }
 
 size_t fa_fwd_workspace_bytes(const fa_fwd_params* p) {
-    const int s = fa_fwd_resolve_splits(p);
+    int s = fa_fwd_resolve_splits(p);
     if (s < 1) return 0;
+    fa_fwd_params q = *p;
     size_t bytes = 0;
     if (p->head_dim % 8 != 0) {
-        fa_fwd_params q = *p;
+        bytes = pad_plan(p).total;
         q.head_dim = pad_plan(p).d8;
-        bytes = pad_plan(p).total + (s > 1 ? partial_bytes(&q, s, nullptr) : 0);
-    } else if (s > 1) {
-        bytes = partial_bytes(p, s, nullptr);
     }
-    return bytes;
+    if (p->num_splits == 0) {
+        int sms = 148, major = 10;
+        if (sm_count_of_current_device(&sms, &major) != FA_OK) return 0;
+        s = planned_parts(&q, s, sms);
+    }
+    return bytes + (s > 1 ? partial_bytes(&q, s, nullptr) : 0);
 }
 
 int fa_fwd(const fa_fwd_params* p) {
@@ -299,7 +323,8 @@ int fa_fwd(const fa_fwd_params* p) {
         const PadPlan pl = pad_plan(p);
         fa_fwd_params q = *p;
         q.head_dim = pl.d8;
-        const size_t part = splits > 1 ? partial_bytes(&q, splits, nullptr) : 0;
+        const int parts = p->num_splits == 0 ? planned_parts(&q, splits, sms) : splits;
+        const size_t part = parts > 1 ? partial_bytes(&q, parts, nullptr) : 0;
         if (!p->workspace || p->workspace_bytes < pl.total + part) return FA_ERR_WORKSPACE;
         if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return FA_ERR_INVALID_ARG;
         char* ws = static_cast<char*>(p->workspace);
@@ -311,7 +336,6 @@ int fa_fwd(const fa_fwd_params* p) {
             launch_repitch(p->v, vp, 2, rk, p->head_dim, pl.d8, stream) != cudaSuccess)
             return FA_ERR_CUDA;
         q.q = qp; q.k = kp; q.v = vp; q.o = op;
-        q.num_splits = splits;
         q.workspace = part ? op + pl.o_bytes : nullptr;
         q.workspace_bytes = part;
         rc = fa_fwd(&q);
@@ -322,47 +346,59 @@ int fa_fwd(const fa_fwd_params* p) {
     }
     FwdArgs a;
     fill_args(p, splits, &a);
-    if (splits > 1) {
+    const bool decode = p->seqlen_q <= 8 && p->accum_o == nullptr;
+    DecodeArgs d;
+    int parts = splits;  // partial results per unit
+    if (decode) {
+        fill_decode_args(p, a, &d);
+        plan_decode(&d, units, splits, p->num_splits > 0, sms);
+        parts = d.merge ? 1 : d.parts;
+    }
+    if (splits > 1 || parts > 1) {
         size_t lse_off = 0;
-        const size_t need = partial_bytes(p, splits, &lse_off);
-        if (!p->workspace || p->workspace_bytes < need) return FA_ERR_WORKSPACE;
-        if (reinterpret_cast<uintptr_t>(p->workspace) & 15u) return FA_ERR_INVALID_ARG;
-        a.o_partial = static_cast<float*>(p->workspace);
-        a.lse_partial = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + lse_off);
+        const size_t need = partial_bytes(p, parts, &lse_off);
+        // (a caller that names its split count provides the workspace of that count, whatever is made of it)
+        const size_t promised = p->num_splits > 0 ? partial_bytes(p, splits, nullptr) : need;
+        const bool missing = !p->workspace || p->workspace_bytes < std::max(need, promised);
+        if (missing && parts > 1 && splits == 1) {
+            // the split count was the library's to choose and the caller keeps no workspace
+            d.parts = 8;
+            d.merge = 1;
+            parts = 1;
+        } else if (missing && (parts > 1 || p->num_splits > 1)) {
+            return FA_ERR_WORKSPACE;
+        }
+        if (parts > 1) {
+            if (reinterpret_cast<uintptr_t>(p->workspace) & 15u) return FA_ERR_INVALID_ARG;
+            a.o_partial = d.o_partial = static_cast<float*>(p->workspace);
+            a.lse_partial = d.lse_partial = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + lse_off);
+        }
     }
     const bool bf16 = p->dtype == FA_DTYPE_BF16;
-    CUtensorMap tq, tk, tv;
-    if ((rc = make_tensor_map(&tq, bf16, p->q, p->head_dim, p->seqlen_q, units)) != FA_OK) return rc;
+    CUtensorMap tk, tv;
     const int units_k = p->batch * kv_heads(p);
     if ((rc = make_tensor_map(&tk, bf16, p->k, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
     if ((rc = make_tensor_map(&tv, bf16, p->v, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
-    // 16-bit output of an unsplit launch is written by TMA stores, one 32-row box per warp
-    CUtensorMap to = tq;
-    a.o_tma = (splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
-    if (a.o_tma && (rc = make_tensor_map(&to, bf16, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
-    if (p->seqlen_q <= 8 && p->accum_o == nullptr) {
+    if (decode) {
         // one to eight query rows per unit: the streaming kernel with keys on the tensor-memory lanes
-        DecodeArgs d;
-        std::memset(&d, 0, sizeof(d));
-        d.q = p->q; d.o = p->o; d.lse = p->lse;
-        d.o_partial = a.o_partial; d.lse_partial = a.lse_partial;
-        d.alibi_slopes = p->alibi_slopes; d.status = p->status;
-        d.heads = p->heads; d.kv_group = a.kv_group; d.seqlen_q = p->seqlen_q; d.seqlen_k = p->seqlen_k; d.head_dim = p->head_dim; d.tc = a.tc;
-        d.num_splits = splits; d.tiles_per_split = a.tiles_per_split; d.scale_log2 = a.scale_log2;
-        d.is_causal = a.is_causal; d.window_left = a.window_left; d.window_right = a.window_right;
-        d.q_pos0 = a.q_pos0; d.k_pos0 = a.k_pos0; d.o_is_fp32 = a.o_is_fp32; d.drop = a.drop;
         if (launch_decode(d, tk, tv, units, bf16, stream) != cudaSuccess) return FA_ERR_CUDA;
-    } else if (launch_fwd_tiled(a, tq, tk, tv, to, units, bf16, p->p_dropout > 0.0f, stream) != cudaSuccess) {
-        return FA_ERR_CUDA;
+    } else {
+        CUtensorMap tq;
+        if ((rc = make_tensor_map(&tq, bf16, p->q, p->head_dim, p->seqlen_q, units)) != FA_OK) return rc;
+        // 16-bit output of an unsplit launch is written by TMA stores, one 32-row box per warp
+        CUtensorMap to = tq;
+        a.o_tma = (splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
+        if (a.o_tma && (rc = make_tensor_map(&to, bf16, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
+        if (launch_fwd_tiled(a, tq, tk, tv, to, units, bf16, p->p_dropout > 0.0f, stream) != cudaSuccess) return FA_ERR_CUDA;
     }
-    if (splits > 1) {
+    if (parts > 1) {
         CombineArgs c;
         c.o_partial = a.o_partial;
         c.lse_partial = a.lse_partial;
         c.o = p->o;
         c.lse = p->lse;
         c.rows_per_unit = p->seqlen_q;
-        c.num_splits = splits;
+        c.num_splits = parts;
         c.head_dim = p->head_dim;
         c.o_dtype = p->o_dtype;
         if (launch_combine(c, units, stream) != cudaSuccess) return FA_ERR_CUDA;
@@ -517,6 +553,7 @@ int fa_fwd_host(const fa_fwd_params* p) {
     probe.heads_k = static_cast<int>(per_k);
     const int splits = fa_fwd_resolve_splits(&probe);
     if (splits < 1) return splits;
+    probe.num_splits = splits;  // one split count for all slices
     const size_t ws_bytes = fa_fwd_workspace_bytes(&probe);
     const size_t slot = align(q_unit * per) + 2 * align(kv_unit * per_k) + align(o_unit * per) + align(lse_unit * per) +
                         align(sizeof(float) * per) + align(ws_bytes) + align(sizeof(int));

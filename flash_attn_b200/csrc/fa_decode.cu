@@ -1,30 +1,39 @@
-// Split-KV decode for sm_100a: one query row per (batch, head) unit against a long
-// K/V.  Replaces the reference's forward_kernel_splitkv (src/flash_forward_splitkv.h:14-344)
-// for seqlen_q = 1, where the work is a pure stream of K and V through the SM: every byte
-// is used once, so the kernel is built around the TMA ring and nothing else may stall it.
+// Split-KV decode for sm_100a: one to eight query rows per (batch, head) unit against a long
+// K/V.  Replaces the reference's forward_kernel_splitkv (src/flash_forward_splitkv.h:14-344) and, where
+// the parts of a unit fit one cluster, its combine kernel (:347-399) for those shapes.  The work is a pure
+// stream of K and V through the SM: every byte is used once, so the kernel is built around the TMA ring and
+// nothing else may stall it.
 //
-// One CTA = one (unit, split).  The operands are swapped so that the 128 lanes of tensor
+// One CTA = one (unit, part of its keys).  The operands are swapped so that the 128 lanes of tensor
 // memory hold KEYS, not queries:
 //     S^T[128 keys x 16] = K_tile[128 x d] * Qpad^T[d x 16]      (tcgen05.mma, M=128, N=16)
 //     O^T[d x 16]       += V_tile^T[d x 128 keys] * P[128 keys x 16]
-// Column 0 of S^T / O^T belongs to the query; columns 1-15 are padding whose inputs (rows
-// 1-15 of the Q and P operand tiles) are never initialised and whose results are never
-// read -- an operand row only influences its own output column.  Thread r of the four
-// softmax warps owns key r of every tile, so masking, ALiBi, exp and dropout are spread over
-// 128 threads; one CTA-wide max per chunk of four tiles keeps them on a common scale.
-// The MMAs are tiny (N = 16): the tensor pipe is a convenient dot-product engine that
+// The first kH columns of S^T / O^T belong to queries; the others are padding whose inputs (rows of the Q
+// and P operand tiles) are never initialised and whose results are never read -- an operand row only
+// influences its own output column.  Thread r of the four softmax warps owns key r of every tile, so masking,
+// ALiBi, exp and dropout are spread over 128 threads; one CTA-wide max per chunk of tiles keeps them on a
+// common scale.  The MMAs are tiny (N = 16): the tensor pipe is a convenient dot-product engine that
 // reads K/V straight from the swizzled TMA tiles, and the kernel stays HBM-bound.
 //
-// Grouped-query attention and short query blocks (kH = 8): the query heads that share one K/V
-// head, and the seqlen_q <= 8 query rows of each, ride in columns 0..7 of the same MMAs (rows
-// 0..7 of the Q and P operand tiles; column = head * seqlen_q + row), so a CTA streams its K/V
-// split once for up to eight queries; every per-query quantity (position, masks, max, sum, ALiBi
-// slope, dropout stream, LSE) becomes an array over the columns.  Groups that need more than
-// eight columns are cut into sub-groups of whole heads, one CTA each.
+// Grouped-query attention and short query blocks: the query heads that share one K/V head, and the
+// seqlen_q <= 8 query rows of each, ride in the columns of the same MMAs (column = head * seqlen_q + row), so
+// a CTA streams its K/V once for up to sixteen queries.  Groups that need more columns are cut into
+// sub-groups of whole heads, one CTA each.  What bounds a CTA beside HBM is the softmax of a chunk (columns x
+// tiles per thread), hence kernels for 1, 4, 8 and 16 columns, no mask arithmetic on chunks that no mask
+// touches, warp maxima by redux, and the running maxima kept one column per lane: [16 x 32 query heads on 8
+// K/V heads, 4097 keys] 56.3 -> 44.6 us (6.0 TB/s), of which 6 us are start and drain; [8 x 32 on 8, 4 rows,
+// 8000 keys] 90 -> 47 us (16 columns instead of two CTAs per K/V head).
 //
-// Stream order of the TMA ring: K(0), K(1), V(0), K(2), V(1), ... (chunks of four tiles), so
+// The parts of a unit (plan_decode) are the CTAs of one cluster: each leaves its un-normalised O, max and sum
+// in its own shared memory, and the CTAs share out the columns and merge them through distributed shared
+// memory, so that no partial goes through HBM and no second kernel follows.
+//
+// Stream order of the TMA ring: K(0), K(1), V(0), K(2), V(1), ... (chunks of kChunk tiles), so
 // the scores of chunk c+1 are computed while the softmax of chunk c runs.
+#include <algorithm>
 #include <atomic>
+#include <cmath>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "fa_internal.h"
@@ -35,19 +44,37 @@ namespace fa {
 namespace {
 
 constexpr int kDThreads = 192;
-constexpr int kChunkTiles = 4;             // KV tiles per softmax chunk
-constexpr int kDStages = 3;                // ring slots of one K or V tile
-constexpr int kDTileBytes = kTile * 128 * 2;  // 32 KB: [128 keys x 128 columns], two 64-column boxes
-constexpr int kPTileBytes = 2048;          // P operand of one tile: two 1 KB atoms, row 0 = 64 keys each
-constexpr int kDSmemRing = 0;
-constexpr int kDSmemP = kDStages * kDTileBytes;                  // 8 KB + 2 KB that garbage rows may touch
-constexpr int kDSmemQ = kDSmemP + kChunkTiles * kPTileBytes + 2048;  // 2 KB + 2 KB slack
-constexpr int kDSmemBar = kDSmemQ + 4096;
-constexpr int kDNumBars = 2 * kDStages + 2 + 2 + 3;
-constexpr int kDSmemRed = kDSmemBar + 8 * kDNumBars;             // float[2][4][8] maxima + float[4][8] sums
-constexpr int kDSmemMisc = kDSmemRed + 384;
-constexpr int kDSmemBytes = kDSmemMisc + 16 + 1024;
-constexpr int kDTmemCols = 256;            // S^T: 2 buffers x 4 tiles x 16 columns; O^T: 16 columns at 128
+constexpr int kDTmemCols = 256;            // S^T: 2 buffers x up to 4 tiles x 16 columns; O^T: 16 columns at 128
+
+// kH = columns in use of the 16 (queries that share the CTA's K/V): 1, 4, 8 or 16.  The work of the softmax
+// warps goes with kH, so the smallest that holds the queries is taken.  D = 64 or 128 (head_dim rounded up).
+template <int kH, int D>
+struct DCfg {
+    // KV tiles per softmax chunk: with 16 columns two, which keeps P and the score registers at the size
+    // that two CTAs per SM allow
+    static constexpr int kChunk = kH == 16 ? 2 : 4;
+    static constexpr int kTileBytes = kTile * D * 2;  // one K or V tile: [128 keys x D], one or two 64-column boxes
+    static constexpr int kStages = D == 64 ? 6 : 3;   // 96 KB in flight either way
+    static constexpr int kNumBars = 2 * kStages + 2 + 2 + 3;
+    // K-major operand of 16 rows (Q, and P of one tile): 1 KB atoms of 8 rows x 64 elements.  Rows 8-15 are
+    // the next atom; with at most 8 columns in use they fall on the second half's atom and are never looked at.
+    static constexpr int kHalfBytes = kH == 16 ? 2048 : 1024;  // from the first 64 elements to the second
+    static constexpr int kOperandBytes = 2 * kHalfBytes;
+    static constexpr int kSmemRing = 0;
+    static constexpr int kSmemP = kStages * kTileBytes;
+    static constexpr int kSmemQ = kSmemP + kChunk * kOperandBytes + (kH == 16 ? 0 : 1024);  // (+ what rows 8-15 touch)
+    static constexpr int kSmemBar = kSmemQ + kOperandBytes + (kH == 16 ? 0 : 1024);
+    static constexpr int kSmemRed = (kSmemBar + 8 * kNumBars + 15) / 16 * 16;  // float[2][4][kH] maxima, float[4][kH] sums
+    static constexpr int kSmemMisc = kSmemRed + 3 * 4 * kH * 4;
+    static constexpr int kSmemEnd = kSmemMisc + 16;
+    // V^T is always an M = 128 operand; with D = 64 its upper 64 rows read the 16 KB behind the tile (the next
+    // slot, or what follows the ring) and only reach accumulator lanes that nobody reads
+    static constexpr int kSmemReach = kSmemP + (D == 64 ? kTile * 128 : 0);
+    static constexpr int kSmemBytes = (kSmemEnd > kSmemReach ? kSmemEnd : kSmemReach) + 1024;  // + alignment slack
+    static_assert(kSmemBytes <= 115712, "two CTAs per SM");
+};
+
+constexpr int kMaxCluster = 16;            // parts of a unit that one cluster merges (above 8: non-portable cluster size)
 
 constexpr float kDLog2e = 1.4426950408889634f;
 constexpr float kDLn2 = 0.6931471805599453f;
@@ -81,32 +108,63 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-// kH columns of one TMEM lane (kH = 1 or 8)
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+// kH columns of one TMEM lane
 template <int kH>
 __device__ __forceinline__ void tmem_ld_heads(uint32_t taddr, uint32_t (&r)[kH]) {
     if constexpr (kH == 1) r[0] = tmem_ld1(taddr);
-    else tmem_ld8(taddr, r);
+    else if constexpr (kH == 4) tmem_ld4(taddr, r);
+    else if constexpr (kH == 8) tmem_ld8(taddr, r);
+    else tmem_ld16(taddr, r);
 }
 template <int kH>
 __device__ __forceinline__ void tmem_st_heads(uint32_t taddr, const uint32_t (&r)[kH]) {
     if constexpr (kH == 1) tmem_st1(taddr, r[0]);
-    else tmem_st8(taddr, r);
+    else if constexpr (kH == 4) tmem_st4(taddr, r);
+    else if constexpr (kH == 8) tmem_st8(taddr, r);
+    else tmem_st16(taddr, r);
+}
+// Maximum over the lanes of a warp.
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 __device__ __forceinline__ bool mbar_wait_warp_ok(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
 }
 __device__ __forceinline__ void named_barrier_128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-template <bool kBf16, int kH>
+// One element of a finished output row, and (thread 0) its log-sum-exp.
+template <bool kBf16>
+__device__ __forceinline__ void store_result(const DecodeArgs& a, long long row, int col, float o_val, float lse_val) {
+    if (col < a.head_dim) {
+        if (a.o_is_fp32) static_cast<float*>(a.o)[row * a.head_dim + col] = o_val;
+        else if (kBf16) static_cast<__nv_bfloat16*>(a.o)[row * a.head_dim + col] = __float2bfloat16_rn(o_val);
+        else static_cast<__half*>(a.o)[row * a.head_dim + col] = __float2half_rn(o_val);
+    }
+    if (col == 0 && a.lse != nullptr) a.lse[row] = lse_val;
+}
+
+template <bool kBf16, int kH, int D, bool kDropout>
 __global__ void __launch_bounds__(kDThreads, 2)
 decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const DecodeArgs a) {
+    using C = DCfg<kH, D>;
+    constexpr int kChunkTiles = C::kChunk, kDStages = C::kStages, kDTileBytes = C::kTileBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t sRing = smem_base + kDSmemRing;
-    const uint32_t sP = smem_base + kDSmemP;
-    const uint32_t sQ = smem_base + kDSmemQ;
-    const uint32_t bar0 = smem_base + kDSmemBar;
+    const uint32_t sRing = smem_base + C::kSmemRing;
+    const uint32_t sP = smem_base + C::kSmemP;
+    const uint32_t sQ = smem_base + C::kSmemQ;
+    const uint32_t bar0 = smem_base + C::kSmemBar;
     const uint32_t bar_full = bar0;                          // [kDStages]
     const uint32_t bar_empty = bar_full + 8 * kDStages;      // [kDStages]
     const uint32_t bar_s_full = bar_empty + 8 * kDStages;    // [2]
@@ -114,54 +172,19 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
     const uint32_t bar_p_full = bar_s_free + 16;
     const uint32_t bar_p_free = bar_p_full + 8;
     const uint32_t bar_o_done = bar_p_free + 8;
-    float* red = reinterpret_cast<float*>(smem_gen + kDSmemRed);
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kDSmemMisc);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + kDSmemMisc + 4);
+    float* red = reinterpret_cast<float*>(smem_gen + C::kSmemRed);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kSmemMisc);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + C::kSmemMisc + 4);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    // the combine kernel behind a split launch may take its place on the SMs as they free up
-    // (it waits for this grid's completion before reading the partials)
+    // the kernel behind this one in the stream may take its place on the SMs as they free up
+    // (it waits for this grid's completion before it touches memory)
     grid_dep_launch_dependents();
-    // kH = 1: one CTA per (query unit, split).  kH = 8: one CTA per (K/V unit, sub-group of up to
-    // eight of its query heads, split); `unit` is then the first query unit of the sub-group.
-    const int cta_unit = blockIdx.x / a.num_splits;
-    const int split = blockIdx.x - cta_unit * a.num_splits;
-    int unit, kv_unit, gh = 1;
-    const int sq = (kH == 1) ? 1 : a.seqlen_q;  // query rows per head (columns per head)
-    if constexpr (kH == 1) {
-        unit = cta_unit;
-        kv_unit = a.kv_group > 1 ? unit / a.kv_group : unit;
-    } else {
-        const int heads_per_cta = kH / sq;
-        kv_unit = cta_unit / a.subgroups;
-        const int sub = cta_unit - kv_unit * a.subgroups;
-        unit = kv_unit * a.kv_group + sub * heads_per_cta;
-        gh = min(heads_per_cta, a.kv_group - sub * heads_per_cta);  // query heads of this CTA
-    }
-    const int nc = gh * sq;  // columns in use: column n = head n / sq, query row n % sq
-
-    // KV tiles of this split, clipped by the masks at tile granularity (as kv_tile_range
-    // of the tiled kernel, for the query rows at positions q_pos0 .. q_pos0 + sq - 1)
-    int lo = a.tiles_per_split * split, hi = min(lo + a.tiles_per_split, a.tc);
-    if (a.window_left >= 0) {
-        const long long w = (a.q_pos0 - a.window_left - a.k_pos0) / kTile;
-        lo = max(lo, static_cast<int>(max(0LL, min(w, static_cast<long long>(a.tc)))));
-    }
-    if (a.window_right >= 0) {
-        const long long last = a.q_pos0 + (sq - 1) + a.window_right - a.k_pos0;
-        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
-    }
-    if (a.is_causal) {
-        const long long last = a.q_pos0 + (sq - 1) - a.k_pos0;
-        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
-    }
-    const int n_tiles = hi > lo ? hi - lo : 0;
-    const int n_chunks = (n_tiles + kChunkTiles - 1) / kChunkTiles;
-    auto chunk_tiles = [&](int c) { return min(kChunkTiles, n_tiles - c * kChunkTiles); };
-
-    if (threadIdx.x == 0) {
+    if (warp == 4 && lane == 0) {
         *abort_flag = 0;
+        tma_prefetch_desc(&tmap_k);
+        tma_prefetch_desc(&tmap_v);
         for (int s = 0; s < kDStages; ++s) {
             mbar_init(bar_full + 8 * s, 1);
             mbar_init(bar_empty + 8 * s, 1);
@@ -175,24 +198,68 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         mbar_init(bar_o_done, 1);
         mbar_fence_init();
     }
+    // kH = 1: one CTA per (query unit, part of its keys).  kH = 8: one CTA per (K/V unit, sub-group of up
+    // to eight of its query heads, part); `unit` is then the first query unit of the sub-group.
+    const int cta_unit = static_cast<int>(fast_div(a.div_parts, blockIdx.x));
+    const int part = static_cast<int>(blockIdx.x) - cta_unit * a.parts;
+    int unit, kv_unit, gh = 1;
+    const int sq = (kH == 1) ? 1 : a.seqlen_q;  // query rows per head (columns per head)
+    if constexpr (kH == 1) {
+        unit = kv_unit = cta_unit;
+    } else {
+        const int heads_per_cta = kH / sq;
+        kv_unit = static_cast<int>(fast_div(a.div_subgroups, static_cast<uint32_t>(cta_unit)));
+        const int sub = cta_unit - kv_unit * a.subgroups;
+        unit = kv_unit * a.kv_group + sub * heads_per_cta;
+        gh = min(heads_per_cta, a.kv_group - sub * heads_per_cta);  // query heads of this CTA
+    }
+    const int nc = gh * sq;  // columns in use: column n = head n / sq, query row n % sq
+
+    // KV tiles of this part.  With dropout the parts are the caller's splits, whose tile ranges are part of
+    // the dropout streams' geometry; otherwise the visible tiles are dealt out evenly.
+    int lo, hi;
+    if (a.by_split) {
+        lo = max(a.tiles_per_split * part, a.vis_lo);
+        hi = min(min(a.tiles_per_split * (part + 1), a.tc), a.vis_hi);
+    } else {
+        const int n = a.vis_hi - a.vis_lo;
+        lo = a.vis_lo + static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(n * part)));
+        hi = a.vis_lo + static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(n * (part + 1))));
+    }
+    const int n_tiles = hi > lo ? hi - lo : 0;
+    const int n_chunks = (n_tiles + kChunkTiles - 1) / kChunkTiles;
+    auto chunk_tiles = [&](int c) { return min(kChunkTiles, n_tiles - c * kChunkTiles); };
+    int pushed = 0;  // tiles whose loads have been issued (producer lane only)
+
     if (warp == 5 && n_tiles > 0) {
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kDTmemCols);
         tmem_relinquish();
     }
-    if (threadIdx.x < 16 * kH && n_tiles > 0) {
-        // query n (head n / sq, row n % sq: consecutive rows of Q) goes to row n of the two Q atoms
-        // (16-byte unit u -> atom u/8, unit (u%8) ^ n: the 128-byte swizzle of row n)
-        const int u = threadIdx.x & 15, n = threadIdx.x >> 4;
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (n < nc && u * 8 < a.head_dim)
-            val = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) +
-                                                  (static_cast<long long>(unit) * sq + n) * a.head_dim + u * 8);
-        *reinterpret_cast<uint4*>(smem_gen + kDSmemQ + (u >> 3) * 1024 + n * 128 + (((u & 7) ^ n) << 4)) = val;
-        fence_proxy_async_smem();
-    }
+    grid_dep_wait();  // every thread, before its first global access
     if (warp == 4 && lane == 0) {
-        tma_prefetch_desc(&tmap_k);
-        tma_prefetch_desc(&tmap_v);
+        // the first K tiles are put in flight before the CTA-wide sync: their latency overlaps Q's
+        const int first = min(min(kDStages, kChunkTiles), n_tiles);
+        for (; pushed < first; ++pushed) {
+            mbar_expect_tx(bar_full + 8 * pushed, kDTileBytes);
+#pragma unroll
+            for (int b = 0; b < D / 64; ++b)
+                tma_load_3d(sRing + pushed * kDTileBytes + b * (kTile * 128), &tmap_k, bar_full + 8 * pushed, b * 64,
+                            (lo + pushed) * kTile, kv_unit);
+        }
+    }
+    if (n_tiles > 0) {
+        // query n (head n / sq, row n % sq: consecutive rows of Q) goes to row n of the Q operand
+        // (16-byte unit u -> half u/8, unit (u%8) ^ (n%8) of row n: the 128-byte swizzle)
+        constexpr int kUnits = D / 8;
+        for (int i = threadIdx.x; i < kUnits * kH; i += kDThreads) {
+            const int u = i % kUnits, n = i / kUnits;
+            uint4 val = make_uint4(0u, 0u, 0u, 0u);
+            if (n < nc && u * 8 < a.head_dim)
+                val = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) +
+                                                      (static_cast<long long>(unit) * sq + n) * a.head_dim + u * 8);
+            *reinterpret_cast<uint4*>(smem_gen + C::kSmemQ + (u >> 3) * C::kHalfBytes + n * 128 + (((u & 7) ^ (n & 7)) << 4)) = val;
+        }
+        fence_proxy_async_smem();
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -205,14 +272,16 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
     if (n_tiles > 0 && warp == 4) {
         // ======================= TMA producer ===================================
         if (lane == 0) {
-            int slot = 0;  // running count of tiles pushed into the ring
+            int slot = 0;  // running count of tiles in stream order
             auto push = [&](const CUtensorMap* map, int tile) -> bool {
+                if (slot < pushed) { ++slot; return true; }  // issued during set-up
                 const int st = slot % kDStages;
                 const uint32_t ph = (slot / kDStages) & 1;
                 if (!mbar_wait(bar_empty + 8 * st, ph ^ 1, abort_flag)) return false;
                 mbar_expect_tx(bar_full + 8 * st, kDTileBytes);
-                tma_load_3d(sRing + st * kDTileBytes, map, bar_full + 8 * st, 0, tile * kTile, kv_unit);
-                tma_load_3d(sRing + st * kDTileBytes + kTile * 128, map, bar_full + 8 * st, 64, tile * kTile, kv_unit);
+#pragma unroll
+                for (int b = 0; b < D / 64; ++b)
+                    tma_load_3d(sRing + st * kDTileBytes + b * (kTile * 128), map, bar_full + 8 * st, b * 64, tile * kTile, kv_unit);
                 ++slot;
                 return true;
             };
@@ -244,9 +313,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                     tc_fence_after_sync();
                     const uint32_t kt = sRing + st * kDTileBytes;
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
+                    for (int ks = 0; ks < D / 16; ++ks) {
                         const uint32_t off = (ks / 4) * (kTile * 128) + (ks % 4) * 32;
-                        const uint32_t qoff = (ks / 4) * 1024 + (ks % 4) * 32;
+                        const uint32_t qoff = (ks / 4) * C::kHalfBytes + (ks % 4) * 32;
                         umma_ss(tmem_base + buf * 64 + t * 16, make_smem_desc(kt + off, 0, 1024),
                                 make_smem_desc(sQ + qoff, 0, 1024), idesc_qk, ks > 0 ? 1u : 0u);
                     }
@@ -267,7 +336,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks) {
                         // A = V^T: 16 keys (2048 bytes) per step, the two 64-column halves 16 KB apart
-                        const uint32_t poff = t * kPTileBytes + (ks / 4) * 1024 + (ks % 4) * 32;
+                        const uint32_t poff = t * C::kOperandBytes + (ks / 4) * C::kHalfBytes + (ks % 4) * 32;
                         umma_ss(tmem_o, make_smem_desc(vt + ks * 2048, kTile * 128, 1024),
                                 make_smem_desc(sP + poff, 0, 1024), idesc_pv, (c > 0 || t > 0 || ks > 0) ? 1u : 0u);
                     }
@@ -289,74 +358,80 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         // ======================= softmax over keys / epilogue ===================
         const int r = threadIdx.x;  // key inside a tile; output column in the epilogue
         const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-        const float scale2 = a.scale_log2;
-        float slope2[kH];
-        int qrow[kH];  // each column's query row; its global position is q_pos0 + qrow
+        // scores stay unscaled and the scale is folded into the exponent's FMA, except with ALiBi
+        const bool alibi = a.alibi_slopes != nullptr;
+        const float scale2 = a.scale_log2, exp_scale = alibi ? 1.0f : a.scale_log2;
+        float m_ref = -INFINITY;  // CTA-wide running max of column `lane` (lanes < kH of every warp), log2 units
+        float l_part[kH];         // this thread's share of each column's row sum
 #pragma unroll
-        for (int n = 0; n < kH; ++n) {
-            slope2[n] = (a.alibi_slopes != nullptr && n < nc) ? a.alibi_slopes[(unit + n / sq) % a.heads] * kDLog2e : 0.0f;
-            qrow[n] = (kH == 1) ? 0 : n % sq;
-        }
-        const bool dropout = a.drop.threshold != 0ull;
-        float m_ref[kH];   // CTA-wide running max per head, log2 units
-        float l_part[kH];  // this thread's share of each head's row sum
-#pragma unroll
-        for (int n = 0; n < kH; ++n) {
-            m_ref[n] = -INFINITY;
-            l_part[n] = 0.0f;
-        }
+        for (int n = 0; n < kH; ++n) l_part[n] = 0.0f;
+        // this key's element of column n in the P operand: row n, 128-byte swizzled
+        uint8_t* p_half = smem_gen + C::kSmemP + (r >> 6) * C::kHalfBytes + (r & 7) * 2;
+        const uint32_t p_unit = static_cast<uint32_t>((r & 63) >> 3);
 
         for (int c = 0; c < n_chunks; ++c) {
             const int buf = c & 1;
             const int nt = chunk_tiles(c);
+            const int tile0 = lo + c * kChunkTiles;
             bool ok = mbar_wait_warp_ok(bar_s_full + 8 * buf, (c >> 1) & 1, abort_flag);
             if (!ok) fail = 3;
             tc_fence_after_sync();
-            float v[kChunkTiles][kH];
+            uint32_t raw[kChunkTiles][kH];
 #pragma unroll
             for (int t = 0; t < kChunkTiles; ++t) {
-                uint32_t raw[kH];
+                if (t < nt) {
+                    tmem_ld_heads<kH>(tmem_base + lane_base + buf * 64 + t * 16, raw[t]);
+                } else {
 #pragma unroll
-                for (int n = 0; n < kH; ++n) raw[n] = 0u;
-                if (t < nt) tmem_ld_heads<kH>(tmem_base + lane_base + buf * 64 + t * 16, raw);
-#pragma unroll
-                for (int n = 0; n < kH; ++n) v[t][n] = __uint_as_float(raw[n]);
+                    for (int n = 0; n < kH; ++n) raw[t][n] = 0xff800000u;  // -inf
+                }
             }
             tmem_wait_ld();
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_s_free + 8 * buf);
-
-            float m_thr[kH];
-#pragma unroll
-            for (int n = 0; n < kH; ++n) m_thr[n] = -INFINITY;
+            float v[kChunkTiles][kH];
 #pragma unroll
             for (int t = 0; t < kChunkTiles; ++t) {
-                const int tile = lo + c * kChunkTiles + t;
-                const long long key = static_cast<long long>(tile) * kTile + r;
-                const long long kpos = a.k_pos0 + key;
-                const bool in_range = t < nt && key < a.seqlen_k;
-                // key position relative to query row 0, saturated far outside any window
-                const long long rel64 = kpos - a.q_pos0;
-                const int rel = static_cast<int>(max(-0x40000000LL, min(rel64, 0x40000000LL)));
 #pragma unroll
-                for (int n = 0; n < kH; ++n) {
-                    const int ahead = rel - qrow[n];  // > 0: the key lies after the query
-                    bool keep = in_range;
-                    if (a.is_causal && ahead > 0) keep = false;
-                    if (a.window_left >= 0 && -ahead > a.window_left) keep = false;
-                    if (a.window_right >= 0 && ahead > a.window_right) keep = false;
-                    float sc = v[t][n] * scale2;
-                    if (slope2[n] != 0.0f) sc = fmaf(-slope2[n], fabsf(static_cast<float>(ahead)), sc);
-                    v[t][n] = keep ? sc : -INFINITY;
-                    m_thr[n] = fmaxf(m_thr[n], v[t][n]);
+                for (int n = 0; n < kH; ++n) v[t][n] = __uint_as_float(raw[t][n]);
+            }
+            // masks and ALiBi, on the chunks that have any (the tiles [full_lo, full_hi) are visible whole)
+            if (alibi || tile0 < a.full_lo || tile0 + nt > a.full_hi) {
+#pragma unroll
+                for (int t = 0; t < kChunkTiles; ++t) {
+                    const long long key = static_cast<long long>(tile0 + t) * kTile + r;
+                    const bool in_range = t < nt && key < a.seqlen_k;
+                    // key position relative to query row 0, saturated far outside any window
+                    const int rel = static_cast<int>(max(-0x40000000LL, min(a.k_pos0 + key - a.q_pos0, 0x40000000LL)));
+#pragma unroll
+                    for (int n = 0; n < kH; ++n) {
+                        const int ahead = rel - ((kH == 1) ? 0 : n % sq);  // > 0: the key lies after the query
+                        bool keep = in_range;
+                        if (a.is_causal && ahead > 0) keep = false;
+                        if (a.window_left >= 0 && -ahead > a.window_left) keep = false;
+                        if (a.window_right >= 0 && ahead > a.window_right) keep = false;
+                        if (alibi && n < nc)
+                            v[t][n] = fmaf(-(a.alibi_slopes[(unit + n / sq) % a.heads] * kDLog2e),
+                                           fabsf(static_cast<float>(ahead)), v[t][n] * scale2);
+                        if (!keep) v[t][n] = -INFINITY;
+                    }
                 }
             }
+            float* red_c = red + buf * 4 * kH;
+            {
+                float m_w[kH];
 #pragma unroll
-            for (int n = 0; n < kH; ++n) {
+                for (int n = 0; n < kH; ++n) {
+                    float m = v[0][n];
 #pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) m_thr[n] = fmaxf(m_thr[n], __shfl_xor_sync(0xffffffffu, m_thr[n], o));
-                if (lane == 0) red[(buf * 4 + warp) * 8 + n] = m_thr[n];
+                    for (int t = 1; t < kChunkTiles; ++t) m = fmaxf(m, v[t][n]);
+                    m_w[n] = warp_max(m);
+                }
+                if (lane == 0) {
+#pragma unroll
+                    for (int n = 0; n < kH; ++n) red_c[warp * kH + n] = m_w[n];
+                }
             }
             named_barrier_128();
 
@@ -365,63 +440,69 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 if (!mbar_wait_warp_ok(bar_p_free, (c - 1) & 1, abort_flag)) fail = 4;
                 tc_fence_after_sync();
             }
-            float m_use[kH], factor[kH];
-            bool any_rescale = false;
-#pragma unroll
-            for (int n = 0; n < kH; ++n) {
-                const float m_chunk = fmaxf(fmaxf(red[(buf * 4) * 8 + n], red[(buf * 4 + 1) * 8 + n]),
-                                            fmaxf(red[(buf * 4 + 2) * 8 + n], red[(buf * 4 + 3) * 8 + n]));
-                float m_new = m_ref[n];
-                factor[n] = 1.0f;
-                if (m_chunk > m_ref[n] + 8.0f || m_ref[n] == -INFINITY) {
-                    m_new = fmaxf(m_ref[n], m_chunk);
-                    factor[n] = (m_ref[n] == -INFINITY) ? 0.0f : ex2f(m_ref[n] - m_new);
-                }
-                if (m_new != m_ref[n]) {
-                    any_rescale = true;
-                    l_part[n] *= factor[n];
-                }
-                m_ref[n] = m_new;
-                m_use[n] = (m_new == -INFINITY) ? 0.0f : m_new;
+            // lane n keeps column n's running max (lazily raised, as in the tiled kernel) and hands it round
+            float m_new = m_ref, factor = 1.0f;
+            if (lane < kH) {
+                const float m_chunk = fmaxf(fmaxf(red_c[lane], red_c[kH + lane]), fmaxf(red_c[2 * kH + lane], red_c[3 * kH + lane])) * exp_scale;
+                if (m_chunk > m_ref + 8.0f || m_ref == -INFINITY) m_new = fmaxf(m_ref, m_chunk);
+                if (m_new != m_ref) factor = (m_ref == -INFINITY) ? 0.0f : ex2f(m_ref - m_new);
             }
-            if (c > 0 && any_rescale) {  // CTA-uniform: every thread sees the same maxima
-                uint32_t ov[kH];
-                tmem_ld_heads<kH>(tmem_o + lane_base, ov);
-                tmem_wait_ld();
+            if (__any_sync(0xffffffffu, m_new != m_ref)) {  // CTA-uniform: every warp sees the same maxima
+                float f[kH];
 #pragma unroll
-                for (int n = 0; n < kH; ++n) ov[n] = __float_as_uint(__uint_as_float(ov[n]) * factor[n]);
-                tmem_st_heads<kH>(tmem_o + lane_base, ov);
-                tmem_wait_st();
+                for (int n = 0; n < kH; ++n) {
+                    f[n] = __shfl_sync(0xffffffffu, factor, n);
+                    l_part[n] *= f[n];
+                }
+                if (c > 0) {
+                    uint32_t ov[kH];
+                    tmem_ld_heads<kH>(tmem_o + lane_base, ov);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int n = 0; n < kH; ++n) ov[n] = __float_as_uint(__uint_as_float(ov[n]) * f[n]);
+                    tmem_st_heads<kH>(tmem_o + lane_base, ov);
+                    tmem_wait_st();
+                }
             }
+            m_ref = m_new;
+            const float neg_lane = (m_new == -INFINITY) ? 0.0f : -m_new;
 
 #pragma unroll
-            for (int t = 0; t < kChunkTiles; ++t) {
-                if (t < nt) {
+            for (int n = 0; n < kH; ++n) {
+                const float neg_m = __shfl_sync(0xffffffffu, neg_lane, n);
+                uint8_t* p_row = p_half + n * 128 + ((p_unit ^ (n & 7)) << 4);
 #pragma unroll
-                    for (int n = 0; n < kH; ++n) {
-                        const float p = ex2f(v[t][n] - m_use[n]);
-                        l_part[n] += p;
-                        bool kept = true;
-                        if (dropout && n < nc) {
-                            // reference draw order for query rows 0..7 (one 8-row group shares its draws):
-                            // draw 64*tile_index + 8*(col/16) + 2*((col%16)/8) + col%2
-                            const unsigned long long subseq =
-                                (a.drop.unit0 + unit + n / sq) * static_cast<unsigned long long>(a.num_splits) +
-                                static_cast<unsigned long long>(split);
-                            const unsigned long long first = continuation(a.drop, n_tiles) +
-                                                             64ull * static_cast<unsigned long long>(c * kChunkTiles + t) +
-                                                             8ull * (r >> 4);
-                            const uint32_t bits = philox_keep4(a.drop, subseq, first);
-                            kept = (bits >> (2 * ((r >> 3) & 1) + (r & 1))) & 1u;
+                for (int t = 0; t < kChunkTiles; t += 2) {
+                    float p[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        p[i] = ex2f(fmaf(v[t + i][n], exp_scale, neg_m));
+                        l_part[n] += p[i];
+                        if constexpr (kDropout) {
+                            if (n < nc && t + i < nt) {
+                                // reference draw order for query rows 0..7 (one 8-row group shares its draws):
+                                // draw 64*tile_index + 8*(col/16) + 2*((col%16)/8) + col%2
+                                const unsigned long long subseq =
+                                    (a.drop.unit0 + unit + n / sq) * static_cast<unsigned long long>(a.parts) +
+                                    static_cast<unsigned long long>(part);
+                                const unsigned long long first = continuation(a.drop, n_tiles) +
+                                                                 64ull * static_cast<unsigned long long>(c * kChunkTiles + t + i) +
+                                                                 8ull * (r >> 4);
+                                const uint32_t bits = philox_keep4(a.drop, subseq, first);
+                                if (!((bits >> (2 * ((r >> 3) & 1) + (r & 1))) & 1u)) p[i] = 0.0f;
+                            }
                         }
-                        const float pk = kept ? p : 0.0f;
-                        uint16_t h;
-                        if constexpr (kBf16) h = __bfloat16_as_ushort(__float2bfloat16_rn(pk));
-                        else h = __half_as_ushort(__float2half_rn(pk));
-                        // P operand row n (head n), 128-byte swizzled like the Q rows
-                        *reinterpret_cast<uint16_t*>(smem_gen + kDSmemP + t * kPTileBytes + (r >> 6) * 1024 + n * 128 +
-                                                     (((((r & 63) >> 3) ^ n) & 7) << 4) + (r & 7) * 2) = h;
                     }
+                    uint32_t h;  // the two tiles' elements, rounded together
+                    if constexpr (kBf16) {
+                        const __nv_bfloat162 x = __floats2bfloat162_rn(p[0], p[1]);
+                        h = *reinterpret_cast<const uint32_t*>(&x);
+                    } else {
+                        const __half2 x = __floats2half2_rn(p[0], p[1]);
+                        h = *reinterpret_cast<const uint32_t*>(&x);
+                    }
+                    if (t < nt) *reinterpret_cast<uint16_t*>(p_row + t * C::kOperandBytes) = static_cast<uint16_t>(h);
+                    if (t + 1 < nt) *reinterpret_cast<uint16_t*>(p_row + (t + 1) * C::kOperandBytes) = static_cast<uint16_t>(h >> 16);
                 }
             }
             fence_proxy_async_smem();
@@ -436,7 +517,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             float l_warp = l_part[n];
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) l_warp += __shfl_xor_sync(0xffffffffu, l_warp, o);
-            if (lane == 0) red[64 + warp * 8 + n] = l_warp;
+            if (lane == 0) red[8 * kH + warp * kH + n] = l_warp;
         }
         named_barrier_128();
         uint32_t o_raw[kH];
@@ -451,25 +532,37 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 fail = 5;
             }
         }
+        float m_col[kH];
 #pragma unroll
-        for (int n = 0; n < kH; ++n) {
-            if (n >= nc) continue;
-            const float l_sum = (red[64 + n] + red[64 + 8 + n]) + (red[64 + 16 + n] + red[64 + 24 + n]);
-            const float inv = l_sum > 0.0f ? a.drop.inv_keep / l_sum : 0.0f;
-            const float lse_val = l_sum > 0.0f ? m_ref[n] * kDLn2 + __logf(l_sum) : -INFINITY;
-            const float o_val = __uint_as_float(o_raw[n]) * inv;
-            // non-split: row (unit + head, query row) of O; split: the same row of this split's partial
-            const long long head_n = unit + n / sq;
-            const long long out_row = (a.num_splits > 1) ? (head_n * a.num_splits + split) * sq + n % sq : head_n * sq + n % sq;
-            if (r < a.head_dim) {
-                if (a.num_splits > 1) a.o_partial[out_row * a.head_dim + r] = o_val;
-                else if (a.o_is_fp32) static_cast<float*>(a.o)[out_row * a.head_dim + r] = o_val;
-                else if (kBf16) static_cast<__nv_bfloat16*>(a.o)[out_row * a.head_dim + r] = __float2bfloat16_rn(o_val);
-                else static_cast<__half*>(a.o)[out_row * a.head_dim + r] = __float2half_rn(o_val);
+        for (int n = 0; n < kH; ++n) m_col[n] = __shfl_sync(0xffffffffu, m_ref, n);
+        if (a.merge) {
+            // this part's un-normalised row of every column, its max and its sum, for the peers to read
+            // (the ring is free: the last P V has completed)
+            float* part_o = reinterpret_cast<float*>(smem_gen + C::kSmemRing);
+#pragma unroll
+            for (int n = 0; n < kH; ++n) {
+                part_o[n * kTile + r] = __uint_as_float(o_raw[n]);
+                if (r == 0) {
+                    const float l_sum = (red[8 * kH + n] + red[9 * kH + n]) + (red[10 * kH + n] + red[11 * kH + n]);
+                    part_o[kH * kTile + 2 * n] = m_col[n];
+                    part_o[kH * kTile + 2 * n + 1] = fail == 0 ? l_sum : 0.0f;
+                }
             }
-            if (r == 0) {
-                if (a.num_splits > 1) a.lse_partial[out_row] = lse_val;
-                else if (a.lse != nullptr) a.lse[out_row] = lse_val;
+        } else {
+#pragma unroll
+            for (int n = 0; n < kH; ++n) {
+                if (n >= nc) continue;
+                const float l_sum = (red[8 * kH + n] + red[9 * kH + n]) + (red[10 * kH + n] + red[11 * kH + n]);
+                const float inv = l_sum > 0.0f ? a.drop.inv_keep / l_sum : 0.0f;
+                const float lse_val = l_sum > 0.0f ? m_col[n] * kDLn2 + __logf(l_sum) : -INFINITY;
+                const float o_val = __uint_as_float(o_raw[n]) * inv;
+                if (a.parts > 1) {  // partial of this part, for the combine kernel
+                    const long long prow = ((unit + n / sq) * static_cast<long long>(a.parts) + part) * sq + n % sq;
+                    if (r < a.head_dim) a.o_partial[prow * a.head_dim + r] = o_val;
+                    if (r == 0) a.lse_partial[prow] = lse_val;
+                } else {
+                    store_result<kBf16>(a, (unit + n / sq) * static_cast<long long>(sq) + n % sq, r, o_val, lse_val);
+                }
             }
         }
     }
@@ -487,36 +580,164 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kDTmemCols);
     }
+    if (a.merge) {
+        // The parts of a unit are one cluster: each CTA reads its share of the columns from all of them
+        // through distributed shared memory and writes the finished rows.  O = sum_j 2^(m_j - m) O_j / l,
+        // l = sum_j 2^(m_j - m) l_j (src/flash_forward_splitkv.h:359-397).
+        __syncwarp();
+        cluster_sync();
+        if (warp < 4) {
+            const int r = threadIdx.x;
+            const uint32_t base = sRing;
+            for (int n = part; n < nc; n += a.parts) {
+                float m_j[kMaxCluster], l_j[kMaxCluster], o_j[kMaxCluster];
+#pragma unroll
+                for (int j = 0; j < kMaxCluster; ++j) {
+                    m_j[j] = -INFINITY;
+                    l_j[j] = o_j[j] = 0.0f;
+                    if (j < a.parts) {
+                        const uint32_t peer = cluster_map(base, j);
+                        m_j[j] = ld_cluster_f32(peer + (kH * kTile + 2 * n) * 4);
+                        l_j[j] = ld_cluster_f32(peer + (kH * kTile + 2 * n + 1) * 4);
+                        o_j[j] = ld_cluster_f32(peer + (n * kTile + r) * 4);
+                    }
+                }
+                float m = m_j[0];
+#pragma unroll
+                for (int j = 1; j < kMaxCluster; ++j) m = fmaxf(m, m_j[j]);
+                float l = 0.0f, o = 0.0f;
+                if (m != -INFINITY) {
+#pragma unroll
+                    for (int j = 0; j < kMaxCluster; ++j) {
+                        // (a part without visible keys has m_j = -inf and weight 0; its o_j is 0)
+                        const float w = ex2f(m_j[j] - m);
+                        l = fmaf(w, l_j[j], l);
+                        o = fmaf(w, o_j[j], o);
+                    }
+                }
+                const float inv = l > 0.0f ? a.drop.inv_keep / l : 0.0f;
+                store_result<kBf16>(a, (unit + n / sq) * static_cast<long long>(sq) + n % sq, r, o * inv,
+                                    l > 0.0f ? m * kDLn2 + __logf(l) : -INFINITY);
+            }
+            __syncwarp();
+        }
+        cluster_sync();  // the peers' shared memory stays until everyone has read it
+    }
 }
 
 }  // namespace
 
+void plan_decode(DecodeArgs* a, int units, int splits, bool forced, int sms) {
+    // key tiles visible to any query row: the tile-granular clip of the masks (src/flash_forward.h:39-48)
+    // for the query rows at positions q_pos0 .. q_pos0 + seqlen_q - 1
+    long long lo = 0, hi = a->tc;
+    auto tiles_to = [&](long long last) { return last < 0 ? 0LL : std::min<long long>(last / kTile + 1, a->tc); };
+    const long long last_q = a->q_pos0 + a->seqlen_q - 1 - a->k_pos0;
+    if (a->window_left >= 0)
+        lo = std::max(0LL, std::min<long long>((a->q_pos0 - a->window_left - a->k_pos0) / kTile, a->tc));
+    if (a->window_right >= 0) hi = std::min(hi, tiles_to(last_q + a->window_right));
+    if (a->is_causal) hi = std::min(hi, tiles_to(last_q));
+    a->vis_lo = static_cast<int>(lo);
+    a->vis_hi = static_cast<int>(std::max(lo, hi));
+    const int n = a->vis_hi - a->vis_lo;
+
+    // tiles that need no mask: inside seqlen_k and visible to every query row
+    long long flo = 0, fhi = a->seqlen_k / kTile;
+    const long long first_q = a->q_pos0 - a->k_pos0;
+    if (a->window_left >= 0) flo = std::max(0LL, (last_q - a->window_left + kTile - 1) / kTile);
+    if (a->window_right >= 0) fhi = std::min(fhi, std::max(0LL, (first_q + a->window_right + 1) / kTile));
+    if (a->is_causal) fhi = std::min(fhi, std::max(0LL, (first_q + 1) / kTile));
+    a->full_lo = static_cast<int>(std::min<long long>(flo, a->tc));
+    a->full_hi = static_cast<int>(fhi);
+
+    // query heads that share a K/V head are packed into one CTA, up to sixteen columns at a time
+    const int queries = a->kv_group * a->seqlen_q;
+    a->columns = queries == 1 ? 1 : queries <= 4 ? 4 : queries <= 8 ? 8 : 16;
+    const int heads_per_cta = a->columns / a->seqlen_q;  // whole heads whose query rows fit the columns
+    a->subgroups = (a->kv_group + heads_per_cta - 1) / heads_per_cta;
+    const long long cta_units = static_cast<long long>(units / a->kv_group) * a->subgroups;
+
+    if (a->drop.threshold != 0ull) {
+        a->parts = splits;
+        a->by_split = splits > 1;
+        a->merge = splits == 2 || splits == 4 || splits == 8 || splits == 16;
+        return;
+    }
+    // How many CTAs share a unit's keys: a model of the kernel's time, in us, fitted to sweeps over 8 to 1024 units
+    // x 1 to 256 tiles on B200.  Two CTAs fit an SM.  A K + V tile takes a CTA `full` when every SM has two (bound
+    // by HBM, 7.4 TB/s); with at most one CTA per SM it takes less as fewer SMs load at a time, down to `least`, the
+    // CTA's own chain of load, MMA, softmax, MMA.  A wave costs 3 us to start and drain, a merge in the cluster 1.2
+    // (16-CTA clusters are slow to place when they do not all fit at once), partials through memory and the combine
+    // kernel 8.  Measured, one CTA per unit against the choice: 8 K/V heads x 1000 keys 10.4 -> 6.3 us, x 32768 keys
+    // 226 -> 25; 128 units x 4097 keys 44.9 -> 44.6 (HBM-bound either way); 64 units x 8000 keys, 16 queries 77 -> 47.
+    a->by_split = 0;
+    const bool narrow = a->head_dim <= 64;
+    const double full = narrow ? 1.3 : 2.3, least = a->columns == 16 ? 1.15 : narrow ? 0.85 : 0.95;
+    int best = 1;
+    double best_t = 1e30;
+    for (int parts = 1; parts <= 64 && (parts == 1 || parts <= n); parts *= 2) {
+        if (parts > kMaxCluster && forced && parts > splits) break;  // (the caller's workspace holds `splits` partials)
+        const double ctas = static_cast<double>(cta_units) * parts, waves = std::floor(ctas / (2.0 * sms));
+        const double rest = ctas - waves * 2.0 * sms, even = static_cast<double>(n) / parts;
+        double t = waves * (full * even + 3.0);
+        if (rest > sms) t += full * even + 3.0;
+        else if (rest > 0) t += std::ceil(even) * std::max(least, 0.65 * full * rest / sms) + 3.0;
+        if (parts > 1) t += parts > kMaxCluster ? 8.0 : (parts == 16 && ctas > sms) ? 7.0 : 1.2;
+        if (t < best_t) { best_t = t; best = parts; }
+    }
+    a->parts = best;
+    a->merge = best > 1 && best <= kMaxCluster;
+}
+
 cudaError_t launch_decode(const DecodeArgs& a_in, const CUtensorMap& tk, const CUtensorMap& tv, int units, bool bf16,
                           cudaStream_t stream) {
-    static std::atomic<bool> configured[4][64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     DecodeArgs a = a_in;
-    // query heads that share a K/V head are packed into one CTA, eight at a time
     if (a.seqlen_q < 1 || a.seqlen_q > 8) return cudaErrorInvalidValue;
-    const bool packed = a.kv_group > 1 || a.seqlen_q > 1;
-    const int heads_per_cta = 8 / a.seqlen_q;  // whole heads whose query rows fit the eight columns
-    a.subgroups = packed ? (a.kv_group + heads_per_cta - 1) / heads_per_cta : 1;
-    const long long cta_units = packed ? static_cast<long long>(units / a.kv_group) * a.subgroups : units;
-    const long long ctas = cta_units * a.num_splits;
+    const long long ctas = static_cast<long long>(units / a.kv_group) * a.subgroups * a.parts;
     if (ctas <= 0 || ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    auto run = [&](auto kern, int which) -> cudaError_t {
-        if (dev < 0 || dev >= 64 || !configured[which][dev].load(std::memory_order_acquire)) {
-            cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDSmemBytes);
+    a.div_parts = make_fastdiv(static_cast<uint32_t>(a.parts));
+    a.div_subgroups = make_fastdiv(static_cast<uint32_t>(a.subgroups));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(kDThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(a.parts);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.merge ? 2 : 1;
+    auto run = [&](auto kern, int smem, std::atomic<bool>* configured) -> cudaError_t {
+        if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+            cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (err == cudaSuccess) err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (err != cudaSuccess) return err;
-            if (dev >= 0 && dev < 64) configured[which][dev].store(true, std::memory_order_release);
+            if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
         }
-        kern<<<static_cast<unsigned>(ctas), kDThreads, kDSmemBytes, stream>>>(tk, tv, a);
-        return cudaGetLastError();
+        cfg.dynamicSmemBytes = smem;
+        return cudaLaunchKernelEx(&cfg, kern, tk, tv, a);
     };
-    if (packed) return bf16 ? run(decode_kernel<true, 8>, 2) : run(decode_kernel<false, 8>, 3);
-    return bf16 ? run(decode_kernel<true, 1>, 0) : run(decode_kernel<false, 1>, 1);
+    auto by_type = [&](auto h, auto wide) -> cudaError_t {
+        constexpr int kH = decltype(h)::value, D = decltype(wide)::value, smem = DCfg<kH, D>::kSmemBytes;
+        static std::atomic<bool> configured[4][64];
+        if (a.drop.threshold != 0ull)
+            return bf16 ? run(decode_kernel<true, kH, D, true>, smem, configured[0]) : run(decode_kernel<false, kH, D, true>, smem, configured[1]);
+        return bf16 ? run(decode_kernel<true, kH, D, false>, smem, configured[2]) : run(decode_kernel<false, kH, D, false>, smem, configured[3]);
+    };
+    auto by_dim = [&](auto h) -> cudaError_t {
+        return a.head_dim <= 64 ? by_type(h, std::integral_constant<int, 64>()) : by_type(h, std::integral_constant<int, 128>());
+    };
+    switch (a.columns) {
+        case 1: return by_dim(std::integral_constant<int, 1>());
+        case 4: return by_dim(std::integral_constant<int, 4>());
+        case 8: return by_dim(std::integral_constant<int, 8>());
+        default: return by_dim(std::integral_constant<int, 16>());
+    }
 }
 
 }  // namespace fa

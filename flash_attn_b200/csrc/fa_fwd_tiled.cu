@@ -130,13 +130,6 @@ struct TileRange {
     int lo, hi;  // KV tiles [lo, hi)
 };
 
-__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t x) {
-    if (f.d == 1) return x;
-    uint32_t q = __umulhi(x, f.m);
-    if (q * f.d > x) --q;
-    return q;
-}
-
 __device__ __forceinline__ TileRange kv_tile_range(const FwdArgs& a, int rb, int split) {
     if (rb >= a.tr) return {0, 0};
     const long long q0 = a.q_pos0 + static_cast<long long>(rb) * kTile;

@@ -21,6 +21,15 @@ inline FastDiv make_fastdiv(uint32_t d) {
     return f;
 }
 
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t x) {
+    if (f.d == 1) return x;
+    uint32_t q = __umulhi(x, f.m);
+    if (q * f.d > x) --q;
+    return q;
+}
+#endif
+
 // Device-side argument block of the tiled forward kernel (the successor of
 // mykernelParamType, include/utils.h:21-44).  Q/K/V travel as TMA tensor maps.
 struct FwdArgs {
@@ -56,28 +65,39 @@ struct FwdArgs {
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const CUtensorMap& to, int units, bool bf16, bool dropout, cudaStream_t stream);
 
-// Device-side argument block of the decode kernel (seqlen_q = 1).
+// Device-side argument block of the decode kernel (seqlen_q <= 8).
 struct DecodeArgs {
-    const void* q;          // [units, d]
-    void* o;                // [units, d] (non-split)
-    float* lse;             // [units] or null
-    float* o_partial;       // [units, splits, d] fp32 (split)
-    float* lse_partial;     // [units, splits]
+    const void* q;          // [units, seqlen_q, d]
+    void* o;                // [units, seqlen_q, d] (a whole unit, or the parts of one merged in its cluster)
+    float* lse;             // [units, seqlen_q] or null
+    float* o_partial;       // [units, parts, seqlen_q, d] fp32 (parts left to the combine kernel)
+    float* lse_partial;     // [units, parts, seqlen_q]
     const float* alibi_slopes;
     int* status;
     int heads;
     int kv_group;           // query units per K/V unit; K/V unit = unit / kv_group
-    int subgroups;          // CTAs (of up to eight query columns) per K/V unit on the packed path; set by launch_decode
+    int columns;            // query columns of a CTA: 1, 4, 8 or 16
+    int subgroups;          // CTAs (each a part of the group's heads) per K/V unit
     int seqlen_q;           // query rows per unit, 1..8
     int seqlen_k, head_dim;
-    int tc;
-    int num_splits, tiles_per_split;
+    int tc;                 // key tiles
+    int vis_lo, vis_hi;     // key tiles that the masks leave visible to some query row: [vis_lo, vis_hi)
+    int full_lo, full_hi;   // key tiles that no mask touches
+    int parts;              // CTAs that share the keys of a unit
+    int merge;              // the parts are one cluster and merge their results themselves
+    int by_split;           // the parts are the caller's splits (dropout), tiles_per_split tiles each
+    int tiles_per_split;
     float scale_log2;
     int is_causal, window_left, window_right;
     long long q_pos0, k_pos0;
     int o_is_fp32;
+    FastDiv div_parts, div_subgroups;
     DropoutParams drop;
 };
+// How many CTAs share the keys of a unit (fills parts, merge, by_split, columns, subgroups and the
+// tile ranges; the problem's fields are set).  `splits` is the resolved split count of the caller.  A plan with parts > 1
+// and merge == 0 writes partials: they need a workspace, and the combine kernel behind.
+void plan_decode(DecodeArgs* a, int units, int splits, bool forced, int sms);
 cudaError_t launch_decode(const DecodeArgs& a, const CUtensorMap& tk, const CUtensorMap& tv, int units, bool bf16,
                           cudaStream_t stream);
 

@@ -58,7 +58,6 @@ int fa_fwd_static_scratch(const fa_fwd_params* p) {
     // Nothing in the scratch has to start at zero: the split kernel writes the
     // partial O and log-sum-exp of every (unit, split, row) it is launched for,
     // empty splits included, and the combine kernel reads only those.
-    q.num_splits = splits;
     q.workspace = scratch;
     q.workspace_bytes = FA_STATIC_SCRATCH_BYTES;
     return fa_fwd(&q);

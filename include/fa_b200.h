@@ -125,11 +125,14 @@ typedef struct fa_fwd_params {
  * Asynchronous on p->stream. */
 int fa_fwd(const fa_fwd_params* p);
 
-/* Bytes of workspace fa_fwd needs for p (0 when it neither splits nor pads head_dim).
+/* Bytes of workspace fa_fwd needs for p (0 when it neither keeps split partials nor pads head_dim).  With
+ * num_splits = n > 1 the partials of n splits; with 0 those of the launch the library plans, which may merge
+ * the parts on chip and keep none.
  * Replaces the cudaMalloc sizing of O_tmp/L/M at src/main.cu:160-162. */
 size_t fa_fwd_workspace_bytes(const fa_fwd_params* p);
 
-/* Split count fa_fwd will use for p (resolves num_splits == 0). */
+/* Split count of p (resolves num_splits == 0).  With dropout it is the geometry of the dropout streams; without,
+ * the kernels may divide the keys among more or fewer CTAs than that, as suits the device. */
 int fa_fwd_resolve_splits(const fa_fwd_params* p);
 
 /* The reference's split policy, same arguments and result as

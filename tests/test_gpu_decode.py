@@ -60,3 +60,21 @@ def test_decode_config4_shape_sampled_units():
         err = np.abs(o[b, h].float().cpu().numpy() - want_o[0, 0])
         assert err.max() <= gpu_util.O_MAX_ABS and err.mean() <= gpu_util.O_MEAN_ABS, (b, h, err.max())
         assert abs(lse[b, h, 0].item() - want_lse[0, 0, 0]) <= gpu_util.LSE_ABS
+
+
+@pytest.mark.parametrize("H,Hk,Nq,nk,d,dtype,kw", [
+    (8, 2, 1, 129, 128, "bfloat16", {}),                      # 4 columns; two tiles, the second with one key
+    (8, 2, 1, 1023, 128, "float16", {}),                      # 8-CTA cluster, one tile each, the last ragged
+    (8, 2, 1, 2100, 64, "bfloat16", {}),                      # 16-CTA cluster, uneven parts, 64-wide tiles
+    (7, 1, 1, 4097, 128, "bfloat16", {}),                     # 8 columns, one unused
+    (8, 2, 4, 3000, 128, "bfloat16", {}),                     # 16 columns: 4 heads x 4 rows
+    (12, 1, 5, 2500, 64, "float16", dict(window=(700, 0))),   # 15 columns, four sub-groups of 3 heads, clipped tiles
+    (4, 2, 8, 1500, 96, "bfloat16", dict(alibi=True)),        # 16 columns with a bias per head
+    (2, 1, 3, 5000, 128, "bfloat16", dict(window=(100, 0))),  # few visible tiles in a long cache
+    (4, 1, 1, 65500, 64, "bfloat16", dict(num_splits=0)),     # more parts than a cluster holds: the combine kernel
+    (4, 1, 2, 900, 128, "float16", dict(p_dropout=0.2, num_splits=4)),   # the caller's splits, merged in the cluster
+    (2, 2, 1, 900, 128, "float16", dict(p_dropout=0.2, num_splits=5)),   # ... and through the workspace
+])
+def test_parts_of_a_unit_and_query_columns(H, Hk, Nq, nk, d, dtype, kw):
+    gpu_util.assert_close(gpu_util.run_case(1, H, Nq, nk, d, dtype, seed=58, causal=True, q_pos0=nk - Nq, heads_k=Hk, **kw),
+                          f"{H}/{Hk} heads, {Nq} rows, {nk} keys, d={d} {kw}")
