@@ -211,15 +211,19 @@ void fill_decode_args(const fa_fwd_params* p, const FwdArgs& a, DecodeArgs* d) {
     d->q_pos0 = a.q_pos0; d->k_pos0 = a.k_pos0; d->o_is_fp32 = a.o_is_fp32; d->drop = a.drop;
 }
 
-// Partial results per unit that a launch with num_splits = 0 keeps in the workspace (1 = none).
+// Partial results per unit that a launch keeps in the workspace (1 = none).
 int planned_parts(const fa_fwd_params* p, int splits, int sms) {
-    if (p->seqlen_q > 8 || p->accum_o != nullptr) return splits;
+    if (p->seqlen_q > 8 || p->accum_o != nullptr) return p->p_dropout > 0.0f ? splits : 1;
     FwdArgs a;
     DecodeArgs d;
     fill_args(p, splits, &a);
     fill_decode_args(p, a, &d);
     plan_decode(&d, p->batch * p->heads, splits, false, sms);
     return d.merge ? 1 : d.parts;
+}
+// What the workspace has to hold: a caller that names its split count provides for that count, whatever is made of it.
+int partials_kept(const fa_fwd_params* p, int splits, int sms) {
+    return p->num_splits == 0 ? planned_parts(p, splits, sms) : splits;
 }
 
 // head_dim that is not a multiple of 8: Q/K/V are copied to a pitch of d8 = ceil8(head_dim)
@@ -238,6 +242,84 @@ PadPlan pad_plan(const fa_fwd_params* p) {
     pl.o_bytes = up(units * p->seqlen_q * pl.d8 * (p->o_dtype == FA_DTYPE_FP32 ? 4 : 2));
     pl.total = pl.q_bytes + 2 * pl.kv_bytes + pl.o_bytes;
     return pl;
+}
+
+// One call whose rows are 16-byte multiples; O has o_dim <= head_dim columns.
+int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
+    int rc = FA_OK;
+    const int units = p->batch * p->heads;
+    cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+    FwdArgs a;
+    fill_args(p, splits, &a);
+    a.o_dim = o_dim;
+    const bool decode = p->seqlen_q <= 8 && p->accum_o == nullptr;
+    DecodeArgs d;
+    const bool dropout = p->p_dropout > 0.0f;
+    int parts = splits;  // partial results per unit
+    if (!decode && !dropout) {
+        // how the keys are shared out is the library's business; the parts of a query block merge on chip
+        a.num_splits = parts = 1;
+        a.tiles_per_split = a.tc;
+        plan_tiled(&a, sms);
+    }
+    if (decode) {
+        fill_decode_args(p, a, &d);
+        d.o_dim = o_dim;
+        plan_decode(&d, units, splits, p->num_splits > 0, sms);
+        parts = d.merge ? 1 : d.parts;
+    }
+    if (splits > 1 || parts > 1) {
+        size_t lse_off = 0;
+        const size_t need = partial_bytes(p, parts, &lse_off);
+        // (a caller that names its split count provides the workspace of that count, whatever is made of it)
+        const size_t promised = p->num_splits > 0 ? partial_bytes(p, splits, nullptr) : need;
+        const bool aligned = (reinterpret_cast<uintptr_t>(p->workspace) & 15u) == 0;
+        const bool missing = !p->workspace || p->workspace_bytes < std::max(need, promised) || (splits == 1 && !aligned);
+        if (missing && parts > 1 && splits == 1) {
+            // the split count was the library's to choose and the caller keeps no workspace
+            d.parts = 8;
+            d.merge = 1;
+            parts = 1;
+        } else if (missing && (parts > 1 || p->num_splits > 1)) {
+            return FA_ERR_WORKSPACE;
+        }
+        if (!missing && !aligned) return FA_ERR_INVALID_ARG;
+        if (parts > 1) {
+            a.o_partial = d.o_partial = static_cast<float*>(p->workspace);
+            a.lse_partial = d.lse_partial = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + lse_off);
+        }
+    }
+    const bool bf16 = p->dtype == FA_DTYPE_BF16;
+    CUtensorMap tk, tv;
+    const int units_k = p->batch * kv_heads(p);
+    if ((rc = make_tensor_map(&tk, bf16, p->k, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
+    if ((rc = make_tensor_map(&tv, bf16, p->v, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
+    if (decode) {
+        // one to eight query rows per unit: the streaming kernel with keys on the tensor-memory lanes
+        if (launch_decode(d, tk, tv, units, bf16, stream) != cudaSuccess) return FA_ERR_CUDA;
+    } else {
+        CUtensorMap tq;
+        if ((rc = make_tensor_map(&tq, bf16, p->q, p->head_dim, a.seqlen_q, a.units)) != FA_OK) return rc;
+        // 16-bit output of an unsplit launch is written by TMA stores, one 32-row box per warp
+        CUtensorMap to = tq;
+        a.o_tma = (!a.staged && a.num_splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
+        if (a.o_tma && (rc = make_tensor_map(&to, bf16, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
+        if (launch_fwd_tiled(a, tq, tk, tv, to, a.units, bf16, dropout, stream) != cudaSuccess) return FA_ERR_CUDA;
+    }
+    if (parts > 1) {
+        CombineArgs c;
+        c.o_partial = a.o_partial;
+        c.lse_partial = a.lse_partial;
+        c.o = p->o;
+        c.lse = p->lse;
+        c.rows_per_unit = p->seqlen_q;
+        c.num_splits = parts;
+        c.head_dim = p->head_dim;
+        c.o_dim = o_dim;
+        c.o_dtype = p->o_dtype;
+        if (launch_combine(c, units, stream) != cudaSuccess) return FA_ERR_CUDA;
+    }
+    return FA_OK;
 }
 
 }  // namespace
@@ -316,93 +398,33 @@ int fa_fwd(const fa_fwd_params* p) {
     if (major != 10) return FA_ERR_NOT_SM100;
     const int splits = resolve_splits(p, sms);
     if (p->accum_o != nullptr && (splits > 1 || p->head_dim % 8 != 0)) return FA_ERR_UNSUPPORTED;
-    const int units = p->batch * p->heads;
+    if (p->head_dim % 8 == 0) return run_fwd(p, p->head_dim, splits, sms);
+
+    // padded pitch: copy Q, K, V into the workspace and run on head_dim = d8; O is written with its own pitch,
+    // except by the dropout kernels for more than eight query rows, whose O is re-pitched from the workspace
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    if (p->head_dim % 8 != 0) {
-        // padded pitch: re-pitch Q, K, V into the workspace, run on head_dim = d8, re-pitch O back
-        const PadPlan pl = pad_plan(p);
-        fa_fwd_params q = *p;
-        q.head_dim = pl.d8;
-        const int parts = p->num_splits == 0 ? planned_parts(&q, splits, sms) : splits;
-        const size_t part = parts > 1 ? partial_bytes(&q, parts, nullptr) : 0;
-        if (!p->workspace || p->workspace_bytes < pl.total + part) return FA_ERR_WORKSPACE;
-        if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return FA_ERR_INVALID_ARG;
-        char* ws = static_cast<char*>(p->workspace);
-        char* qp = ws; char* kp = qp + pl.q_bytes; char* vp = kp + pl.kv_bytes; char* op = vp + pl.kv_bytes;
-        const long long rq = static_cast<long long>(units) * p->seqlen_q;
-        const long long rk = static_cast<long long>(p->batch) * kv_heads(p) * p->seqlen_k;
-        if (launch_repitch(p->q, qp, 2, rq, p->head_dim, pl.d8, stream) != cudaSuccess ||
-            launch_repitch(p->k, kp, 2, rk, p->head_dim, pl.d8, stream) != cudaSuccess ||
-            launch_repitch(p->v, vp, 2, rk, p->head_dim, pl.d8, stream) != cudaSuccess)
-            return FA_ERR_CUDA;
-        q.q = qp; q.k = kp; q.v = vp; q.o = op;
-        q.workspace = part ? op + pl.o_bytes : nullptr;
-        q.workspace_bytes = part;
-        rc = fa_fwd(&q);
-        if (rc != FA_OK) return rc;
-        if (launch_repitch(op, p->o, p->o_dtype == FA_DTYPE_FP32 ? 4 : 2, rq, pl.d8, p->head_dim, stream) != cudaSuccess)
-            return FA_ERR_CUDA;
-        return FA_OK;
-    }
-    FwdArgs a;
-    fill_args(p, splits, &a);
-    const bool decode = p->seqlen_q <= 8 && p->accum_o == nullptr;
-    DecodeArgs d;
-    int parts = splits;  // partial results per unit
-    if (decode) {
-        fill_decode_args(p, a, &d);
-        plan_decode(&d, units, splits, p->num_splits > 0, sms);
-        parts = d.merge ? 1 : d.parts;
-    }
-    if (splits > 1 || parts > 1) {
-        size_t lse_off = 0;
-        const size_t need = partial_bytes(p, parts, &lse_off);
-        // (a caller that names its split count provides the workspace of that count, whatever is made of it)
-        const size_t promised = p->num_splits > 0 ? partial_bytes(p, splits, nullptr) : need;
-        const bool missing = !p->workspace || p->workspace_bytes < std::max(need, promised);
-        if (missing && parts > 1 && splits == 1) {
-            // the split count was the library's to choose and the caller keeps no workspace
-            d.parts = 8;
-            d.merge = 1;
-            parts = 1;
-        } else if (missing && (parts > 1 || p->num_splits > 1)) {
-            return FA_ERR_WORKSPACE;
-        }
-        if (parts > 1) {
-            if (reinterpret_cast<uintptr_t>(p->workspace) & 15u) return FA_ERR_INVALID_ARG;
-            a.o_partial = d.o_partial = static_cast<float*>(p->workspace);
-            a.lse_partial = d.lse_partial = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + lse_off);
-        }
-    }
-    const bool bf16 = p->dtype == FA_DTYPE_BF16;
-    CUtensorMap tk, tv;
-    const int units_k = p->batch * kv_heads(p);
-    if ((rc = make_tensor_map(&tk, bf16, p->k, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
-    if ((rc = make_tensor_map(&tv, bf16, p->v, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
-    if (decode) {
-        // one to eight query rows per unit: the streaming kernel with keys on the tensor-memory lanes
-        if (launch_decode(d, tk, tv, units, bf16, stream) != cudaSuccess) return FA_ERR_CUDA;
-    } else {
-        CUtensorMap tq;
-        if ((rc = make_tensor_map(&tq, bf16, p->q, p->head_dim, p->seqlen_q, units)) != FA_OK) return rc;
-        // 16-bit output of an unsplit launch is written by TMA stores, one 32-row box per warp
-        CUtensorMap to = tq;
-        a.o_tma = (splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
-        if (a.o_tma && (rc = make_tensor_map(&to, bf16, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
-        if (launch_fwd_tiled(a, tq, tk, tv, to, units, bf16, p->p_dropout > 0.0f, stream) != cudaSuccess) return FA_ERR_CUDA;
-    }
-    if (parts > 1) {
-        CombineArgs c;
-        c.o_partial = a.o_partial;
-        c.lse_partial = a.lse_partial;
-        c.o = p->o;
-        c.lse = p->lse;
-        c.rows_per_unit = p->seqlen_q;
-        c.num_splits = parts;
-        c.head_dim = p->head_dim;
-        c.o_dtype = p->o_dtype;
-        if (launch_combine(c, units, stream) != cudaSuccess) return FA_ERR_CUDA;
-    }
+    const long long units = static_cast<long long>(p->batch) * p->heads;
+    const PadPlan pl = pad_plan(p);
+    fa_fwd_params q = *p;
+    q.head_dim = pl.d8;
+    const int parts = partials_kept(&q, splits, sms);
+    const size_t part = parts > 1 ? partial_bytes(&q, parts, nullptr) : 0;
+    if (!p->workspace || p->workspace_bytes < pl.total + part) return FA_ERR_WORKSPACE;
+    if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return FA_ERR_INVALID_ARG;
+    char* ws = static_cast<char*>(p->workspace);
+    char* qp = ws; char* kp = qp + pl.q_bytes; char* vp = kp + pl.kv_bytes; char* op = vp + pl.kv_bytes;
+    const long long rq = units * p->seqlen_q;
+    const long long rk = static_cast<long long>(p->batch) * kv_heads(p) * p->seqlen_k;
+    if (launch_pad_qkv(p->q, p->k, p->v, qp, kp, vp, rq, rk, p->head_dim, pl.d8, stream) != cudaSuccess) return FA_ERR_CUDA;
+    q.q = qp; q.k = kp; q.v = vp;
+    q.workspace = part ? op + pl.o_bytes : nullptr;
+    q.workspace_bytes = part;
+    const bool direct = !(p->p_dropout > 0.0f) || p->seqlen_q <= 8 || splits > 1;
+    if (direct) return run_fwd(&q, p->head_dim, splits, sms);
+    q.o = op;
+    if ((rc = run_fwd(&q, pl.d8, splits, sms)) != FA_OK) return rc;
+    if (launch_repitch(op, p->o, p->o_dtype == FA_DTYPE_FP32 ? 4 : 2, rq, pl.d8, p->head_dim, stream) != cudaSuccess)
+        return FA_ERR_CUDA;
     return FA_OK;
 }
 

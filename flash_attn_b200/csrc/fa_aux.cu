@@ -40,7 +40,7 @@ __global__ void combine_kernel(const CombineArgs a, long long total_rows) {
         for (int j = 0; j < a.num_splits; ++j) l += __expf(lp[j * a.rows_per_unit] - m);
     const float lse = (m == -INFINITY) ? -INFINITY : m + __logf(l);
     if (lane == 0 && a.lse != nullptr) a.lse[row] = lse;
-    for (int c = lane; c < a.head_dim; c += 32) {
+    for (int c = lane; c < a.o_dim; c += 32) {
         float acc = 0.0f;
         if (m != -INFINITY) {
             for (int j = 0; j < a.num_splits; ++j) {
@@ -49,7 +49,7 @@ __global__ void combine_kernel(const CombineArgs a, long long total_rows) {
                 acc += w * a.o_partial[prow * a.head_dim + c];
             }
         }
-        store_out(a.o, a.o_dtype, row * a.head_dim + c, acc);
+        store_out(a.o, a.o_dtype, row * a.o_dim + c, acc);
     }
 }
 
@@ -99,6 +99,34 @@ __global__ void repitch_kernel(const T* src, T* dst, long long rows, int d_src, 
     const long long r = i / d_dst;
     const int c = static_cast<int>(i - r * d_dst);
     dst[i] = c < d_src ? src[r * d_src + c] : T(0);
+}
+
+// Q, K, V together: eight elements of a padded row per thread, written as one 16-byte store.  (One launch instead of
+// three, and it starts while the kernel in front drains: short problems are bound by the launches, not by the bytes.)
+struct PadArgs {
+    const uint16_t* src[3];
+    uint4* dst[3];
+    long long chunks[3];  // 16-byte chunks of each destination
+    int d_src;
+    FastDiv per_row;      // chunks per row
+};
+__global__ void pad_qkv_kernel(const PadArgs a) {
+    grid_dep_launch_dependents();
+    grid_dep_wait();
+    const int t = blockIdx.y;
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < a.chunks[t]; i += stride) {
+        const long long row = i <= 0xffffffffLL ? static_cast<long long>(fast_div(a.per_row, static_cast<uint32_t>(i))) : i / a.per_row.d;
+        const int c0 = static_cast<int>(i - row * a.per_row.d) * 8;
+        const uint16_t* src = a.src[t] + row * a.d_src + c0;
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t lo = c0 + 2 * e < a.d_src ? src[2 * e] : 0u, hi = c0 + 2 * e + 1 < a.d_src ? src[2 * e + 1] : 0u;
+            w[e] = lo | (hi << 16);
+        }
+        a.dst[t][i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
 }
 
 // keep[unit, row, col] for the geometry in `a` (same map as the tiled kernel).
@@ -193,6 +221,35 @@ cudaError_t launch_repitch(const void* src, void* dst, int elem_bytes, long long
     else
         repitch_kernel<uint32_t><<<blocks, threads, 0, stream>>>(static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), rows, d_src, d_dst);
     return cudaGetLastError();
+}
+
+cudaError_t launch_pad_qkv(const void* q, const void* k, const void* v, void* qp, void* kp, void* vp, long long rows_q,
+                           long long rows_k, int d_src, int d_dst, cudaStream_t stream) {
+    PadArgs a;
+    const void* src[3] = {q, k, v};
+    void* dst[3] = {qp, kp, vp};
+    const int per_row = d_dst / 8;
+    long long most = 0;
+    for (int i = 0; i < 3; ++i) {
+        a.src[i] = static_cast<const uint16_t*>(src[i]);
+        a.dst[i] = static_cast<uint4*>(dst[i]);
+        a.chunks[i] = (i == 0 ? rows_q : rows_k) * per_row;
+        most = a.chunks[i] > most ? a.chunks[i] : most;
+    }
+    a.d_src = d_src;
+    a.per_row = make_fastdiv(static_cast<uint32_t>(per_row));
+    const int threads = 256;
+    const long long blocks = (most + threads - 1) / threads;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks < 1184 ? blocks : 1184), 3);  // (at most 8 blocks an SM and tensor)
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, pad_qkv_kernel, a);
 }
 
 cudaError_t launch_dropout_mask(const FwdArgs& a, uint8_t* keep, long long units, cudaStream_t stream) {

@@ -145,10 +145,10 @@ __device__ __forceinline__ void named_barrier_128() { asm volatile("bar.sync 1, 
 // One element of a finished output row, and (thread 0) its log-sum-exp.
 template <bool kBf16>
 __device__ __forceinline__ void store_result(const DecodeArgs& a, long long row, int col, float o_val, float lse_val) {
-    if (col < a.head_dim) {
-        if (a.o_is_fp32) static_cast<float*>(a.o)[row * a.head_dim + col] = o_val;
-        else if (kBf16) static_cast<__nv_bfloat16*>(a.o)[row * a.head_dim + col] = __float2bfloat16_rn(o_val);
-        else static_cast<__half*>(a.o)[row * a.head_dim + col] = __float2half_rn(o_val);
+    if (col < a.o_dim) {
+        if (a.o_is_fp32) static_cast<float*>(a.o)[row * a.o_dim + col] = o_val;
+        else if (kBf16) static_cast<__nv_bfloat16*>(a.o)[row * a.o_dim + col] = __float2bfloat16_rn(o_val);
+        else static_cast<__half*>(a.o)[row * a.o_dim + col] = __float2half_rn(o_val);
     }
     if (col == 0 && a.lse != nullptr) a.lse[row] = lse_val;
 }
@@ -613,6 +613,13 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                         const float w = ex2f(m_j[j] - m);
                         l = fmaf(w, l_j[j], l);
                         o = fmaf(w, o_j[j], o);
+                    }
+                } else {
+                    // no visible key (all zero), or nothing but NaN
+#pragma unroll
+                    for (int j = 0; j < kMaxCluster; ++j) {
+                        l += l_j[j];
+                        o += o_j[j];
                     }
                 }
                 const float inv = l > 0.0f ? a.drop.inv_keep / l : 0.0f;

@@ -130,11 +130,21 @@ struct TileRange {
     int lo, hi;  // KV tiles [lo, hi)
 };
 
+template <bool kStaged>
 __device__ __forceinline__ TileRange kv_tile_range(const FwdArgs& a, int rb, int split) {
     if (rb >= a.tr) return {0, 0};
-    const long long q0 = a.q_pos0 + static_cast<long long>(rb) * kTile;
+    int first = rb * kTile, last_row = first + kTile - 1;  // rows of the tile
+    if (kStaged && a.pack_rows > 0) {
+        // rows of stacked heads: a tile that reaches into another head has every position of a head
+        last_row = min(last_row, a.seqlen_q - 1);
+        const int h0 = static_cast<int>(fast_div(a.div_pack, static_cast<uint32_t>(first)));
+        const int h1 = static_cast<int>(fast_div(a.div_pack, static_cast<uint32_t>(last_row)));
+        first = h0 == h1 ? first - h0 * a.pack_rows : 0;
+        last_row = h0 == h1 ? last_row - h0 * a.pack_rows : a.pack_rows - 1;
+    }
+    const long long q0 = a.q_pos0 + first, q1 = a.q_pos0 + last_row;
     int lo = 0, hi = a.tc;
-    if (a.num_splits > 1) {  // src/flash_forward_splitkv.h:40-43
+    if (!kStaged && a.num_splits > 1) {  // src/flash_forward_splitkv.h:40-43
         lo = a.tiles_per_split * split;
         hi = min(lo + a.tiles_per_split, a.tc);
     }
@@ -143,11 +153,11 @@ __device__ __forceinline__ TileRange kv_tile_range(const FwdArgs& a, int rb, int
         lo = max(lo, static_cast<int>(max(0LL, min(w, static_cast<long long>(a.tc)))));
     }
     if (a.window_right >= 0) {  // src/flash_forward.h:42-44
-        const long long last = q0 + kTile - 1 + a.window_right - a.k_pos0;
+        const long long last = q1 + a.window_right - a.k_pos0;
         hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
     }
     if (a.is_causal) {  // src/flash_forward.h:46-48
-        const long long last = q0 + kTile - 1 - a.k_pos0;
+        const long long last = q1 - a.k_pos0;
         hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
     }
     if (hi < lo) hi = lo;
@@ -306,7 +316,101 @@ __device__ __forceinline__ void issue_qk_bias(uint32_t d_tmem, uint32_t qa_lo, u
         : "memory");
 }
 
-template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout>
+// The end of a staged launch: the CTAs of a cluster hold, for the same NQ * 128 query rows, the un-normalised
+// rows, maxima and sums over their own keys (one CTA, parts = 1: all keys).  Each CTA finishes an equal share of the
+// rows from all of them, O = sum_j 2^(m_j - m) O_j / l, l = sum_j 2^(m_j - m) l_j
+// (src/flash_forward_splitkv.h:359-397), and writes them a row or two per warp instruction.
+template <int D, int NQ, bool kBf16>
+__device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, uint32_t smem_base, int part, int unit, int qb) {
+    using C = Cfg<D, NQ>;
+    constexpr int kRows = NQ * kTile, kThreads = NQ * 128;
+    const int r_lo = static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(kRows * part)));
+    const int r_hi = min(static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(kRows * (part + 1)))), a.seqlen_q - qb * kRows);
+    const int n_rows = max(r_hi - r_lo, 0);
+    // a thread per row: the weights of the parts (float [n_rows][parts], behind the (m, l) pairs in the Q buffers,
+    // which the peers read) and the log-sum-exp
+    float* wts = reinterpret_cast<float*>(smem_gen + C::kSmemQ + kRows * 8);
+    const long long row0 = static_cast<long long>(unit) * a.seqlen_q + qb * kRows + r_lo;
+    for (int k = threadIdx.x; k < n_rows; k += kThreads) {
+        const uint32_t ml = smem_base + C::kSmemQ + (r_lo + k) * 8;
+        float* w = wts + k * a.parts;
+        float m = -INFINITY, l = 0.0f;
+        for (int j0 = 0; j0 < a.parts; j0 += 4) {  // (four remote loads in flight)
+            float2 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = ld_cluster_f32x2(cluster_map(ml, min(j0 + i, a.parts - 1)));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (j0 + i >= a.parts) break;
+                const float m_new = fmaxf(m, v[i].x);
+                // (a part that saw no key has m = -inf, l = 0; one that saw only NaN has m = -inf, l = NaN)
+                l = m_new == -INFINITY ? l + v[i].y : fmaf(l, fast_exp2(m - m_new), v[i].y * fast_exp2(v[i].x - m_new));
+                m = m_new;
+                w[j0 + i] = v[i].x;
+            }
+        }
+        float inv = l == 0.0f ? 0.0f : 1.0f / l;
+        float lse = l > 0.0f ? m * kLn2 + __logf(l) : -INFINITY;
+        for (int j = 0; j < a.parts; ++j) w[j] = inv == 0.0f ? 0.0f : fast_exp2(w[j] - m) * inv;
+        if (a.lse != nullptr) a.lse[row0 + k] = lse;
+    }
+    __syncwarp();
+    asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
+
+    constexpr int kLanes = D / 4, kPerWarp = 32 / kLanes;  // 16-byte chunks of a row; rows per warp instruction
+    constexpr int kStep = NQ * 4 * kPerWarp, kUnroll = 4;  // rows per CTA instruction; loads in flight
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int chunk = lane % kLanes, col = chunk * 4;
+    const bool aligned = a.o_dim % 8 == 0;  // (a padded problem's own rows start anywhere)
+    for (int k0 = warp * kPerWarp + lane / kLanes; k0 < n_rows; k0 += kStep * kUnroll) {
+        float4 acc[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) acc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
+        for (int j = 0; j < a.parts; ++j) {
+            const bool own = j == part;
+            const uint32_t base = own ? smem_base + C::kSmemK : cluster_map(smem_base + C::kSmemK, j);
+            float4 v[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const int row = r_lo + k0 + u * kStep;
+                const uint32_t addr = base + row * (D * 4) + (chunk ^ (row & 7)) * 16;
+                v[u] = own ? ld_shared_f32x4_if(addr, k0 + u * kStep < n_rows) : ld_cluster_f32x4_if(addr, k0 + u * kStep < n_rows);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const float w = wts[min(k0 + u * kStep, n_rows - 1) * a.parts + j];
+                if (w != 0.0f) {
+                    acc[u].x = fmaf(w, v[u].x, acc[u].x);
+                    acc[u].y = fmaf(w, v[u].y, acc[u].y);
+                    acc[u].z = fmaf(w, v[u].z, acc[u].z);
+                    acc[u].w = fmaf(w, v[u].w, acc[u].w);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int k = k0 + u * kStep;
+            if (k >= n_rows || col >= a.o_dim) continue;
+            const float4 o = acc[u];
+            const long long at = (row0 + k) * a.o_dim + col;
+            if (aligned) {
+                if (a.o_is_fp32) *reinterpret_cast<float4*>(static_cast<float*>(a.o) + at) = o;
+                else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.o) + at) = make_uint2(pack2<kBf16>(o.x, o.y), pack2<kBf16>(o.z, o.w));
+            } else {
+                const float e[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (col + i >= a.o_dim) continue;
+                    if (a.o_is_fp32) static_cast<float*>(a.o)[at + i] = e[i];
+                    else static_cast<uint16_t*>(a.o)[at + i] = static_cast<uint16_t>(pack2<kBf16>(e[i], 0.0f));
+                }
+            }
+        }
+    }
+}
+
+template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged>
 __global__ void __launch_bounds__(Cfg<D, NQ>::kThreads, NQ == 1 ? 2 : 1)
 fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
@@ -368,10 +472,12 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // flight (one group) stays far below the L2 size.
     // (the divisors are launch constants: multiply-high instead of the hardware's slow integer divide,
     // which sat on the path to the first TMA load)
-    const uint32_t group = fast_div(a.div_group_ctas, blockIdx.x);
+    const uint32_t block = kStaged ? fast_div(a.div_parts, blockIdx.x) : blockIdx.x;
+    const int part = kStaged ? static_cast<int>(blockIdx.x - block * a.div_parts.d) : 0;  // (= the CTA's rank in its cluster)
+    const uint32_t group = fast_div(a.div_group_ctas, block);
     const int unit0 = static_cast<int>(group) * a.unit_group;
     const bool full_group = unit0 + a.unit_group <= a.units;
-    const uint32_t rem = blockIdx.x - group * a.div_group_ctas.d;
+    const uint32_t rem = block - group * a.div_group_ctas.d;
     const uint32_t bx = fast_div(full_group ? a.div_gsize : a.div_last_gsize, rem);
     const int unit = unit0 + static_cast<int>(rem - bx * (full_group ? a.div_gsize.d : a.div_last_gsize.d));
     const int kv_unit = static_cast<int>(fast_div(a.div_kv_group, static_cast<uint32_t>(unit)));  // grouped-query attention: K/V head of this unit
@@ -402,7 +508,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // (the NQ ranges are worked out side by side on lanes 0..NQ-1 and handed round)
     TileRange range[NQ];
     {
-        const TileRange mine = kv_tile_range(a, qb * NQ + (lane & (NQ - 1)), split);
+        const TileRange mine = kv_tile_range<kStaged>(a, qb * NQ + (lane & (NQ - 1)), split);
 #pragma unroll
         for (int i = 0; i < NQ; ++i) {
             range[i].lo = NQ == 1 ? mine.lo : __shfl_sync(0xffffffffu, mine.lo, i);
@@ -415,6 +521,23 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (range[i].hi > range[i].lo) {
             lo = min(lo, range[i].lo);
             hi = max(hi, range[i].hi);
+        }
+    }
+    if constexpr (kStaged) {
+        // this CTA's share of the KV tiles that its query block sees
+        const int n_all = hi > lo ? hi - lo : 0, lo_all = hi > lo ? lo : 0;
+        const int p_lo = lo_all + static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(n_all * part)));
+        const int p_hi = lo_all + static_cast<int>(fast_div(a.div_parts, static_cast<uint32_t>(n_all * (part + 1))));
+        lo = 0x7fffffff;
+        hi = 0;
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            range[i].lo = max(range[i].lo, p_lo);
+            range[i].hi = max(min(range[i].hi, p_hi), range[i].lo);
+            if (range[i].hi > range[i].lo) {
+                lo = min(lo, range[i].lo);
+                hi = max(hi, range[i].hi);
+            }
         }
     }
     const int n_union = hi > lo ? hi - lo : 0;  // KV tiles streamed by this CTA: [lo, hi)
@@ -571,16 +694,18 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             const uint64_t dqk = make_smem_desc(0, 0, 1024);
             const uint64_t dvv = make_smem_desc(0, kTile * 128, 1024);
             const uint32_t desc_hi = static_cast<uint32_t>(dqk >> 32);
-            const uint32_t q_lo = static_cast<uint32_t>(dqk) | (sQ >> 4);
-            const uint32_t k_lo = static_cast<uint32_t>(dqk) | (sK >> 4);
-            const uint32_t v_lo = static_cast<uint32_t>(dvv) | (sV >> 4);
+            // (the address field has 14 bits: in a cluster a CTA's own shared addresses carry its rank above them)
+            constexpr uint32_t kAddrMask = 0x3FFFFu;
+            const uint32_t q_lo = static_cast<uint32_t>(dqk) | ((sQ & kAddrMask) >> 4);
+            const uint32_t k_lo = static_cast<uint32_t>(dqk) | ((sK & kAddrMask) >> 4);
+            const uint32_t v_lo = static_cast<uint32_t>(dvv) | ((sV & kAddrMask) >> 4);
             auto issue_qk = [&](int i, int st) {
                 issue_qk_block<D>(tmem_base + i * kTile, q_lo + ((i * C::kTileBytes) >> 4),
                                   k_lo + ((st * C::kTileBytes) >> 4), desc_hi, idesc_qk);
                 if constexpr (kBias) {
                     if (bias_in_mma)
-                        issue_qk_bias(tmem_base + i * kTile, static_cast<uint32_t>(dqk) | ((smem_base + C::kSmemBiasQ) >> 4),
-                                      static_cast<uint32_t>(dqk) | ((smem_base + C::kSmemBiasK) >> 4), desc_hi, idesc_qk);
+                        issue_qk_bias(tmem_base + i * kTile, static_cast<uint32_t>(dqk) | (((smem_base + C::kSmemBiasQ) & kAddrMask) >> 4),
+                                      static_cast<uint32_t>(dqk) | (((smem_base + C::kSmemBiasK) & kAddrMask) >> 4), desc_hi, idesc_qk);
                 }
             };
             auto issue_pv_a = [&](int i, int st, uint32_t accumulate) {
@@ -667,7 +792,10 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int rb = qb * NQ + qi;                     // its 128-row block inside the unit
         const int r = threadIdx.x & 127;                 // row inside the tile
         const int row = rb * kTile + r;                  // row inside the unit
-        const long long qpos = a.q_pos0 + row;
+        int row_pos = row;  // position inside the head
+        if (kStaged && a.pack_rows > 0)
+            row_pos = row - static_cast<int>(fast_div(a.div_pack, static_cast<uint32_t>(row))) * a.pack_rows;
+        const long long qpos = a.q_pos0 + row_pos;
         const TileRange mine_r = (qi == 0) ? range[0] : range[NQ - 1];
         const int t_lo = mine_r.lo;
         const int n_tiles = mine_r.hi - mine_r.lo;
@@ -898,6 +1026,30 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             else fail = 9;
         }
         FA_TR(96);
+        if constexpr (kStaged) {
+            // un-normalised rows, maxima and sums go to shared memory (the ring is free once the MMAs of both
+            // query tiles have completed, the Q tiles too); merge_rows below finishes them
+            asm volatile("bar.sync 5, %0;" ::"n"(NQ * 128) : "memory");
+            const uint32_t stage = sK + (qi * kTile + r) * (D * 4);
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+                uint32_t orow[32];
+                if (have_o) {
+                    tmem_ld32(tmem_o + lane_base + c * 32, orow);
+                    tmem_wait_ld();
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) orow[i] = 0u;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {  // 16-byte chunks, spread over the banks by the row
+                    const uint32_t chunk = static_cast<uint32_t>((c * 32 + i) >> 2) ^ static_cast<uint32_t>(r & 7);
+                    st_shared_v4(stage + chunk * 16, orow[i], orow[i + 1], orow[i + 2], orow[i + 3]);
+                }
+            }
+            *reinterpret_cast<float2*>(smem_gen + C::kSmemQ + (qi * kTile + r) * 8) =
+                make_float2(have_o ? m_ref : -INFINITY, have_o ? l_sum : 0.0f);
+        } else {
         float inv = 0.0f;
         if (l_sum > 0.0f) inv = (kDropout ? a.drop.inv_keep : 1.0f) / l_sum;
         const bool row_ok = row < a.seqlen_q;
@@ -1057,6 +1209,16 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
         }
         }
+        }
+    }
+
+    if constexpr (kStaged) {
+        __syncwarp();
+        if (a.parts > 1) cluster_sync();
+        else __syncthreads();
+        if (warp < NQ * 4) merge_rows<D, NQ, kBf16>(a, smem_gen, smem_base, part, unit, qb);
+        __syncwarp();
+        if (a.parts > 1) cluster_sync();  // the peers' shared memory stays until everyone has read it
     }
 
     // ---- teardown ------------------------------------------------------------------
@@ -1078,10 +1240,10 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
 }
 
-template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout>
+template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged>
 cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                        const CUtensorMap& to, int units, cudaStream_t stream) {
-    auto kern = fwd_tiled_kernel<D, NQ, kBf16, kAlibi, kDropout>;
+    auto kern = fwd_tiled_kernel<D, NQ, kBf16, kAlibi, kDropout, kStaged>;
     constexpr int smem = (kAlibi && Cfg<D, NQ>::kBiasBoxes) ? Cfg<D, NQ>::kSmemBytesBias : Cfg<D, NQ>::kSmemBytes;
     static_assert(smem <= 232448, "beyond the 227 KB a CTA may have");
     static std::atomic<bool> configured[64];
@@ -1090,12 +1252,13 @@ cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, 
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (kStaged && e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
     const int trq = (a.tr + NQ - 1) / NQ;
     const long long per_unit = static_cast<long long>(trq) * a.num_splits;
-    const long long ctas = static_cast<long long>(units) * per_unit;
+    const long long ctas = static_cast<long long>(units) * per_unit * (kStaged ? a.parts : 1);
     if (ctas <= 0 || ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     a.div_group_ctas = make_fastdiv(static_cast<uint32_t>(std::min<long long>(a.unit_group * per_unit, 0x7fffffffLL)));
     a.div_gsize = make_fastdiv(static_cast<uint32_t>(a.unit_group));
@@ -1109,23 +1272,34 @@ cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, 
     cfg.blockDim = dim3(Cfg<D, NQ>::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (kStaged) {
+        a.div_parts = make_fastdiv(static_cast<uint32_t>(a.parts));
+        a.div_pack = make_fastdiv(static_cast<uint32_t>(a.pack_rows));
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(a.parts);
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        if (a.parts > 1) cfg.numAttrs = 2;
+    }
     return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, a);
 }
 
 template <int D, int NQ, bool kBf16>
 cudaError_t launch_flags(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, int units, bool alibi, bool dropout, cudaStream_t stream) {
+    if (a.staged)  // (never with dropout)
+        return alibi ? launch_one<D, NQ, kBf16, true, false, true>(a, tq, tk, tv, to, units, stream)
+                     : launch_one<D, NQ, kBf16, false, false, true>(a, tq, tk, tv, to, units, stream);
     if (alibi) {
-        return dropout ? launch_one<D, NQ, kBf16, true, true>(a, tq, tk, tv, to, units, stream)
-                       : launch_one<D, NQ, kBf16, true, false>(a, tq, tk, tv, to, units, stream);
+        return dropout ? launch_one<D, NQ, kBf16, true, true, false>(a, tq, tk, tv, to, units, stream)
+                       : launch_one<D, NQ, kBf16, true, false, false>(a, tq, tk, tv, to, units, stream);
     }
-    return dropout ? launch_one<D, NQ, kBf16, false, true>(a, tq, tk, tv, to, units, stream)
-                   : launch_one<D, NQ, kBf16, false, false>(a, tq, tk, tv, to, units, stream);
+    return dropout ? launch_one<D, NQ, kBf16, false, true, false>(a, tq, tk, tv, to, units, stream)
+                   : launch_one<D, NQ, kBf16, false, false, false>(a, tq, tk, tv, to, units, stream);
 }
 
 template <int D, int NQ>
@@ -1135,16 +1309,66 @@ cudaError_t launch_dtype(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
                 : launch_flags<D, NQ, false>(a, tq, tk, tv, to, units, alibi, dropout, stream);
 }
 
+// two query tiles per CTA once a unit has more than one; a single tile (decode-like
+// shapes) keeps two independent CTAs per SM instead
+// (with two query tiles and a causal mask the pair would spend half its time on the diagonal tile that
+// only one of them can use: 277 against 308 TFLOP/s at [128,16,256,128])
+bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && !a.is_causal); }
+
 }  // namespace
+
+void plan_tiled(FwdArgs* a, int sms) {
+    a->parts = 1;
+    a->pack_rows = 0;
+    // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
+    // unit of heads * seqlen_q rows without a copy.  Done where it saves query tiles (a remainder per unit instead of
+    // one per head); a tile of several heads has every position, so it is not done for whole tiles, whose causal
+    // range is tighter.  (ALiBi slopes and the running pair's rows go by head.)
+    const int heads = a->kv_group;
+    if (heads > 1 && a->alibi_slopes == nullptr && a->accum_o == nullptr) {
+        const long long rows = static_cast<long long>(heads) * a->seqlen_q;
+        const long long packed = (rows + kTile - 1) / kTile;
+        if (packed < static_cast<long long>(heads) * a->tr && rows <= 0x3fffffffLL) {
+            a->pack_rows = a->seqlen_q;
+            a->seqlen_q = static_cast<int>(rows);
+            a->tr = static_cast<int>(packed);
+            a->units /= heads;
+            a->kv_group = 1;
+        }
+    }
+    // How many CTAs share the keys of a query block: as long as all of them find a place at once (one pair of query
+    // tiles an SM, or two single ones; a second wave of clusters waits for whole clusters to leave: [1 x 32 heads on 8,
+    // 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4), the split with the least time by
+    // a model fitted to sweeps of 4 to 128 blocks x 2 to 157 tiles: 1.6 us a KV tile (1.3 for a single query tile),
+    // 4.5 us + 0.25 a part for staging, two cluster barriers and the merge, whose distributed-shared-memory reads run
+    // at about 11 bytes a clock and SM; sixteen parts are slow to place.  [8 heads, 1021 x 1021] 4 parts 13.5 us
+    // against 20 unsplit, [16 units, 512 x 512, d = 64] 11.0 against 9.2, [8 blocks, 4000 keys, one tile] 8 parts 15.6
+    // against 51.6.
+    const bool pair = two_tiles(*a);
+    const long long blocks = static_cast<long long>(a->units) * (pair ? (a->tr + 1) / 2 : a->tr);
+    // KV tiles of the longest query block
+    long long n = a->tc;
+    if (a->window_left >= 0 && (a->window_right >= 0 || a->is_causal)) {
+        const long long rows = pair ? 2 * kTile : kTile, right = a->is_causal ? 0 : a->window_right;
+        n = std::min<long long>(n, (rows + a->window_left + right + kTile - 1) / kTile + 1);
+    }
+    const long long slots = pair ? sms : 2 * sms;
+    double best_t = 1e30;
+    for (int parts = 1; parts <= 16 && parts <= n; parts += parts < 8 ? 1 : 8) {
+        if (parts > 1 && blocks * parts > slots) break;
+        const double t = (pair ? 1.6 : 1.3) * static_cast<double>((n + parts - 1) / parts) +
+                         (parts == 1 ? 0.0 : parts <= 8 ? 4.5 + 0.25 * parts : 12.0);
+        if (t < best_t) { best_t = t; a->parts = parts; }
+    }
+    // (a running pair is merged by the unstaged epilogue, each query tile as it finishes)
+    if (a->accum_o != nullptr) a->parts = 1;
+    a->staged = a->parts > 1 || a->pack_rows > 0 || a->o_dim != a->head_dim;
+}
 
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const CUtensorMap& to, int units, bool bf16, bool dropout, cudaStream_t stream) {
     const bool alibi = a.alibi_slopes != nullptr;
-    // two query tiles per CTA once a unit has more than one; a single tile (decode-like
-    // shapes) keeps two independent CTAs per SM instead
-    // (with two query tiles and a causal mask the pair would spend half its time on the diagonal tile that
-    // only one of them can use: 277 against 308 TFLOP/s at [128,16,256,128])
-    const bool pair = a.tr > 2 || (a.tr == 2 && !a.is_causal);
+    const bool pair = two_tiles(a);
     if (a.head_dim <= 64) {
         return pair ? launch_dtype<64, 2>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream)
                     : launch_dtype<64, 1>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream);

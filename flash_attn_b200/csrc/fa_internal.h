@@ -55,10 +55,20 @@ struct FwdArgs {
     float* accum_lse;       // running log-sum-exp [units, Nq]
     int accum_first;        // nothing is carried yet: the running pair is only written
     int accum_final;        // last block: o / lse receive the merged result (the running O is then left as it is)
+    // The launches whose rows leave through shared memory (fwd_tiled_kernel with kStaged):
+    int staged;
+    int parts;              // CTAs (one cluster) that share the keys of a query block
+    int pack_rows;          // query rows per head when the heads of a K/V head are stacked into one unit, else 0
+    int o_dim;              // columns (and row pitch) of O: head_dim, or less when Q, K, V are padded copies
     // launch order of the CTAs (filled by launch_fwd_tiled): divisors of the block index
     FastDiv div_group_ctas, div_gsize, div_last_gsize, div_splits, div_kv_group;
+    FastDiv div_parts, div_pack;
     DropoutParams drop;
 };
+
+// Decides how a launch without dropout is cut (fills staged, parts and, for short grouped queries, restates the
+// problem with the heads of a K/V head stacked: units, heads, kv_group, seqlen_q, tr, pack_rows).
+void plan_tiled(FwdArgs* a, int sms);
 
 // Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O
 // (32-row boxes); it is read only when a.o_tma is set.
@@ -80,6 +90,7 @@ struct DecodeArgs {
     int subgroups;          // CTAs (each a part of the group's heads) per K/V unit
     int seqlen_q;           // query rows per unit, 1..8
     int seqlen_k, head_dim;
+    int o_dim;              // columns (and row pitch) of O: head_dim, or less when Q, K, V are padded copies
     int tc;                 // key tiles
     int vis_lo, vis_hi;     // key tiles that the masks leave visible to some query row: [vis_lo, vis_hi)
     int full_lo, full_hi;   // key tiles that no mask touches
@@ -106,6 +117,7 @@ struct CombineArgs {
     void* o; float* lse;
     long long rows_per_unit;   // Nq
     int num_splits, head_dim;
+    int o_dim;                 // columns (and row pitch) of O, at most head_dim
     int o_dtype;               // FA_DTYPE_*
 };
 cudaError_t launch_combine(const CombineArgs& a, long long units, cudaStream_t stream);
@@ -114,6 +126,9 @@ cudaError_t launch_merge(float* o_acc, float* lse_acc, const void* o_part, const
 cudaError_t launch_cast(const float* src, void* dst, int o_dtype, long long n, cudaStream_t stream);
 cudaError_t launch_repitch(const void* src, void* dst, int elem_bytes, long long rows, int d_src, int d_dst,
                            cudaStream_t stream);
+// Q, K and V (16-bit rows of d_src elements) to rows of d_dst, in one launch.
+cudaError_t launch_pad_qkv(const void* q, const void* k, const void* v, void* qp, void* kp, void* vp, long long rows_q,
+                           long long rows_k, int d_src, int d_dst, cudaStream_t stream);
 cudaError_t launch_dropout_mask(const FwdArgs& a, uint8_t* keep, long long units, cudaStream_t stream);
 
 }  // namespace fa

@@ -91,6 +91,30 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ float2 ld_cluster_f32x2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+// 16 bytes, or zeros where `take` is false.
+__device__ __forceinline__ float4 ld_cluster_f32x4_if(uint32_t addr, bool take) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "@p ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "r"(addr), "r"(take ? 1 : 0));
+    return v;
+}
+__device__ __forceinline__ float4 ld_shared_f32x4_if(uint32_t addr, bool take) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "r"(addr), "r"(take ? 1 : 0));
+    return v;
+}
 
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem() {

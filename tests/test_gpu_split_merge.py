@@ -1,0 +1,38 @@
+"""Query blocks whose keys are shared out over the CTAs of a cluster, and grouped queries stacked into common query
+tiles: few query blocks against many keys, so that every case is split.  Same tolerances as the unsplit kernel."""
+import pytest
+import torch
+
+import gpu_util
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [
+    dict(H=8, heads_k=2, Nq=130, Nk=3000, d=128, causal=True, q_pos0=2870),                  # stacked, tiles across heads
+    dict(H=4, Nq=100, Nk=2000, d=64, dtype="float16"),                                       # one query tile a unit
+    dict(H=6, heads_k=2, Nq=40, Nk=2500, d=128, causal=True, q_pos0=2460, window=(300, 0)),  # stacked, left window
+    dict(H=6, heads_k=2, Nq=43, Nk=900, d=64, q_pos0=400, window=(100, 60)),                 # stacked, both windows
+    dict(H=4, heads_k=2, Nq=300, Nk=2500, d=64, causal=True, q_pos0=2200, alibi=True),       # slopes go by head: not stacked
+    dict(H=2, Nq=257, Nk=1500, d=96, dtype="float16", window=(200, 100), q_pos0=600),
+    dict(H=8, heads_k=1, Nq=20, Nk=700, d=31, dtype="float16", out_dtype=torch.float32),     # padded rows, scalar stores
+    dict(H=2, Nq=400, Nk=2000, d=128, causal=True, q_pos0=50),                               # parts without a visible key
+    dict(H=4, Nq=384, Nk=1100, d=128, num_splits=3),
+    dict(H=2, Nq=9, Nk=1100, d=20, dtype="float16"),                                         # fewest rows, 4-byte rows of O
+])
+def test_split_and_stacked_blocks_match_the_oracle(case):
+    case = dict(case)
+    H, Nq, Nk, d = (case.pop(x) for x in ("H", "Nq", "Nk", "d"))
+    case.setdefault("num_splits", 0)
+    gpu_util.assert_close(gpu_util.run_case(1, H, Nq, Nk, d, seed=71, **case), str((H, Nq, Nk, d, case)))
+
+
+@pytest.mark.parametrize("Nq,Nk", [(1, 2000), (4, 2000), (40, 2000), (300, 2000)])
+def test_nan_reaches_its_rows_through_the_merge(Nq, Nk):
+    import flash_attn_b200 as fa
+    torch.manual_seed(5)
+    q, k, v = (torch.randn(1, 2, n, 128, device="cuda", dtype=torch.bfloat16) for n in (Nq, Nk, Nk))
+    q[0, 1, Nq - 1] = float("nan")
+    o, _ = fa.flash_attn_forward(q, k, v, num_splits=0)
+    assert torch.isnan(o[0, 1, Nq - 1]).all()
+    assert torch.isfinite(o[0, 0]).all() and torch.isfinite(o[0, 1, : Nq - 1]).all()
