@@ -361,7 +361,7 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
     constexpr int kStep = NQ * 4 * kPerWarp, kUnroll = 4;  // rows per CTA instruction; loads in flight
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int chunk = lane % kLanes, col = chunk * 4;
-    const bool aligned = a.o_dim % 8 == 0;  // (a padded problem's own rows start anywhere)
+    const bool aligned = a.o_dim % 8 == 0;
     for (int k0 = warp * kPerWarp + lane / kLanes; k0 < n_rows; k0 += kStep * kUnroll) {
         float4 acc[kUnroll];
 #pragma unroll
@@ -388,22 +388,41 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
                 }
             }
         }
+        if (aligned) {
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const int k = k0 + u * kStep;
-            if (k >= n_rows || col >= a.o_dim) continue;
-            const float4 o = acc[u];
-            const long long at = (row0 + k) * a.o_dim + col;
-            if (aligned) {
+            for (int u = 0; u < kUnroll; ++u) {
+                const int k = k0 + u * kStep;
+                if (k >= n_rows || col >= a.o_dim) continue;
+                const float4 o = acc[u];
+                const long long at = (row0 + k) * a.o_dim + col;
                 if (a.o_is_fp32) *reinterpret_cast<float4*>(static_cast<float*>(a.o) + at) = o;
                 else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.o) + at) = make_uint2(pack2<kBf16>(o.x, o.y), pack2<kBf16>(o.z, o.w));
-            } else {
-                const float e[4] = {o.x, o.y, o.z, o.w};
+            }
+        } else {
+            // a padded problem's own rows start anywhere: the finished rows go back to this CTA's own stage (nobody
+            // else reads these rows there) and leave element by element, neighbouring lanes to neighbouring elements
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (col + i >= a.o_dim) continue;
-                    if (a.o_is_fp32) static_cast<float*>(a.o)[at + i] = e[i];
-                    else static_cast<uint16_t*>(a.o)[at + i] = static_cast<uint16_t>(pack2<kBf16>(e[i], 0.0f));
+            for (int u = 0; u < kUnroll; ++u) {
+                const int row = r_lo + k0 + u * kStep;
+                if (k0 + u * kStep < n_rows)
+                    st_shared_v4(smem_base + C::kSmemK + row * (D * 4) + (chunk ^ (row & 7)) * 16, __float_as_uint(acc[u].x),
+                                 __float_as_uint(acc[u].y), __float_as_uint(acc[u].z), __float_as_uint(acc[u].w));
+            }
+            const unsigned lanes = kLanes == 32 ? 0xffffffffu : 0xffffu << (lane & 16);  // the lanes of this row
+            __syncwarp(lanes);
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const int k = k0 + u * kStep;
+                if (k >= n_rows) continue;
+                const int row = r_lo + k;
+                const float* src = reinterpret_cast<const float*>(smem_gen + C::kSmemK + row * (D * 4));
+                const long long at = (row0 + k) * a.o_dim;
+#pragma unroll
+                for (int c = chunk; c < D; c += kLanes) {
+                    if (c >= a.o_dim) continue;
+                    const float e = src[((c >> 2) ^ (row & 7)) * 4 + (c & 3)];
+                    if (a.o_is_fp32) static_cast<float*>(a.o)[at + c] = e;
+                    else static_cast<uint16_t*>(a.o)[at + c] = static_cast<uint16_t>(pack2<kBf16>(e, 0.0f));
                 }
             }
         }
@@ -1313,56 +1332,68 @@ cudaError_t launch_dtype(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
 // shapes) keeps two independent CTAs per SM instead
 // (with two query tiles and a causal mask the pair would spend half its time on the diagonal tile that
 // only one of them can use: 277 against 308 TFLOP/s at [128,16,256,128])
-bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && !a.is_causal); }
+// (tiles of stacked heads have no diagonal of their own)
+bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causal || a.pack_rows > 0)); }
+
+// How many CTAs share the keys of a query block, and the time that takes (us), by a model fitted to sweeps of 4 to 128
+// blocks x 2 to 157 KV tiles: 1.6 us a KV tile (a single query tile 1.3, with two on an SM 2.4) and 5 to start and
+// drain; the blocks of an unsplit launch that fills the device follow one another.  A split is taken only as long as all its CTAs find a place
+// at once (one pair of query tiles an SM, or two single ones; a second wave of clusters waits for whole clusters to
+// leave: [1 x 32 heads on 8, 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4); it pays
+// 4.5 us + 0.25 a part for staging, two cluster barriers and the merge, whose distributed-shared-memory reads run at
+// about 11 bytes a clock and SM; sixteen parts are slow to place.  [8 heads, 1021 x 1021] 4 parts 13.5 us against 20
+// unsplit, [16 units, 512 x 512, d = 64] 11.0 against 9.2, [8 blocks, 4000 keys, one tile] 8 parts 15.6 against 51.6.
+struct Split {
+    int parts;
+    double us;
+};
+Split best_split(const FwdArgs& a, int sms, bool staged) {
+    const bool pair = two_tiles(a);
+    const long long blocks = static_cast<long long>(a.units) * (pair ? (a.tr + 1) / 2 : a.tr);
+    long long n = a.tc;  // KV tiles of the longest query block
+    if (a.window_left >= 0 && (a.window_right >= 0 || a.is_causal)) {
+        const long long rows = pair ? 2 * kTile : kTile, right = a.is_causal ? 0 : a.window_right;
+        n = std::min<long long>(n, (rows + a.window_left + right + kTile - 1) / kTile + 1);
+    }
+    const long long slots = pair ? sms : 2 * sms;
+    auto tile_us = [&](int parts) { return pair ? 1.6 : blocks * parts > sms ? 2.4 : 1.3; };
+    Split best = {1, (tile_us(1) * n + 5.0 + (staged ? 4.0 : 0.0)) * std::max(1.0, static_cast<double>(blocks) / slots)};
+    for (int parts = 2; parts <= 16 && parts <= n && blocks * parts <= slots; parts += parts < 8 ? 1 : 8) {
+        const double us = tile_us(parts) * static_cast<double>((n + parts - 1) / parts) + 5.0 + (parts <= 8 ? 4.5 + 0.25 * parts : 12.0);
+        if (us < best.us) best = {parts, us};
+    }
+    return best;
+}
 
 }  // namespace
 
 void plan_tiled(FwdArgs* a, int sms) {
     a->parts = 1;
     a->pack_rows = 0;
+    a->staged = a->o_dim != a->head_dim;
+    if (a->accum_o != nullptr) return;  // (a running pair is merged by the unstaged epilogue, each query tile as it finishes)
+    Split split = best_split(*a, sms, a->staged != 0);
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
-    // unit of heads * seqlen_q rows without a copy.  Done where it saves query tiles (a remainder per unit instead of
-    // one per head); a tile of several heads has every position, so it is not done for whole tiles, whose causal
-    // range is tighter.  (ALiBi slopes and the running pair's rows go by head.)
+    // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the
+    // model says that it saves a tenth: below that the staged epilogue, slower than TMA stores, eats the gain ([64 heads
+    // on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.)
     const int heads = a->kv_group;
-    if (heads > 1 && a->alibi_slopes == nullptr && a->accum_o == nullptr) {
-        const long long rows = static_cast<long long>(heads) * a->seqlen_q;
-        const long long packed = (rows + kTile - 1) / kTile;
-        if (packed < static_cast<long long>(heads) * a->tr && rows <= 0x3fffffffLL) {
-            a->pack_rows = a->seqlen_q;
-            a->seqlen_q = static_cast<int>(rows);
-            a->tr = static_cast<int>(packed);
-            a->units /= heads;
-            a->kv_group = 1;
+    const long long rows = static_cast<long long>(heads) * a->seqlen_q;
+    if (heads > 1 && a->alibi_slopes == nullptr && rows <= 0x3fffffffLL) {
+        FwdArgs b = *a;
+        b.pack_rows = a->seqlen_q;
+        b.seqlen_q = static_cast<int>(rows);
+        b.tr = static_cast<int>((rows + kTile - 1) / kTile);
+        b.units = a->units / heads;
+        b.kv_group = 1;
+        const Split packed = best_split(b, sms, true);
+        if (b.tr < heads * a->tr && packed.us < 0.9 * split.us) {
+            *a = b;
+            split = packed;
         }
     }
-    // How many CTAs share the keys of a query block: as long as all of them find a place at once (one pair of query
-    // tiles an SM, or two single ones; a second wave of clusters waits for whole clusters to leave: [1 x 32 heads on 8,
-    // 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4), the split with the least time by
-    // a model fitted to sweeps of 4 to 128 blocks x 2 to 157 tiles: 1.6 us a KV tile (1.3 for a single query tile),
-    // 4.5 us + 0.25 a part for staging, two cluster barriers and the merge, whose distributed-shared-memory reads run
-    // at about 11 bytes a clock and SM; sixteen parts are slow to place.  [8 heads, 1021 x 1021] 4 parts 13.5 us
-    // against 20 unsplit, [16 units, 512 x 512, d = 64] 11.0 against 9.2, [8 blocks, 4000 keys, one tile] 8 parts 15.6
-    // against 51.6.
-    const bool pair = two_tiles(*a);
-    const long long blocks = static_cast<long long>(a->units) * (pair ? (a->tr + 1) / 2 : a->tr);
-    // KV tiles of the longest query block
-    long long n = a->tc;
-    if (a->window_left >= 0 && (a->window_right >= 0 || a->is_causal)) {
-        const long long rows = pair ? 2 * kTile : kTile, right = a->is_causal ? 0 : a->window_right;
-        n = std::min<long long>(n, (rows + a->window_left + right + kTile - 1) / kTile + 1);
-    }
-    const long long slots = pair ? sms : 2 * sms;
-    double best_t = 1e30;
-    for (int parts = 1; parts <= 16 && parts <= n; parts += parts < 8 ? 1 : 8) {
-        if (parts > 1 && blocks * parts > slots) break;
-        const double t = (pair ? 1.6 : 1.3) * static_cast<double>((n + parts - 1) / parts) +
-                         (parts == 1 ? 0.0 : parts <= 8 ? 4.5 + 0.25 * parts : 12.0);
-        if (t < best_t) { best_t = t; a->parts = parts; }
-    }
-    // (a running pair is merged by the unstaged epilogue, each query tile as it finishes)
-    if (a->accum_o != nullptr) a->parts = 1;
-    a->staged = a->parts > 1 || a->pack_rows > 0 || a->o_dim != a->head_dim;
+    a->parts = split.parts;
+    a->staged = a->staged || a->parts > 1 || a->pack_rows > 0;
 }
 
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,

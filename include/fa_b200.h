@@ -77,7 +77,10 @@ typedef struct fa_fwd_params {
     uint64_t unit0;           /* global b*H+h index of this call's first (batch, head) unit:
                                  keeps the dropout mask independent of how units are sharded  */
     int num_splits;           /* 0 = fa_num_splits_heuristic with the device's SM count,
-                                 1 = no split, n = forced                  (param.split_num) */
+                                 1 = no split, n = forced                  (param.split_num).
+                                 With dropout the count is part of the mask's geometry; without,
+                                 it only says what the workspace has to hold, and the kernels
+                                 share the keys out as suits the device                       */
     int64_t q_pos0, k_pos0;   /* global position of query row 0 / key column 0 (0 = reference
                                  behaviour; used to run one block of a sharded sequence)      */
     void* workspace;          /* device; split partials (param.O_tmp, param.L, param.M) */

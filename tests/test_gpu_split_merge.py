@@ -18,6 +18,8 @@ pytestmark = pytest.mark.gpu
     dict(H=8, heads_k=1, Nq=20, Nk=700, d=31, dtype="float16", out_dtype=torch.float32),     # padded rows, scalar stores
     dict(H=2, Nq=400, Nk=2000, d=128, causal=True, q_pos0=50),                               # parts without a visible key
     dict(H=4, Nq=384, Nk=1100, d=128, num_splits=3),
+    dict(H=16, heads_k=4, Nq=62, Nk=1300, d=128, causal=True, q_pos0=1238),                  # two stacked tiles, one pair
+    dict(H=128, Nq=257, Nk=300, d=100, dtype="float16", out_dtype=torch.float32),            # padded rows, unsplit
     dict(H=2, Nq=9, Nk=1100, d=20, dtype="float16"),                                         # fewest rows, 4-byte rows of O
 ])
 def test_split_and_stacked_blocks_match_the_oracle(case):
