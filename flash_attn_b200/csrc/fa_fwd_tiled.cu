@@ -1339,7 +1339,9 @@ bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causa
 // blocks x 2 to 157 KV tiles: 1.6 us a KV tile (a single query tile 1.3, with two on an SM 2.4) and 5 to start and
 // drain; the blocks of an unsplit launch that fills the device follow one another.  A split is taken only as long as all its CTAs find a place
 // at once (one pair of query tiles an SM, or two single ones; a second wave of clusters waits for whole clusters to
-// leave: [1 x 32 heads on 8, 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4); it pays
+// leave: [1 x 32 heads on 8, 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4;
+// [6 x 32 on 8, 62 rows, 2419 keys] is 48,
+// 46.7 at 3 each, 29.1 at 2; [2 x 32 on 8, 62 rows, 2419 keys] is 16, 40.3 at 8 each, 32.9 unsplit); it pays
 // 4.5 us + 0.25 a part for staging, two cluster barriers and the merge, whose distributed-shared-memory reads run at
 // about 11 bytes a clock and SM; sixteen parts are slow to place.  [8 heads, 1021 x 1021] 4 parts 13.5 us against 20
 // unsplit, [16 units, 512 x 512, d = 64] 11.0 against 9.2, [8 blocks, 4000 keys, one tile] 8 parts 15.6 against 51.6.
@@ -1358,7 +1360,9 @@ Split best_split(const FwdArgs& a, int sms, bool staged) {
     const long long slots = pair ? sms : 2 * sms;
     auto tile_us = [&](int parts) { return pair ? 1.6 : blocks * parts > sms ? 2.4 : 1.3; };
     Split best = {1, (tile_us(1) * n + 5.0 + (staged ? 4.0 : 0.0)) * std::max(1.0, static_cast<double>(blocks) / slots)};
-    for (int parts = 2; parts <= 16 && parts <= n && blocks * parts <= slots; parts += parts < 8 ? 1 : 8) {
+    for (int parts = 2; parts <= 16 && parts <= n; parts += parts < 8 ? 1 : 8) {
+        // (a cluster lies within a GPC: the larger it is, the more SMs stay without one)
+        if (blocks * parts > (parts == 2 ? slots : parts <= 4 || !pair ? slots * 9 / 10 : slots * 8 / 10)) break;
         const double us = tile_us(parts) * static_cast<double>((n + parts - 1) / parts) + 5.0 + (parts <= 8 ? 4.5 + 0.25 * parts : 12.0);
         if (us < best.us) best = {parts, us};
     }
