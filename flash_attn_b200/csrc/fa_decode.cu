@@ -39,6 +39,18 @@
 #include "fa_internal.h"
 #include "sm100_ptx.cuh"
 
+// Test build only (-DFA_TEST_SHORT_WAIT): the producer can be told to leave out the loads of one tile of the stream, so
+// that a consumer's bounded wait runs out and the give-up path can be checked without faulting or hanging anything.
+#ifdef FA_TEST_SHORT_WAIT
+__device__ int fa_test_decode_skip = -1;
+extern "C" int fa_test_skip_decode_tile(int t) {
+    return static_cast<int>(cudaMemcpyToSymbol(fa_test_decode_skip, &t, sizeof(int)));
+}
+#define FA_TEST_SKIPS(t) (fa_test_decode_skip == (t))
+#else
+#define FA_TEST_SKIPS(t) false
+#endif
+
 namespace fa {
 
 namespace {
@@ -278,6 +290,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 const int st = slot % kDStages;
                 const uint32_t ph = (slot / kDStages) & 1;
                 if (!mbar_wait(bar_empty + 8 * st, ph ^ 1, abort_flag)) return false;
+                if (FA_TEST_SKIPS(slot)) { ++slot; return true; }
                 mbar_expect_tx(bar_full + 8 * st, kDTileBytes);
 #pragma unroll
                 for (int b = 0; b < D / 64; ++b)
@@ -519,7 +532,6 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             for (int o = 16; o >= 1; o >>= 1) l_warp += __shfl_xor_sync(0xffffffffu, l_warp, o);
             if (lane == 0) red[8 * kH + warp * kH + n] = l_warp;
         }
-        named_barrier_128();
         uint32_t o_raw[kH];
 #pragma unroll
         for (int n = 0; n < kH; ++n) o_raw[n] = 0u;
@@ -532,6 +544,15 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 fail = 5;
             }
         }
+        named_barrier_128();
+        // A wait of this CTA gave up (the flag was set by whoever waited, before the barrier above): none of its columns
+        // may pass for the part of a softmax, so they and their sums are NaN, which the merges carry on; and the copies
+        // still in flight land first, since they write where the columns are staged.
+        const bool gave_up = *abort_flag != 0;
+        if (gave_up) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 200000) { }
+        }
         float m_col[kH];
 #pragma unroll
         for (int n = 0; n < kH; ++n) m_col[n] = __shfl_sync(0xffffffffu, m_ref, n);
@@ -541,11 +562,11 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             float* part_o = reinterpret_cast<float*>(smem_gen + C::kSmemRing);
 #pragma unroll
             for (int n = 0; n < kH; ++n) {
-                part_o[n * kTile + r] = __uint_as_float(o_raw[n]);
+                part_o[n * kTile + r] = gave_up ? __int_as_float(0x7fc00000) : __uint_as_float(o_raw[n]);
                 if (r == 0) {
                     const float l_sum = (red[8 * kH + n] + red[9 * kH + n]) + (red[10 * kH + n] + red[11 * kH + n]);
                     part_o[kH * kTile + 2 * n] = m_col[n];
-                    part_o[kH * kTile + 2 * n + 1] = fail == 0 ? l_sum : 0.0f;
+                    part_o[kH * kTile + 2 * n + 1] = gave_up ? __int_as_float(0x7fc00000) : l_sum;
                 }
             }
         } else {
@@ -559,7 +580,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 if (a.parts > 1) {  // partial of this part, for the combine kernel
                     const long long prow = ((unit + n / sq) * static_cast<long long>(a.parts) + part) * sq + n % sq;
                     if (r < a.head_dim) a.o_partial[prow * a.head_dim + r] = o_val;
-                    if (r == 0) a.lse_partial[prow] = lse_val;
+                    if (r == 0) a.lse_partial[prow] = gave_up ? __int_as_float(0x7fc00000) : lse_val;
                 } else {
                     store_result<kBf16>(a, (unit + n / sq) * static_cast<long long>(sq) + n % sq, r, o_val, lse_val);
                 }

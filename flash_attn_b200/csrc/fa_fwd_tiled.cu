@@ -1049,6 +1049,14 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             // un-normalised rows, maxima and sums go to shared memory (the ring is free once the MMAs of both
             // query tiles have completed, the Q tiles too); merge_rows below finishes them
             asm volatile("bar.sync 5, %0;" ::"n"(NQ * 128) : "memory");
+            // A wait of this CTA gave up (the flag was set by whoever waited, before the barrier above): none of its rows
+            // may pass for the part of a softmax, so every row sum is NaN, which the merge carries to O (and to
+            // LSE = -inf); and the copies still in flight land first, since they write where the rows are staged.
+            const bool gave_up = *abort_flag != 0;
+            if (gave_up) {
+                const long long t0 = clock64();
+                while (clock64() - t0 < 200000) { }
+            }
             const uint32_t stage = sK + (qi * kTile + r) * (D * 4);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -1067,7 +1075,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 }
             }
             *reinterpret_cast<float2*>(smem_gen + C::kSmemQ + (qi * kTile + r) * 8) =
-                make_float2(have_o ? m_ref : -INFINITY, have_o ? l_sum : 0.0f);
+                make_float2(have_o ? m_ref : -INFINITY, gave_up ? __int_as_float(0x7fc00000) : have_o ? l_sum : 0.0f);
         } else {
         float inv = 0.0f;
         if (l_sum > 0.0f) inv = (kDropout ? a.drop.inv_keep : 1.0f) / l_sum;

@@ -29,8 +29,11 @@ def test_lib():
     for name in ("fa_fwd", "fa_fwd_host"):
         getattr(L, name).argtypes = [pp]
         getattr(L, name).restype = ctypes.c_int
-    L.fa_test_skip_kv_tile.argtypes = [ctypes.c_int]
-    L.fa_test_skip_kv_tile.restype = ctypes.c_int
+    for name in ("fa_test_skip_kv_tile", "fa_test_skip_decode_tile"):
+        getattr(L, name).argtypes = [ctypes.c_int]
+        getattr(L, name).restype = ctypes.c_int
+    L.fa_fwd_workspace_bytes.argtypes = [pp]
+    L.fa_fwd_workspace_bytes.restype = ctypes.c_size_t
     return L
 
 
@@ -84,3 +87,45 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_stays_usable(test_lib):
     assert np.abs(lse.cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
     assert L.fa_fwd_host(ctypes.byref(_params(hq, hk, hv, ho, hl))) == 0
     assert np.abs(ho.float().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
+
+
+@pytest.mark.parametrize("skip,H,Hk,Nq,Nk,d", [
+    ("fa_test_skip_kv_tile", 8, 8, 256, 1100, 128),     # the parts of a query block, merged in their cluster
+    ("fa_test_skip_kv_tile", 8, 8, 100, 1100, 64),
+    ("fa_test_skip_decode_tile", 2, 2, 1, 1100, 128),   # decode: eight parts in a cluster, of which one gives up
+    ("fa_test_skip_decode_tile", 4, 1, 1, 65628, 64),   # ... and parts that the combine kernel merges
+])
+def test_a_part_that_gave_up_leaves_no_plausible_row(test_lib, skip, H, Hk, Nq, Nk, d):
+    """The other parts of the keys are complete, so only the part that gave up can keep the merged rows from looking
+    like a result: its sum is NaN."""
+    from flash_attn_b200 import _lib
+    L = test_lib
+    qh, kh, vh = synth.qkv(41, 1, H, Nq, Nk, d, "bfloat16")
+    kh, vh = np.ascontiguousarray(kh[:, :Hk]), np.ascontiguousarray(vh[:, :Hk])
+    q, k, v = (gpu_util.to_dev(x, "bfloat16") for x in (qh, kh, vh))
+    o = torch.zeros_like(q)
+    lse = torch.zeros((1, H, Nq), device="cuda", dtype=torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = _params(q, k, v, o, lse, status)
+    p.heads_k, p.num_splits = Hk, 0
+    need = L.fa_fwd_workspace_bytes(ctypes.byref(p))
+    ws = torch.empty(max(need, 16), device="cuda", dtype=torch.uint8)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    # tiled: the second KV tile of every CTA that has one; decode: a slot of the K/V stream that only the longest part has
+    tile = 1 if skip == "fa_test_skip_kv_tile" else 3 if Nk == 1100 else 17
+    try:
+        assert getattr(L, skip)(tile) == 0
+        assert L.fa_fwd(ctypes.byref(p)) == 0
+        torch.cuda.synchronize()
+        code = int(status.item())
+        assert (100 < code < 200) if Nq > 8 else (200 < code < 300), code
+        assert torch.isnan(o).all() and not torch.isfinite(lse).any()
+    finally:
+        assert getattr(L, skip)(-1) == 0
+    status.zero_()
+    assert L.fa_fwd(ctypes.byref(p)) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    want_o, want_lse = oracle_lib.forward(qh, np.repeat(kh, H // Hk, 1), np.repeat(vh, H // Hk, 1), d ** -0.5)
+    assert np.abs(o.float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
+    assert np.abs(lse.cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
