@@ -958,13 +958,16 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (__any_sync(0xffffffffu, rescale)) {
                 // P V of the previous tile has completed (its commit precedes s_full), so O is stable.
                 const float f = rescale ? factor : 1.0f;
+                // A row that has seen no key yet starts from zero, whatever the masked values left (0 * inf, 0 * NaN):
+                // where heads are stacked a query tile walks KV tiles past those of its rows.
+                const bool fresh = kStaged && rescale && m_ref == -INFINITY;
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c) {
                     uint32_t orow[32];
                     tmem_ld32(tmem_o + lane_base + c * 32, orow);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) orow[i] = __float_as_uint(__uint_as_float(orow[i]) * f);
+                    for (int i = 0; i < 32; ++i) orow[i] = fresh ? 0u : __float_as_uint(__uint_as_float(orow[i]) * f);
                     tmem_st32(tmem_o + lane_base + c * 32, orow);
                 }
             }
@@ -1388,10 +1391,13 @@ void plan_tiled(FwdArgs* a, int sms) {
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
     // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the
     // model says that it saves a tenth: below that the staged epilogue, slower than TMA stores, eats the gain ([64 heads
-    // on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.)
+    // on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.  A tile
+    // across heads walks the KV tiles of all of a head's positions; those past a row's own come first, and the row starts
+    // afresh behind them, but those before a left window would come last and bring masked infinities and NaN with them:
+    // with one, only heads of a single tile are stacked, whose rows walked all of these tiles anyway.)
     const int heads = a->kv_group;
     const long long rows = static_cast<long long>(heads) * a->seqlen_q;
-    if (heads > 1 && a->alibi_slopes == nullptr && rows <= 0x3fffffffLL) {
+    if (heads > 1 && a->alibi_slopes == nullptr && rows <= 0x3fffffffLL && (a->window_left < 0 || a->seqlen_q <= kTile)) {
         FwdArgs b = *a;
         b.pack_rows = a->seqlen_q;
         b.seqlen_q = static_cast<int>(rows);

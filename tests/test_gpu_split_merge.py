@@ -38,3 +38,20 @@ def test_nan_reaches_its_rows_through_the_merge(Nq, Nk):
     o, _ = fa.flash_attn_forward(q, k, v, num_splits=0)
     assert torch.isnan(o[0, 1, Nq - 1]).all()
     assert torch.isfinite(o[0, 0]).all() and torch.isfinite(o[0, 1, : Nq - 1]).all()
+
+
+@pytest.mark.parametrize("B,H,Hk,Nq,Nk,window,poisoned,rows", [
+    (1, 32, 8, 300, 8492, (-1, -1), slice(8448, 8492), slice(0, 256)),  # keys that only the last query tile of a head reaches
+    (8, 64, 8, 140, 1000, (300, 0), slice(0, 640), slice(128, 140)),    # ... that only the first one reaches
+])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_masked_values_stay_out_of_query_tiles_that_do_not_reach_them(B, H, Hk, Nq, Nk, window, poisoned, rows, value):
+    """V rows that are not finite (an unused part of a cache) reach the 128-row query tiles of a head that walk their KV
+    tile, as P = 0 times them, and no others, however the launch is cut."""
+    import flash_attn_b200 as fa
+    torch.manual_seed(6)
+    q, k, v = (torch.randn(B, h, n, 128, device="cuda", dtype=torch.bfloat16) for h, n in ((H, Nq), (Hk, Nk), (Hk, Nk)))
+    call = lambda: fa.flash_attn_forward(q, k, v, causal=True, window=window, q_pos0=Nk - Nq, num_splits=0)[0][:, :, rows]
+    clean = call()
+    v[:, :, poisoned] = value
+    assert torch.equal(call(), clean)
