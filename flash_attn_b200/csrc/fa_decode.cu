@@ -374,6 +374,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         // scores stay unscaled and the scale is folded into the exponent's FMA, except with ALiBi
         const bool alibi = a.alibi_slopes != nullptr;
         const float scale2 = a.scale_log2, exp_scale = alibi ? 1.0f : a.scale_log2;
+        float slope = 0.0f;  // ALiBi slope of column `lane`, handed round like the maxima
+        if (alibi && lane < nc) slope = a.alibi_slopes[(unit + lane / sq) % a.heads] * kDLog2e;
         float m_ref = -INFINITY;  // CTA-wide running max of column `lane` (lanes < kH of every warp), log2 units
         float l_part[kH];         // this thread's share of each column's row sum
 #pragma unroll
@@ -411,24 +413,29 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             }
             // masks and ALiBi, on the chunks that have any (the tiles [full_lo, full_hi) are visible whole)
             if (alibi || tile0 < a.full_lo || tile0 + nt > a.full_hi) {
+                int rel[kChunkTiles];      // key positions relative to query row 0, saturated far outside any window
+                bool in_range[kChunkTiles];
 #pragma unroll
                 for (int t = 0; t < kChunkTiles; ++t) {
                     const long long key = static_cast<long long>(tile0 + t) * kTile + r;
-                    const bool in_range = t < nt && key < a.seqlen_k;
-                    // key position relative to query row 0, saturated far outside any window
-                    const int rel = static_cast<int>(max(-0x40000000LL, min(a.k_pos0 + key - a.q_pos0, 0x40000000LL)));
+                    in_range[t] = t < nt && key < a.seqlen_k;
+                    rel[t] = static_cast<int>(max(-0x40000000LL, min(a.k_pos0 + key - a.q_pos0, 0x40000000LL)));
+                }
+                int q_row = 0;  // query row of column n, n % sq
 #pragma unroll
-                    for (int n = 0; n < kH; ++n) {
-                        const int ahead = rel - ((kH == 1) ? 0 : n % sq);  // > 0: the key lies after the query
-                        bool keep = in_range;
+                for (int n = 0; n < kH; ++n) {
+                    const float slope_n = alibi ? __shfl_sync(0xffffffffu, slope, n) : 0.0f;
+#pragma unroll
+                    for (int t = 0; t < kChunkTiles; ++t) {
+                        const int ahead = rel[t] - q_row;  // > 0: the key lies after the query
+                        bool keep = in_range[t];
                         if (a.is_causal && ahead > 0) keep = false;
                         if (a.window_left >= 0 && -ahead > a.window_left) keep = false;
                         if (a.window_right >= 0 && ahead > a.window_right) keep = false;
-                        if (alibi && n < nc)
-                            v[t][n] = fmaf(-(a.alibi_slopes[(unit + n / sq) % a.heads] * kDLog2e),
-                                           fabsf(static_cast<float>(ahead)), v[t][n] * scale2);
+                        if (alibi) v[t][n] = fmaf(-slope_n, fabsf(static_cast<float>(ahead)), v[t][n] * scale2);
                         if (!keep) v[t][n] = -INFINITY;
                     }
+                    if (++q_row == sq) q_row = 0;
                 }
             }
             float* red_c = red + buf * 4 * kH;
