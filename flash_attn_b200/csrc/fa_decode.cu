@@ -487,6 +487,25 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             m_ref = m_new;
             const float neg_lane = (m_new == -INFINITY) ? 0.0f : -m_new;
 
+            // Keep bits of this key, tile t's column n at bit 16 t + n.  The rows of a head share their draws (the reference's
+            // draw order gives one 8-row group the same: draw 64*tile_index + 8*(col/16) + 2*((col%16)/8) + col%2), so one
+            // Philox block per head and tile serves them all.
+            unsigned long long kept = 0ull;
+            if constexpr (kDropout) {
+#pragma unroll 1
+                for (int t = 0; t < nt; ++t) {
+                    const unsigned long long first = continuation(a.drop, n_tiles) +
+                                                     64ull * static_cast<unsigned long long>(c * kChunkTiles + t) + 8ull * (r >> 4);
+#pragma unroll 1
+                    for (int h = 0; h < gh; ++h) {
+                        const unsigned long long subseq = (a.drop.unit0 + unit + h) * static_cast<unsigned long long>(a.parts) +
+                                                          static_cast<unsigned long long>(part);
+                        const uint32_t bits = philox_keep4(a.drop, subseq, first);
+                        if ((bits >> (2 * ((r >> 3) & 1) + (r & 1))) & 1u) kept |= ((1ull << sq) - 1ull) << (16 * t + h * sq);
+                    }
+                }
+            }
+
 #pragma unroll
             for (int n = 0; n < kH; ++n) {
                 const float neg_m = __shfl_sync(0xffffffffu, neg_lane, n);
@@ -499,18 +518,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                         p[i] = ex2f(fmaf(v[t + i][n], exp_scale, neg_m));
                         l_part[n] += p[i];
                         if constexpr (kDropout) {
-                            if (n < nc && t + i < nt) {
-                                // reference draw order for query rows 0..7 (one 8-row group shares its draws):
-                                // draw 64*tile_index + 8*(col/16) + 2*((col%16)/8) + col%2
-                                const unsigned long long subseq =
-                                    (a.drop.unit0 + unit + n / sq) * static_cast<unsigned long long>(a.parts) +
-                                    static_cast<unsigned long long>(part);
-                                const unsigned long long first = continuation(a.drop, n_tiles) +
-                                                                 64ull * static_cast<unsigned long long>(c * kChunkTiles + t + i) +
-                                                                 8ull * (r >> 4);
-                                const uint32_t bits = philox_keep4(a.drop, subseq, first);
-                                if (!((bits >> (2 * ((r >> 3) & 1) + (r & 1))) & 1u)) p[i] = 0.0f;
-                            }
+                            if (!((kept >> (16 * (t + i) + n)) & 1ull)) p[i] = 0.0f;
                         }
                     }
                     uint32_t h;  // the two tiles' elements, rounded together

@@ -78,3 +78,14 @@ def test_decode_config4_shape_sampled_units():
 def test_parts_of_a_unit_and_query_columns(H, Hk, Nq, nk, d, dtype, kw):
     gpu_util.assert_close(gpu_util.run_case(1, H, Nq, nk, d, dtype, seed=58, causal=True, q_pos0=nk - Nq, heads_k=Hk, **kw),
                           f"{H}/{Hk} heads, {Nq} rows, {nk} keys, d={d} {kw}")
+
+
+@pytest.mark.parametrize("H,Hk,Nq,nk,kw", [
+    (8, 2, 4, 700, {}),                                   # 4 heads x 4 rows of a K/V head, a ragged last chunk
+    (10, 2, 3, 300, dict(offset=6)),                      # 5 heads x 3 rows, draws that straddle two Philox blocks
+    (2, 2, 6, 1100, dict(num_splits=3)),                  # one head's rows share their draws
+    (16, 2, 1, 600, dict(num_splits=2, launch_index=3)),  # 8 heads, a later launch of a loop
+])
+def test_dropout_of_query_rows_and_heads_that_share_keys(H, Hk, Nq, nk, kw):
+    gpu_util.assert_close(gpu_util.run_case(2, H, Nq, nk, 64, "bfloat16", seed=59, causal=True, q_pos0=nk - Nq, heads_k=Hk,
+                                            p_dropout=0.25, drop_seed=7, **kw), f"{H}/{Hk} heads, {Nq} rows, {nk} keys {kw}")
