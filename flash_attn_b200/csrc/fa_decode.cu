@@ -226,6 +226,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         gh = min(heads_per_cta, a.kv_group - sub * heads_per_cta);  // query heads of this CTA
     }
     const int nc = gh * sq;  // columns in use: column n = head n / sq, query row n % sq
+    const long long row0 = static_cast<long long>(unit) * sq;  // column n is row row0 + n of Q, O and LSE
 
     // KV tiles of this part.  With dropout the parts are the caller's splits, whose tile ranges are part of
     // the dropout streams' geometry; otherwise the visible tiles are dealt out evenly.
@@ -268,7 +269,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             uint4 val = make_uint4(0u, 0u, 0u, 0u);
             if (n < nc && u * 8 < a.head_dim)
                 val = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) +
-                                                      (static_cast<long long>(unit) * sq + n) * a.head_dim + u * 8);
+                                                      (row0 + n) * a.head_dim + u * 8);
             *reinterpret_cast<uint4*>(smem_gen + C::kSmemQ + (u >> 3) * C::kHalfBytes + n * 128 + (((u & 7) ^ (n & 7)) << 4)) = val;
         }
         fence_proxy_async_smem();
@@ -585,6 +586,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 }
             }
         } else {
+            long long prow = (unit * static_cast<long long>(a.parts) + part) * sq;  // row of column n in the partials
+            int q_row = 0;
 #pragma unroll
             for (int n = 0; n < kH; ++n) {
                 if (n >= nc) continue;
@@ -593,11 +596,15 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 const float lse_val = l_sum > 0.0f ? m_col[n] * kDLn2 + __logf(l_sum) : -INFINITY;
                 const float o_val = __uint_as_float(o_raw[n]) * inv;
                 if (a.parts > 1) {  // partial of this part, for the combine kernel
-                    const long long prow = ((unit + n / sq) * static_cast<long long>(a.parts) + part) * sq + n % sq;
                     if (r < a.head_dim) a.o_partial[prow * a.head_dim + r] = o_val;
                     if (r == 0) a.lse_partial[prow] = gave_up ? __int_as_float(0x7fc00000) : lse_val;
+                    ++prow;
+                    if (++q_row == sq) {  // the next head's partials
+                        q_row = 0;
+                        prow += static_cast<long long>(a.parts - 1) * sq;
+                    }
                 } else {
-                    store_result<kBf16>(a, (unit + n / sq) * static_cast<long long>(sq) + n % sq, r, o_val, lse_val);
+                    store_result<kBf16>(a, row0 + n, r, o_val, lse_val);
                 }
             }
         }
@@ -659,8 +666,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                     }
                 }
                 const float inv = l > 0.0f ? a.drop.inv_keep / l : 0.0f;
-                store_result<kBf16>(a, (unit + n / sq) * static_cast<long long>(sq) + n % sq, r, o * inv,
-                                    l > 0.0f ? m * kDLn2 + __logf(l) : -INFINITY);
+                store_result<kBf16>(a, row0 + n, r, o * inv, l > 0.0f ? m * kDLn2 + __logf(l) : -INFINITY);
             }
             __syncwarp();
         }
