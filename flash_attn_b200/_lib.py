@@ -14,7 +14,7 @@ FA_OK = 0
 FA_ACCUM_FIRST, FA_ACCUM_FINAL = 1, 2
 
 #: every symbol include/fa_b200.h declares
-EXPORTS = ["fa_fwd", "fa_fwd_workspace_bytes", "fa_fwd_resolve_splits", "fa_num_splits_heuristic",
+EXPORTS = ["fa_fwd", "fa_fwd_workspace_bytes", "fa_fwd_resolve_splits", "fa_fwd_plan", "fa_num_splits_heuristic",
            "fa_dropout_mask", "fa_merge_partial", "fa_cast_output", "fa_fwd_host", "fa_fwd_host_release",
            "fa_fwd_static_scratch", "fa_static_scratch_bytes", "fa_launch_reference_params", "fa_strerror", "fa_version",
            "fa_ring_fwd", "fa_ring_message_bytes", "fa_ring_unique_id", "fa_ring_comm_create", "fa_ring_comm_destroy"]
@@ -67,6 +67,11 @@ class _ParamsArg:
     @classmethod
     def from_param(cls, x):
         return ctypes.c_char_p.from_param(x) if type(x) is bytes else ctypes.POINTER(FwdParams).from_param(x)
+
+
+class FwdPlan(ctypes.Structure):
+    """struct fa_fwd_plan_info"""
+    _fields_ = [(n, ctypes.c_int) for n in ("decode", "parts", "merged", "columns", "staged", "stacked_rows")]
 
 
 class RingParams(ctypes.Structure):
@@ -135,6 +140,8 @@ def load():
     L.fa_launch_reference_params.restype = ctypes.c_int
     L.fa_fwd_workspace_bytes.argtypes = [pp]
     L.fa_fwd_workspace_bytes.restype = ctypes.c_size_t
+    L.fa_fwd_plan.argtypes = [pp, ctypes.c_int, ctypes.POINTER(FwdPlan)]
+    L.fa_fwd_plan.restype = ctypes.c_int
     L.fa_fwd_resolve_splits.argtypes = [pp]
     L.fa_fwd_resolve_splits.restype = ctypes.c_int
     L.fa_num_splits_heuristic.argtypes = [ctypes.c_int] * 5

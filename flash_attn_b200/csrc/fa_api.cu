@@ -372,6 +372,39 @@ int fa_fwd_resolve_splits(const fa_fwd_params* p) {
     return resolve_splits(p, sms);
 }
 
+int fa_fwd_plan(const fa_fwd_params* p, int num_sms, fa_fwd_plan_info* plan) {
+    int rc = validate(p);
+    if (rc != FA_OK) return rc;
+    if (!plan || num_sms < 1) return FA_ERR_INVALID_ARG;
+    const int splits = resolve_splits(p, num_sms);
+    fa_fwd_params q = *p;
+    q.head_dim = (p->head_dim + 7) / 8 * 8;
+    FwdArgs a;
+    fill_args(&q, splits, &a);
+    std::memset(plan, 0, sizeof(*plan));
+    if (p->seqlen_q <= 8 && p->accum_o == nullptr) {
+        DecodeArgs d;
+        fill_decode_args(&q, a, &d);
+        plan_decode(&d, p->batch * p->heads, splits, p->num_splits > 0, num_sms);
+        plan->decode = 1;
+        plan->parts = d.parts;
+        plan->merged = d.merge;
+        plan->columns = d.columns;
+        return FA_OK;
+    }
+    if (p->p_dropout > 0.0f) {
+        plan->parts = splits;
+        return FA_OK;
+    }
+    a.o_dim = p->head_dim;
+    plan_tiled(&a, num_sms);
+    plan->parts = a.parts;
+    plan->merged = a.parts > 1;
+    plan->staged = a.staged;
+    plan->stacked_rows = a.pack_rows;
+    return FA_OK;
+}
+
 size_t fa_fwd_workspace_bytes(const fa_fwd_params* p) {
     int s = fa_fwd_resolve_splits(p);
     if (s < 1) return 0;

@@ -130,6 +130,25 @@ struct TileRange {
     int lo, hi;  // KV tiles [lo, hi)
 };
 
+// The KV tiles of [lo, hi) that the masks leave visible to queries at positions q0 .. q1.
+__host__ __device__ __forceinline__ TileRange clip_tiles(const FwdArgs& a, long long q0, long long q1, int lo, int hi) {
+    const long long tc = a.tc;
+    if (a.window_left >= 0) {  // src/flash_forward.h:39
+        const long long w = (q0 - a.window_left - a.k_pos0) / kTile;  // truncating, like the reference
+        lo = max(lo, static_cast<int>(max(0LL, min(w, tc))));
+    }
+    if (a.window_right >= 0) {  // src/flash_forward.h:42-44
+        const long long last = q1 + a.window_right - a.k_pos0;
+        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, tc)));
+    }
+    if (a.is_causal) {  // src/flash_forward.h:46-48
+        const long long last = q1 - a.k_pos0;
+        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, tc)));
+    }
+    if (hi < lo) hi = lo;
+    return {lo, hi};
+}
+
 template <bool kStaged>
 __device__ __forceinline__ TileRange kv_tile_range(const FwdArgs& a, int rb, int split) {
     if (rb >= a.tr) return {0, 0};
@@ -142,26 +161,12 @@ __device__ __forceinline__ TileRange kv_tile_range(const FwdArgs& a, int rb, int
         first = h0 == h1 ? first - h0 * a.pack_rows : 0;
         last_row = h0 == h1 ? last_row - h0 * a.pack_rows : a.pack_rows - 1;
     }
-    const long long q0 = a.q_pos0 + first, q1 = a.q_pos0 + last_row;
     int lo = 0, hi = a.tc;
     if (!kStaged && a.num_splits > 1) {  // src/flash_forward_splitkv.h:40-43
         lo = a.tiles_per_split * split;
         hi = min(lo + a.tiles_per_split, a.tc);
     }
-    if (a.window_left >= 0) {  // src/flash_forward.h:39
-        const long long w = (q0 - a.window_left - a.k_pos0) / kTile;  // truncating, like the reference
-        lo = max(lo, static_cast<int>(max(0LL, min(w, static_cast<long long>(a.tc)))));
-    }
-    if (a.window_right >= 0) {  // src/flash_forward.h:42-44
-        const long long last = q1 + a.window_right - a.k_pos0;
-        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
-    }
-    if (a.is_causal) {  // src/flash_forward.h:46-48
-        const long long last = q1 - a.k_pos0;
-        hi = min(hi, last < 0 ? 0 : static_cast<int>(min(last / kTile + 1, static_cast<long long>(a.tc))));
-    }
-    if (hi < lo) hi = lo;
-    return {lo, hi};
+    return clip_tiles(a, a.q_pos0 + first, a.q_pos0 + last_row, lo, hi);
 }
 
 template <bool kBf16>
@@ -1360,14 +1365,33 @@ struct Split {
     int parts;
     double us;
 };
+// KV tiles that query block `qb` (two query tiles if `pair`) walks, as kv_tile_range has it.
+int block_tiles(const FwdArgs& a, long long qb, bool pair) {
+    int lo = a.tc, hi = 0;
+    for (long long rb = pair ? 2 * qb : qb; rb < (pair ? 2 * qb + 2 : qb + 1) && rb < a.tr; ++rb) {
+        long long first = rb * kTile, last = first + kTile - 1;
+        if (a.pack_rows > 0) {
+            last = std::min<long long>(last, a.seqlen_q - 1);
+            const bool one_head = first / a.pack_rows == last / a.pack_rows;
+            first = one_head ? first % a.pack_rows : 0;
+            last = one_head ? last % a.pack_rows : a.pack_rows - 1;
+        }
+        const TileRange r = clip_tiles(a, a.q_pos0 + first, a.q_pos0 + last, 0, a.tc);
+        if (r.hi > r.lo) {
+            lo = std::min(lo, r.lo);
+            hi = std::max(hi, r.hi);
+        }
+    }
+    return std::max(hi - lo, 0);
+}
+
 Split best_split(const FwdArgs& a, int sms, bool staged) {
     const bool pair = two_tiles(a);
-    const long long blocks = static_cast<long long>(a.units) * (pair ? (a.tr + 1) / 2 : a.tr);
-    long long n = a.tc;  // KV tiles of the longest query block
-    if (a.window_left >= 0 && (a.window_right >= 0 || a.is_causal)) {
-        const long long rows = pair ? 2 * kTile : kTile, right = a.is_causal ? 0 : a.window_right;
-        n = std::min<long long>(n, (rows + a.window_left + right + kTile - 1) / kTile + 1);
-    }
+    const long long per_unit = pair ? (a.tr + 1) / 2 : a.tr;
+    const long long blocks = a.units * per_unit;
+    // KV tiles of the longest query block.  (The masks and not the length of K decide: a prompt written into a longer cache
+    // sees its beginning only.  The count rises or falls along a unit's blocks, or is cut off at both of its ends.)
+    const int n = std::max(block_tiles(a, per_unit / 2, pair), std::max(block_tiles(a, 0, pair), block_tiles(a, per_unit - 1, pair)));
     const long long slots = pair ? sms : 2 * sms;
     auto tile_us = [&](int parts) { return pair ? 1.6 : blocks * parts > sms ? 2.4 : 1.3; };
     Split best = {1, (tile_us(1) * n + 5.0 + (staged ? 4.0 : 0.0)) * std::max(1.0, static_cast<double>(blocks) / slots)};

@@ -138,6 +138,18 @@ size_t fa_fwd_workspace_bytes(const fa_fwd_params* p);
  * the kernels may divide the keys among more or fewer CTAs than that, as suits the device. */
 int fa_fwd_resolve_splits(const fa_fwd_params* p);
 
+/* How fa_fwd would cut p on a device of num_sms SMs (host arithmetic only; the pointers of p are not followed).
+ * Of use to whoever wants to know why a shape takes the time it takes, and to the tests. */
+typedef struct fa_fwd_plan_info {
+    int decode;               /* 1: the kernel for seqlen_q <= 8, 0: the tiled kernel */
+    int parts;                /* CTAs that share the keys of a query block (decode: of a unit) */
+    int merged;               /* the parts are one cluster and merge on chip (0 with parts > 1: the combine kernel) */
+    int columns;              /* decode: query columns of a CTA */
+    int staged;               /* tiled: finished rows leave through shared memory */
+    int stacked_rows;         /* tiled: the heads of a K/V head are stacked into one unit, this many rows each; 0 = not */
+} fa_fwd_plan_info;
+int fa_fwd_plan(const fa_fwd_params* p, int num_sms, fa_fwd_plan_info* plan);
+
 /* The reference's split policy, same arguments and result as
  * num_splits_heuristic (src/main.cu:391-422). */
 int fa_num_splits_heuristic(int batch_nheads_mblocks, int num_sms, int num_n_blocks, int max_splits,

@@ -1,0 +1,20 @@
+"""fa_fwd_plan for a shape, as a FwdPlan: how the library would cut the call on a B200 (148 SMs unless told otherwise)."""
+import ctypes
+
+from flash_attn_b200 import _lib
+
+
+def plan(B, H, Nq, Nk, d, heads_k=0, causal=False, window=(-1, -1), alibi=False, p_dropout=0.0, num_splits=0, q_pos0=0,
+         k_pos0=0, fp32_out=False, sms=148):
+    p = _lib.FwdParams()
+    p.q = p.k = p.v = p.o = 4096  # (not followed)
+    p.batch, p.heads, p.heads_k, p.seqlen_q, p.seqlen_k, p.head_dim = B, H, heads_k, Nq, Nk, d
+    p.dtype = _lib.FA_DTYPE_BF16
+    p.o_dtype = _lib.FA_DTYPE_FP32 if fp32_out else p.dtype
+    p.softmax_scale, p.is_causal, p.window_left, p.window_right = d ** -0.5, int(causal), *window
+    p.alibi_slopes = 4096 if alibi else None
+    p.p_dropout, p.num_splits, p.q_pos0, p.k_pos0 = p_dropout, num_splits, q_pos0, k_pos0
+    out = _lib.FwdPlan()
+    rc = _lib.load().fa_fwd_plan(ctypes.byref(p), sms, ctypes.byref(out))
+    assert rc == 0, _lib.strerror(rc)
+    return out

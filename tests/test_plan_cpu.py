@@ -1,0 +1,35 @@
+"""How a call is cut (fa_fwd_plan, host arithmetic): the plan goes by the keys that the masks leave visible."""
+import pytest
+
+from plan_util import plan
+
+
+@pytest.mark.parametrize("B,H,Hk,Nq,Nk,kw", [
+    (1, 16, 16, 256, 8192, {}),              # a prompt written into a longer cache: two KV tiles are visible
+    (1, 32, 8, 512, 32768, {}),
+    (1, 32, 8, 300, 32768, {}),
+    (1, 32, 8, 300, 8492, {}),
+    (8, 32, 8, 22, 2839, {}),
+    (1, 16, 16, 256, 8192, dict(k_pos0=8000, q_pos0=8000)),
+    (1, 16, 16, 256, 8192, dict(causal=False, window=(-1, 0))),    # a right window alone bounds it as well
+])
+def test_keys_that_no_query_sees_do_not_count(B, H, Hk, Nq, Nk, kw):
+    got = plan(B, H, Nq, Nk, 128, heads_k=Hk, **dict(dict(causal=True), **kw))
+    assert (got.decode, got.parts, got.staged, got.stacked_rows) == (0, 1, 0, 0)
+
+
+def test_the_same_blocks_at_the_end_of_the_cache_are_cut():
+    assert plan(1, 16, 256, 8192, 128, causal=True, q_pos0=7936).parts > 1
+    got = plan(1, 32, 300, 8492, 128, heads_k=8, causal=True, q_pos0=8192)
+    assert got.parts > 1 and got.merged == 1 and got.stacked_rows == 300
+
+
+@pytest.mark.parametrize("kw", [dict(causal=True), dict(causal=True, window=(300, 0)), dict(window=(100, 60))])
+def test_the_plan_of_a_block_is_that_of_its_visible_keys(kw):
+    # (cut off at the last visible key, the cache gives the same plan; positions on both sides of the tiles' edges)
+    for q0 in (0, 127, 128, 1000, 3000):
+        for Nq in (9, 128, 129, 300):
+            right = kw["window"][1] if kw.get("window", (-1, -1))[1] >= 0 else 0
+            whole = plan(1, 8, Nq, 9000, 64, heads_k=2, q_pos0=q0, **kw)
+            short = plan(1, 8, Nq, (q0 + Nq + 255) // 128 * 128 + (right + 127) // 128 * 128, 64, heads_k=2, q_pos0=q0, **kw)
+            assert bytes(whole) == bytes(short), (q0, Nq, kw)
