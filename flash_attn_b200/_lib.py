@@ -140,7 +140,7 @@ def load():
     L.fa_launch_reference_params.restype = ctypes.c_int
     L.fa_fwd_workspace_bytes.argtypes = [pp]
     L.fa_fwd_workspace_bytes.restype = ctypes.c_size_t
-    L.fa_fwd_plan.argtypes = [pp, ctypes.c_int, ctypes.POINTER(FwdPlan)]
+    L.fa_fwd_plan.argtypes = [pp, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(FwdPlan)]
     L.fa_fwd_plan.restype = ctypes.c_int
     L.fa_fwd_resolve_splits.argtypes = [pp]
     L.fa_fwd_resolve_splits.restype = ctypes.c_int

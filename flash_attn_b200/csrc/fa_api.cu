@@ -260,7 +260,7 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
         // how the keys are shared out is the library's business; the parts of a query block merge on chip
         a.num_splits = parts = 1;
         a.tiles_per_split = a.tc;
-        plan_tiled(&a, sms);
+        plan_tiled(&a, sms, cluster_room(sms));
     }
     if (decode) {
         fill_decode_args(p, a, &d);
@@ -372,10 +372,12 @@ int fa_fwd_resolve_splits(const fa_fwd_params* p) {
     return resolve_splits(p, sms);
 }
 
-int fa_fwd_plan(const fa_fwd_params* p, int num_sms, fa_fwd_plan_info* plan) {
+int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd_plan_info* plan) {
     int rc = validate(p);
     if (rc != FA_OK) return rc;
     if (!plan || num_sms < 1) return FA_ERR_INVALID_ARG;
+    ClusterRoom room = {};
+    for (int i = 1; i <= ClusterRoom::kMax; ++i) room.one_per_sm[i] = i == 1 ? num_sms : clusters ? clusters[i] : 0;
     const int splits = resolve_splits(p, num_sms);
     fa_fwd_params q = *p;
     q.head_dim = (p->head_dim + 7) / 8 * 8;
@@ -397,7 +399,7 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, fa_fwd_plan_info* plan) {
         return FA_OK;
     }
     a.o_dim = p->head_dim;
-    plan_tiled(&a, num_sms);
+    plan_tiled(&a, num_sms, room);
     plan->parts = a.parts;
     plan->merged = a.parts > 1;
     plan->staged = a.staged;

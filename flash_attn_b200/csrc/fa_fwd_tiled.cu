@@ -30,6 +30,8 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
+#include <mutex>
 #include <type_traits>
 #include "fa_internal.h"
 #include "sm100_ptx.cuh"
@@ -1351,19 +1353,32 @@ cudaError_t launch_dtype(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
 // (tiles of stacked heads have no diagonal of their own)
 bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causal || a.pack_rows > 0)); }
 
-// How many CTAs share the keys of a query block, and the time that takes (us), by a model fitted to sweeps of 4 to 128
-// blocks x 2 to 157 KV tiles: 1.6 us a KV tile (a single query tile 1.3, with two on an SM 2.4) and 5 to start and
-// drain; the blocks of an unsplit launch that fills the device follow one another.  A split is taken only as long as all its CTAs find a place
-// at once (one pair of query tiles an SM, or two single ones; a second wave of clusters waits for whole clusters to
-// leave: [1 x 32 heads on 8, 300 rows, 8492 keys] is 40 blocks, 117 us unsplit, 51 at 3 CTAs each, 78 at 4;
-// [6 x 32 on 8, 62 rows, 2419 keys] is 48,
-// 46.7 at 3 each, 29.1 at 2; [2 x 32 on 8, 62 rows, 2419 keys] is 16, 40.3 at 8 each, 32.9 unsplit); it pays
-// 4.5 us + 0.25 a part for staging, two cluster barriers and the merge, whose distributed-shared-memory reads run at
-// about 11 bytes a clock and SM; sixteen parts are slow to place.  [8 heads, 1021 x 1021] 4 parts 13.5 us against 20
-// unsplit, [16 units, 512 x 512, d = 64] 11.0 against 9.2, [8 blocks, 4000 keys, one tile] 8 parts 15.6 against 51.6.
+// How many CTAs share the keys of a query block, and the time that takes (us).  The model is fitted to sweeps over 4 to 160
+// blocks x 4 to 67 KV tiles with every part count (D = 128 and 64, two query tiles a CTA and one) and over 81 grouped shapes with and
+// without stacking: what it takes is 1 % slower than the best on average.  Where it leaves more than a tenth, blocks do not
+// fit the device at once ([160 blocks, 67 tiles] 231 us unsplit, 203 in three parts and four waves).
+//   A CTA takes `base` to start and drain and `rate` for a KV tile.  The rate grows with the CTAs at work: by `crowd` up to one an
+//   SM (L2 and HBM; grouped queries share their K/V), by `over` for a second one on the SM (single query tiles only).
+//   A split pays `merge` + `merge_each` a part for staging, two cluster barriers and the merge (its distributed-shared-memory
+//   reads run at about 11 bytes a clock and SM), part counts that are no power of two a little more, few rows less.
+//   It is taken only where all its clusters are resident at once (ClusterRoom): a second wave waits for whole clusters to
+//   leave.  [16 blocks, 19 tiles] 34.0 unsplit, 20.6 / 20.5 / 22.2 / 40.3 in 4 / 5 / 6 / 7 parts (15 clusters of 7 fit),
+//   [48 blocks, 67 tiles] 107 unsplit, 70.8 / 96.6 in 2 / 3 (45 clusters of 3 fit).
+struct Cost {
+    double base, rate, crowd, over, merge, merge_each;
+};
+constexpr Cost kCost[2][2] = {  // [two query tiles][D = 128]
+    {{3.2, 1.05, 0.45, 0.35, 2.9, 0.23}, {3.6, 1.25, 0.95, 0.45, 5.1, 0.30}},
+    {{4.2, 1.46, 0.08, 0.0, 3.4, 0.35}, {4.9, 1.45, 0.40, 0.0, 4.4, 0.75}},
+};
+double launch_us(const Cost& c, double ctas, int sms, double tiles) {
+    const double f = ctas / sms, g = std::min(1.0, f), second = std::max(0.0, f - 1.0);
+    return c.base + 1.5 * second + (c.rate + c.crowd * g * std::sqrt(g) + c.over * second) * tiles;
+}
 struct Split {
     int parts;
     double us;
+    bool even;  // the query blocks are of about one length
 };
 // KV tiles that query block `qb` (two query tiles if `pair`) walks, as kv_tile_range has it.
 int block_tiles(const FwdArgs& a, long long qb, bool pair) {
@@ -1385,40 +1400,120 @@ int block_tiles(const FwdArgs& a, long long qb, bool pair) {
     return std::max(hi - lo, 0);
 }
 
-Split best_split(const FwdArgs& a, int sms, bool staged) {
+Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged) {
     const bool pair = two_tiles(a);
+    Cost c = kCost[pair][a.head_dim > 64];
+    if (pair && (a.kv_group > 1 || a.pack_rows > 0)) c.crowd = std::min(c.crowd, 0.1);
+    if (a.alibi_slopes != nullptr && !a.is_causal && a.window_right != 0) c.rate *= 1.6;  // (a bias per element)
     const long long per_unit = pair ? (a.tr + 1) / 2 : a.tr;
-    const long long blocks = a.units * per_unit;
-    // KV tiles of the longest query block.  (The masks and not the length of K decide: a prompt written into a longer cache
-    // sees its beginning only.  The count rises or falls along a unit's blocks, or is cut off at both of its ends.)
-    const int n = std::max(block_tiles(a, per_unit / 2, pair), std::max(block_tiles(a, 0, pair), block_tiles(a, per_unit - 1, pair)));
-    const long long slots = pair ? sms : 2 * sms;
-    auto tile_us = [&](int parts) { return pair ? 1.6 : blocks * parts > sms ? 2.4 : 1.3; };
-    Split best = {1, (tile_us(1) * n + 5.0 + (staged ? 4.0 : 0.0)) * std::max(1.0, static_cast<double>(blocks) / slots)};
-    for (int parts = 2; parts <= 16 && parts <= n; parts += parts < 8 ? 1 : 8) {
-        // (a cluster lies within a GPC: the larger it is, the more SMs stay without one)
-        if (blocks * parts > (parts == 2 ? slots : parts <= 4 || !pair ? slots * 9 / 10 : slots * 8 / 10)) break;
-        const double us = tile_us(parts) * static_cast<double>((n + parts - 1) / parts) + 5.0 + (parts <= 8 ? 4.5 + 0.25 * parts : 12.0);
-        if (us < best.us) best = {parts, us};
+    const long long blocks = a.units * per_unit, slots = pair ? sms : 2 * sms;
+    // KV tiles of a unit's query blocks, on at most nine of them.  (The masks and not the length of K decide: a prompt written
+    // into a longer cache sees its beginning only.)
+    int n = a.tc, least = a.tc;
+    double mean = a.tc;
+    if (a.is_causal || a.window_left >= 0 || a.window_right >= 0) {
+        const long long samples = std::min<long long>(per_unit, 9);
+        n = 0;
+        mean = 0.0;
+        for (long long i = 0; i < samples; ++i) {
+            const int tiles = block_tiles(a, samples == 1 ? 0 : i * (per_unit - 1) / (samples - 1), pair);
+            n = std::max(n, tiles);
+            least = std::min(least, tiles);
+            mean += static_cast<double>(tiles) / samples;
+        }
+    }
+    const int tile_rows = pair ? 2 * kTile : kTile;
+    const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
+    const double stage = staged ? 0.3 * c.merge * rows : 0.0;
+    Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, least >= 0.8 * n};
+    if (blocks > slots) {
+        const double waves = static_cast<double>(blocks) / slots;
+        if (!best.even) {  // blocks of different lengths: the longest first, shorter ones fill up
+            best.us = std::max(best.us, waves * (launch_us(c, static_cast<double>(slots), sms, mean) + stage));
+        } else if (pair) {  // of about one length: wave after wave
+            const long long rest = blocks % slots;
+            best.us *= static_cast<double>(blocks / slots);
+            if (rest > 0) best.us += launch_us(c, static_cast<double>(rest), sms, n) + stage;
+        } else {  // two CTAs an SM get out of step
+            best.us *= waves;
+        }
+    }
+    for (int parts = 2; parts <= ClusterRoom::kMax && parts <= n; parts += parts < 8 ? 1 : 8) {
+        if (blocks > room.fits(parts, pair ? 1 : 2)) continue;
+        const double merge = c.merge * ((parts & (parts - 1)) ? 1.15 : 1.0) + c.merge_each * std::min(parts, 10);
+        const double us = launch_us(c, static_cast<double>(blocks * parts), sms, (n + parts - 1) / parts) + merge * rows +
+                          (parts == 16 ? 1.5 : 0.0);
+        if (us < best.us * (best.parts == 1 ? 0.96 : 1.0)) best = {parts, us, best.even};
     }
     return best;
 }
 
 }  // namespace
 
-void plan_tiled(FwdArgs* a, int sms) {
+int ClusterRoom::fits(int parts, int ctas_per_sm) const {
+    // (two CTAs an SM: two sets of clusters, or clusters over half as many SMs, whichever are more)
+    const int once = one_per_sm[parts];
+    return ctas_per_sm == 1 || once == 0 ? once : std::max(2 * once, one_per_sm[(parts + 1) / 2]);
+}
+
+ClusterRoom cluster_room(int sms) {
+    // asked once per device; concurrent first calls store the same answer
+    static ClusterRoom kept[64];
+    static std::atomic<bool> ready[64];
+    int dev = -1;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    if (known && ready[dev].load(std::memory_order_acquire)) return kept[dev];
+    ClusterRoom room = {};
+    room.one_per_sm[1] = sms;
+    auto kern = fwd_tiled_kernel<128, 2, true, false, false, true>;  // (one CTA an SM)
+    constexpr int smem = Cfg<128, 2>::kSmemBytes;
+    bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+              cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int parts = 2; parts <= ClusterRoom::kMax && ok; parts += parts < 8 ? 1 : 8) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(parts);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(parts * sms));
+        cfg.blockDim = dim3(Cfg<128, 2>::kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        ok = cudaOccupancyMaxActiveClusters(&room.one_per_sm[parts], kern, &cfg) == cudaSuccess;
+    }
+    if (!ok) {  // no clusters then, this time
+        (void)cudaGetLastError();
+        room = {};
+        room.one_per_sm[1] = sms;
+        return room;
+    }
+    if (known) {
+        static std::mutex mutex;
+        std::lock_guard<std::mutex> lock(mutex);
+        if (!ready[dev].load(std::memory_order_relaxed)) {
+            kept[dev] = room;
+            ready[dev].store(true, std::memory_order_release);
+        }
+    }
+    return room;
+}
+
+void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
     a->parts = 1;
     a->pack_rows = 0;
     a->staged = a->o_dim != a->head_dim;
     if (a->accum_o != nullptr) return;  // (a running pair is merged by the unstaged epilogue, each query tile as it finishes)
-    Split split = best_split(*a, sms, a->staged != 0);
+    Split split = best_split(*a, sms, room, a->staged != 0);
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
-    // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the
-    // model says that it saves a tenth: below that the staged epilogue, slower than TMA stores, eats the gain ([64 heads
-    // on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.  A tile
-    // across heads walks the KV tiles of all of a head's positions; those past a row's own come first, and the row starts
-    // afresh behind them, but those before a left window would come last and bring masked infinities and NaN with them:
-    // with one, only heads of a single tile are stacked, whose rows walked all of these tiles anyway.)
+    // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the query
+    // blocks are of about one length (tiles across heads have the longest: [4 x 12 heads on 2, 1940 rows, 1241 keys, causal]
+    // 72 us stacked, 50 not), it saves a tenth of the query tiles, and the model says 7 % and half a microsecond of the time:
+    // below that the staged epilogue, slower than TMA stores, eats the gain ([64 heads on 8, 720 rows, 25871 keys], 184
+    // blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all
+    // of a head's positions; those past a row's own come first, and the row starts afresh behind them, but those before a
+    // left window would come last and bring masked infinities and NaN with them: with one, only heads of a single tile are
+    // stacked, whose rows walked all of these tiles anyway.)
     const int heads = a->kv_group;
     const long long rows = static_cast<long long>(heads) * a->seqlen_q;
     if (heads > 1 && a->alibi_slopes == nullptr && rows <= 0x3fffffffLL && (a->window_left < 0 || a->seqlen_q <= kTile)) {
@@ -1428,8 +1523,9 @@ void plan_tiled(FwdArgs* a, int sms) {
         b.tr = static_cast<int>((rows + kTile - 1) / kTile);
         b.units = a->units / heads;
         b.kv_group = 1;
-        const Split packed = best_split(b, sms, true);
-        if (b.tr < heads * a->tr && packed.us < 0.9 * split.us) {
+        const bool fewer = 10LL * b.tr <= 9LL * heads * a->tr;
+        const Split packed = split.even && fewer ? best_split(b, sms, room, true) : Split{1, 1e30, true};
+        if (packed.us < 0.93 * split.us - 0.5) {
             *a = b;
             split = packed;
         }

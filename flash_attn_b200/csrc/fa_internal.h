@@ -66,9 +66,18 @@ struct FwdArgs {
     DropoutParams drop;
 };
 
+// Clusters that the device holds at once.  A cluster lies within a GPC, and GPCs differ in their SMs from device to device: a
+// B200 with 148 SMs holds 74 clusters of 2 CTAs at one CTA an SM, 45 of 3, 33 of 4, 26 of 5, 22 of 6, 15 of 7 or 8, 7 of 16.
+struct ClusterRoom {
+    static constexpr int kMax = 16;
+    int one_per_sm[kMax + 1];  // by size (1 to 8 and 16), with one CTA an SM
+    int fits(int parts, int ctas_per_sm) const;
+};
+ClusterRoom cluster_room(int sms);  // of the current device; none above one CTA where the runtime does not say
+
 // Decides how a launch without dropout is cut (fills staged, parts and, for short grouped queries, restates the
 // problem with the heads of a K/V head stacked: units, heads, kv_group, seqlen_q, tr, pack_rows).
-void plan_tiled(FwdArgs* a, int sms);
+void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room);
 
 // Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O
 // (32-row boxes); it is read only when a.o_tma is set.

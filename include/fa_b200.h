@@ -138,7 +138,9 @@ size_t fa_fwd_workspace_bytes(const fa_fwd_params* p);
  * the kernels may divide the keys among more or fewer CTAs than that, as suits the device. */
 int fa_fwd_resolve_splits(const fa_fwd_params* p);
 
-/* How fa_fwd would cut p on a device of num_sms SMs (host arithmetic only; the pointers of p are not followed).
+/* How fa_fwd would cut p on a device of num_sms SMs that holds clusters[n] clusters of n CTAs at once, with one CTA an SM
+ * (cudaOccupancyMaxActiveClusters; 17 entries, of which 2 to 8 and 16 are read; NULL: it holds none).  Host arithmetic
+ * only; the pointers of p are not followed.
  * Of use to whoever wants to know why a shape takes the time it takes, and to the tests. */
 typedef struct fa_fwd_plan_info {
     int decode;               /* 1: the kernel for seqlen_q <= 8, 0: the tiled kernel */
@@ -148,7 +150,7 @@ typedef struct fa_fwd_plan_info {
     int staged;               /* tiled: finished rows leave through shared memory */
     int stacked_rows;         /* tiled: the heads of a K/V head are stacked into one unit, this many rows each; 0 = not */
 } fa_fwd_plan_info;
-int fa_fwd_plan(const fa_fwd_params* p, int num_sms, fa_fwd_plan_info* plan);
+int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd_plan_info* plan);
 
 /* The reference's split policy, same arguments and result as
  * num_splits_heuristic (src/main.cu:391-422). */

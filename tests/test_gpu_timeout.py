@@ -14,6 +14,7 @@ import torch
 import gpu_util
 import oracle_lib
 import synth
+from plan_util import plan
 
 pytestmark = pytest.mark.gpu
 
@@ -90,8 +91,8 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_stays_usable(test_lib):
 
 
 @pytest.mark.parametrize("skip,H,Hk,Nq,Nk,d", [
-    ("fa_test_skip_kv_tile", 8, 8, 256, 1100, 128),     # the parts of a query block, merged in their cluster
-    ("fa_test_skip_kv_tile", 8, 8, 100, 1100, 64),
+    ("fa_test_skip_kv_tile", 8, 8, 256, 2400, 128),     # the parts of a query block, merged in their cluster
+    ("fa_test_skip_kv_tile", 8, 8, 100, 2400, 64),
     ("fa_test_skip_decode_tile", 2, 2, 1, 1100, 128),   # decode: eight parts in a cluster, of which one gives up
     ("fa_test_skip_decode_tile", 4, 1, 1, 65628, 64),   # ... and parts that the combine kernel merges
 ])
@@ -111,8 +112,10 @@ def test_a_part_that_gave_up_leaves_no_plausible_row(test_lib, skip, H, Hk, Nq, 
     need = L.fa_fwd_workspace_bytes(ctypes.byref(p))
     ws = torch.empty(max(need, 16), device="cuda", dtype=torch.uint8)
     p.workspace, p.workspace_bytes = ws.data_ptr(), need
-    # tiled: the second KV tile of every CTA that has one; decode: a slot of the K/V stream that only the longest part has
-    tile = 1 if skip == "fa_test_skip_kv_tile" else 3 if Nk == 1100 else 17
+    # a KV tile (decode: a slot of the K/V stream) that only the longest parts have
+    parts, tiles = plan(1, H, Nq, Nk, d, heads_k=Hk).parts, (Nk + 127) // 128
+    assert parts > 1 and tiles % parts != 0
+    tile = tiles // parts if skip == "fa_test_skip_kv_tile" else 3 if Nk == 1100 else 17
     try:
         assert getattr(L, skip)(tile) == 0
         assert L.fa_fwd(ctypes.byref(p)) == 0

@@ -1,7 +1,7 @@
 """How a call is cut (fa_fwd_plan, host arithmetic): the plan goes by the keys that the masks leave visible."""
 import pytest
 
-from plan_util import plan
+from plan_util import B200_CLUSTERS, plan
 
 
 @pytest.mark.parametrize("B,H,Hk,Nq,Nk,kw", [
@@ -33,3 +33,29 @@ def test_the_plan_of_a_block_is_that_of_its_visible_keys(kw):
             whole = plan(1, 8, Nq, 9000, 64, heads_k=2, q_pos0=q0, **kw)
             short = plan(1, 8, Nq, (q0 + Nq + 255) // 128 * 128 + (right + 127) // 128 * 128, 64, heads_k=2, q_pos0=q0, **kw)
             assert bytes(whole) == bytes(short), (q0, Nq, kw)
+
+
+@pytest.mark.parametrize("sms,clusters", [(148, B200_CLUSTERS), (132, (0, 132, 66, 40, 30, 24, 18, 12, 12, 12, 10, 7, 7, 7, 7, 7, 6)),
+                                          (148, (0, 148) + (0,) * 15)])
+@pytest.mark.parametrize("Nq,per_sm", [(256, 1), (100, 2)])
+def test_the_clusters_of_a_split_are_resident_at_once(sms, clusters, Nq, per_sm):
+    seen = set()
+    for blocks in range(1, 200):
+        for Nk in (500, 1024, 2419, 8492):
+            parts = plan(1, blocks, Nq, Nk, 128, sms=sms, clusters=clusters).parts
+            seen.add(parts)
+            room = clusters[parts] if per_sm == 1 else max(2 * clusters[parts], clusters[(parts + 1) // 2])
+            assert parts == 1 or blocks <= room, (blocks, Nk, parts)
+    assert (seen == {1}) == (clusters[2] == 0)
+
+
+@pytest.mark.parametrize("B,H,Hk,Nq,Nk,causal,parts", [
+    (2, 32, 8, 62, 2419, True, (4, 5)),      # 16 stacked blocks: 20.7 us in four parts, 40.4 in seven, 31.7 unsplit and unstacked
+    (1, 16, 16, 256, 2419, False, (4, 5)),
+    (1, 48, 48, 256, 8492, False, (2,)),     # 45 clusters of three fit, not 48
+    (1, 48, 48, 100, 1024, False, (1,)),     # 14.4 us unsplit, 15.7 in four parts
+    (1, 32, 8, 300, 8492, True, (3,)),
+    (8, 16, 16, 2048, 2048, True, (1,)),
+])
+def test_part_counts(B, H, Hk, Nq, Nk, causal, parts):
+    assert plan(B, H, Nq, Nk, 128, heads_k=Hk, causal=causal, q_pos0=Nk - Nq if causal else 0).parts in parts
