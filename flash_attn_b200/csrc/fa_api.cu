@@ -211,6 +211,12 @@ void fill_decode_args(const fa_fwd_params* p, const FwdArgs& a, DecodeArgs* d) {
     d->q_pos0 = a.q_pos0; d->k_pos0 = a.k_pos0; d->o_is_fp32 = a.o_is_fp32; d->drop = a.drop;
 }
 
+// Parts of a unit that the decode kernel may be cut into: with a split count of the caller's no more partials than it has
+// room for.
+int most_parts(const fa_fwd_params* p, int splits) {
+    return p->num_splits > 0 ? std::max(kDecodeCluster, splits) : kDecodeParts;
+}
+
 // Partial results per unit that a launch keeps in the workspace (1 = none).
 int planned_parts(const fa_fwd_params* p, int splits, int sms) {
     if (p->seqlen_q > 8 || p->accum_o != nullptr) return p->p_dropout > 0.0f ? splits : 1;
@@ -218,14 +224,9 @@ int planned_parts(const fa_fwd_params* p, int splits, int sms) {
     DecodeArgs d;
     fill_args(p, splits, &a);
     fill_decode_args(p, a, &d);
-    plan_decode(&d, p->batch * p->heads, splits, false, sms);
+    plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), sms);
     return d.merge ? 1 : d.parts;
 }
-// What the workspace has to hold: a caller that names its split count provides for that count, whatever is made of it.
-int partials_kept(const fa_fwd_params* p, int splits, int sms) {
-    return p->num_splits == 0 ? planned_parts(p, splits, sms) : splits;
-}
-
 // head_dim that is not a multiple of 8: Q/K/V are copied to a pitch of d8 = ceil8(head_dim)
 // elements (zero columns), the kernels run on the padded problem, O is copied back.
 struct PadPlan {
@@ -265,25 +266,23 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
     if (decode) {
         fill_decode_args(p, a, &d);
         d.o_dim = o_dim;
-        plan_decode(&d, units, splits, p->num_splits > 0, sms);
+        plan_decode(&d, units, splits, most_parts(p, splits), sms);
         parts = d.merge ? 1 : d.parts;
     }
     if (splits > 1 || parts > 1) {
         size_t lse_off = 0;
-        const size_t need = partial_bytes(p, parts, &lse_off);
+        size_t need = parts > 1 ? partial_bytes(p, parts, &lse_off) : 0;
         // (a caller that names its split count provides the workspace of that count, whatever is made of it)
-        const size_t promised = p->num_splits > 0 ? partial_bytes(p, splits, nullptr) : need;
+        if (p->num_splits > 0) need = std::max(need, partial_bytes(p, splits, nullptr));
+        const bool enough = need == 0 || (p->workspace && p->workspace_bytes >= need);
         const bool aligned = (reinterpret_cast<uintptr_t>(p->workspace) & 15u) == 0;
-        const bool missing = !p->workspace || p->workspace_bytes < std::max(need, promised) || (splits == 1 && !aligned);
-        if (missing && parts > 1 && splits == 1) {
-            // the split count was the library's to choose and the caller keeps no workspace
-            d.parts = 8;
-            d.merge = 1;
+        if (!enough && (p->num_splits > 0 || dropout)) return FA_ERR_WORKSPACE;
+        if (enough && !aligned && splits > 1) return FA_ERR_INVALID_ARG;
+        if (parts > 1 && (!enough || !aligned)) {
+            // the count is the library's to choose: what a cluster merges needs no workspace
+            plan_decode(&d, units, splits, kDecodeCluster, sms);
             parts = 1;
-        } else if (missing && (parts > 1 || p->num_splits > 1)) {
-            return FA_ERR_WORKSPACE;
         }
-        if (!missing && !aligned) return FA_ERR_INVALID_ARG;
         if (parts > 1) {
             a.o_partial = d.o_partial = static_cast<float*>(p->workspace);
             a.lse_partial = d.lse_partial = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + lse_off);
@@ -387,7 +386,7 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd
     if (p->seqlen_q <= 8 && p->accum_o == nullptr) {
         DecodeArgs d;
         fill_decode_args(&q, a, &d);
-        plan_decode(&d, p->batch * p->heads, splits, p->num_splits > 0, num_sms);
+        plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), num_sms);
         plan->decode = 1;
         plan->parts = d.parts;
         plan->merged = d.merge;
@@ -442,9 +441,9 @@ int fa_fwd(const fa_fwd_params* p) {
     const PadPlan pl = pad_plan(p);
     fa_fwd_params q = *p;
     q.head_dim = pl.d8;
-    const int parts = partials_kept(&q, splits, sms);
-    const size_t part = parts > 1 ? partial_bytes(&q, parts, nullptr) : 0;
-    if (!p->workspace || p->workspace_bytes < pl.total + part) return FA_ERR_WORKSPACE;
+    // (without dropout a count of the library's own choosing goes by the workspace there is)
+    const int kept = p->num_splits > 0 ? splits : p->p_dropout > 0.0f ? planned_parts(&q, splits, sms) : 1;
+    if (!p->workspace || p->workspace_bytes < pl.total + (kept > 1 ? partial_bytes(&q, kept, nullptr) : 0)) return FA_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(p->workspace) & 255u) return FA_ERR_INVALID_ARG;
     char* ws = static_cast<char*>(p->workspace);
     char* qp = ws; char* kp = qp + pl.q_bytes; char* vp = kp + pl.kv_bytes; char* op = vp + pl.kv_bytes;
@@ -452,8 +451,8 @@ int fa_fwd(const fa_fwd_params* p) {
     const long long rk = static_cast<long long>(p->batch) * kv_heads(p) * p->seqlen_k;
     if (launch_pad_qkv(p->q, p->k, p->v, qp, kp, vp, rq, rk, p->head_dim, pl.d8, stream) != cudaSuccess) return FA_ERR_CUDA;
     q.q = qp; q.k = kp; q.v = vp;
-    q.workspace = part ? op + pl.o_bytes : nullptr;
-    q.workspace_bytes = part;
+    q.workspace_bytes = p->workspace_bytes - pl.total;
+    q.workspace = q.workspace_bytes > 0 ? op + pl.o_bytes : nullptr;
     const bool direct = !(p->p_dropout > 0.0f) || p->seqlen_q <= 8 || splits > 1;
     if (direct) return run_fwd(&q, p->head_dim, splits, sms);
     q.o = op;

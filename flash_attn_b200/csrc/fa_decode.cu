@@ -86,8 +86,6 @@ struct DCfg {
     static_assert(kSmemBytes <= 115712, "two CTAs per SM");
 };
 
-constexpr int kMaxCluster = 16;            // parts of a unit that one cluster merges (above 8: non-portable cluster size)
-
 constexpr float kDLog2e = 1.4426950408889634f;
 constexpr float kDLn2 = 0.6931471805599453f;
 
@@ -633,9 +631,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
             const int r = threadIdx.x;
             const uint32_t base = sRing;
             for (int n = part; n < nc; n += a.parts) {
-                float m_j[kMaxCluster], l_j[kMaxCluster], o_j[kMaxCluster];
+                float m_j[kDecodeCluster], l_j[kDecodeCluster], o_j[kDecodeCluster];
 #pragma unroll
-                for (int j = 0; j < kMaxCluster; ++j) {
+                for (int j = 0; j < kDecodeCluster; ++j) {
                     m_j[j] = -INFINITY;
                     l_j[j] = o_j[j] = 0.0f;
                     if (j < a.parts) {
@@ -647,11 +645,11 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 }
                 float m = m_j[0];
 #pragma unroll
-                for (int j = 1; j < kMaxCluster; ++j) m = fmaxf(m, m_j[j]);
+                for (int j = 1; j < kDecodeCluster; ++j) m = fmaxf(m, m_j[j]);
                 float l = 0.0f, o = 0.0f;
                 if (m != -INFINITY) {
 #pragma unroll
-                    for (int j = 0; j < kMaxCluster; ++j) {
+                    for (int j = 0; j < kDecodeCluster; ++j) {
                         // (a part without visible keys has m_j = -inf and weight 0; its o_j is 0)
                         const float w = ex2f(m_j[j] - m);
                         l = fmaf(w, l_j[j], l);
@@ -660,7 +658,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
                 } else {
                     // no visible key (all zero), or nothing but NaN
 #pragma unroll
-                    for (int j = 0; j < kMaxCluster; ++j) {
+                    for (int j = 0; j < kDecodeCluster; ++j) {
                         l += l_j[j];
                         o += o_j[j];
                     }
@@ -676,7 +674,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
 
 }  // namespace
 
-void plan_decode(DecodeArgs* a, int units, int splits, bool forced, int sms) {
+void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms) {
     // key tiles visible to any query row: the tile-granular clip of the masks (src/flash_forward.h:39-48)
     // for the query rows at positions q_pos0 .. q_pos0 + seqlen_q - 1
     long long lo = 0, hi = a->tc;
@@ -724,18 +722,17 @@ void plan_decode(DecodeArgs* a, int units, int splits, bool forced, int sms) {
     const double full = narrow ? 1.3 : 2.3, least = a->columns == 16 ? 1.15 : narrow ? 0.85 : 0.95;
     int best = 1;
     double best_t = 1e30;
-    for (int parts = 1; parts <= 64 && (parts == 1 || parts <= n); parts *= 2) {
-        if (parts > kMaxCluster && forced && parts > splits) break;  // (the caller's workspace holds `splits` partials)
+    for (int parts = 1; parts <= most && (parts == 1 || parts <= n); parts *= 2) {
         const double ctas = static_cast<double>(cta_units) * parts, waves = std::floor(ctas / (2.0 * sms));
         const double rest = ctas - waves * 2.0 * sms, even = static_cast<double>(n) / parts;
         double t = waves * (full * even + 3.0);
         if (rest > sms) t += full * even + 3.0;
         else if (rest > 0) t += std::ceil(even) * std::max(least, 0.65 * full * rest / sms) + 3.0;
-        if (parts > 1) t += parts > kMaxCluster ? 8.0 : (parts == 16 && ctas > sms) ? 7.0 : 1.2;
+        if (parts > 1) t += parts > kDecodeCluster ? 8.0 : (parts == 16 && ctas > sms) ? 7.0 : 1.2;
         if (t < best_t) { best_t = t; best = parts; }
     }
     a->parts = best;
-    a->merge = best > 1 && best <= kMaxCluster;
+    a->merge = best > 1 && best <= kDecodeCluster;
 }
 
 cudaError_t launch_decode(const DecodeArgs& a_in, const CUtensorMap& tk, const CUtensorMap& tv, int units, bool bf16,

@@ -89,3 +89,41 @@ def test_parts_of_a_unit_and_query_columns(H, Hk, Nq, nk, d, dtype, kw):
 def test_dropout_of_query_rows_and_heads_that_share_keys(H, Hk, Nq, nk, kw):
     gpu_util.assert_close(gpu_util.run_case(2, H, Nq, nk, 64, "bfloat16", seed=59, causal=True, q_pos0=nk - Nq, heads_k=Hk,
                                             p_dropout=0.25, drop_seed=7, **kw), f"{H}/{Hk} heads, {Nq} rows, {nk} keys {kw}")
+
+
+@pytest.mark.parametrize("tiles", [509, 512])  # a prime number of key tiles, and one that splits in many ways
+@pytest.mark.parametrize("d", [64, 60])        # 60: padded copies, which do need a workspace
+def test_a_plan_of_many_parts_does_without_their_workspace(tiles, d):
+    """num_splits = 0 leaves the count to the library: with no room for the partials of its plan the parts are as many as a
+    cluster merges.  (The C entry point; the Python one always brings the workspace that was asked for.)"""
+    import ctypes
+    import flash_attn_b200 as fa
+    from flash_attn_b200 import _lib
+    L = _lib.load()
+    H, Hk, Nk = 4, 1, 128 * tiles
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    q, k, v = (torch.randn((1, h, n, d), generator=g, device="cuda").bfloat16() for h, n in ((H, 1), (Hk, Nk), (Hk, Nk)))
+    want_o, want_lse = fa.flash_attn_forward(q, k, v, num_splits=0)
+    p = _lib.FwdParams()
+    p.q, p.k, p.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
+    p.dtype = p.o_dtype = _lib.FA_DTYPE_BF16
+    p.batch, p.heads, p.heads_k, p.seqlen_q, p.seqlen_k, p.head_dim = 1, H, Hk, 1, Nk, d
+    p.softmax_scale, p.window_left, p.window_right = d ** -0.5, -1, -1
+    p.stream = torch.cuda.current_stream().cuda_stream
+    o, lse = torch.zeros_like(want_o), torch.zeros_like(want_lse)
+    p.o, p.lse = o.data_ptr(), lse.data_ptr()
+    need = L.fa_fwd_workspace_bytes(ctypes.byref(p))
+    p.num_splits = 1
+    least = L.fa_fwd_workspace_bytes(ctypes.byref(p))  # of the padded copies alone
+    p.num_splits = 0
+    assert need > least and (least > 0) == (d == 60)
+    ws = torch.empty(need, device="cuda", dtype=torch.uint8)
+    p.workspace = ws.data_ptr() if least else None
+    p.workspace_bytes = least
+    assert L.fa_fwd(ctypes.byref(p)) == 0
+    torch.cuda.synchronize()
+    assert (o.float() - want_o.float()).abs().max() <= gpu_util.O_MAX_ABS
+    assert (lse - want_lse).abs().max() <= gpu_util.LSE_ABS
+    p.num_splits = 32  # a count of the caller's: its workspace is asked for, as ever
+    assert L.fa_fwd(ctypes.byref(p)) == -3
