@@ -55,3 +55,22 @@ def test_masked_values_stay_out_of_query_tiles_that_do_not_reach_them(B, H, Hk, 
     clean = call()
     v[:, :, poisoned] = value
     assert torch.equal(call(), clean)
+
+
+@pytest.mark.parametrize("num_splits", [0, 32])
+def test_host_call_keeps_no_room_for_partials_that_nobody_writes(num_splits):
+    from flash_attn_b200 import _lib, api
+    L = _lib.load()
+    H, Hk, Nq, Nk, d = 32, 8, 300, 8492, 128  # (partials of 32 and more splits: 158 MB and more; a slot's tensors: 20 MB)
+    q, k, v = (torch.randn(1, h, n, d).bfloat16().pin_memory() for h, n in ((H, Nq), (Hk, Nk), (Hk, Nk)))
+    api.flash_attn_forward_host(q, k, v, num_splits=1)  # (kernels and streams are in place)
+    L.fa_fwd_host_release()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    o, _ = api.flash_attn_forward_host(q, k, v, num_splits=num_splits)
+    held = before - torch.cuda.mem_get_info()[0]
+    L.fa_fwd_host_release()
+    assert 0 < held < 100 << 20, held
+    import flash_attn_b200 as fa
+    want = fa.flash_attn_forward(q.cuda(), k.cuda(), v.cuda())[0].cpu()
+    assert (o.float() - want.float()).abs().max() <= gpu_util.O_MAX_ABS
