@@ -224,7 +224,7 @@ int planned_parts(const fa_fwd_params* p, int splits, int sms) {
     DecodeArgs d;
     fill_args(p, splits, &a);
     fill_decode_args(p, a, &d);
-    plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), sms);
+    plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), sms, cluster_room(sms));
     return d.merge ? 1 : d.parts;
 }
 // head_dim that is not a multiple of 8: Q/K/V are copied to a pitch of d8 = ceil8(head_dim)
@@ -266,7 +266,7 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
     if (decode) {
         fill_decode_args(p, a, &d);
         d.o_dim = o_dim;
-        plan_decode(&d, units, splits, most_parts(p, splits), sms);
+        plan_decode(&d, units, splits, most_parts(p, splits), sms, cluster_room(sms));
         parts = d.merge ? 1 : d.parts;
     }
     if (splits > 1 || parts > 1) {
@@ -280,7 +280,7 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
         if (enough && !aligned && splits > 1) return FA_ERR_INVALID_ARG;
         if (parts > 1 && (!enough || !aligned)) {
             // the count is the library's to choose: what a cluster merges needs no workspace
-            plan_decode(&d, units, splits, kDecodeCluster, sms);
+            plan_decode(&d, units, splits, kDecodeCluster, sms, cluster_room(sms));
             parts = 1;
         }
         if (parts > 1) {
@@ -386,7 +386,7 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd
     if (p->seqlen_q <= 8 && p->accum_o == nullptr) {
         DecodeArgs d;
         fill_decode_args(&q, a, &d);
-        plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), num_sms);
+        plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), num_sms, room);
         plan->decode = 1;
         plan->parts = d.parts;
         plan->merged = d.merge;

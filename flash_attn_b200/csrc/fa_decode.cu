@@ -674,7 +674,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
 
 }  // namespace
 
-void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms) {
+void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms, const ClusterRoom& room) {
     // key tiles visible to any query row: the tile-granular clip of the masks (src/flash_forward.h:39-48)
     // for the query rows at positions q_pos0 .. q_pos0 + seqlen_q - 1
     long long lo = 0, hi = a->tc;
@@ -697,42 +697,58 @@ void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms) {
     a->full_lo = static_cast<int>(std::min<long long>(flo, a->tc));
     a->full_hi = static_cast<int>(fhi);
 
-    // query heads that share a K/V head are packed into one CTA, up to sixteen columns at a time
-    const int queries = a->kv_group * a->seqlen_q;
-    a->columns = queries == 1 ? 1 : queries <= 4 ? 4 : queries <= 8 ? 8 : 16;
-    const int heads_per_cta = a->columns / a->seqlen_q;  // whole heads whose query rows fit the columns
-    a->subgroups = (a->kv_group + heads_per_cta - 1) / heads_per_cta;
-    const long long cta_units = static_cast<long long>(units / a->kv_group) * a->subgroups;
-
-    if (a->drop.threshold != 0ull) {
-        a->parts = splits;
-        a->by_split = splits > 1;
-        a->merge = splits == 2 || splits == 4 || splits == 8 || splits == 16;
-        return;
+    // How many columns a CTA has (query heads that share a K/V head are packed into one CTA, whole heads with their query rows;
+    // what does not fit goes to further sub-groups, CTAs of their own that read the same K/V) and how many CTAs share a unit's
+    // keys: the fastest by a model of the kernel's time, in us, fitted to 461 shapes of 8 to 512 K/V heads x 1 to 256 tiles, each
+    // swept over its columns and parts: what it takes is 0.2 % slower than the best on average, at most 8 %.
+    //   A CTA takes `fixed` to start, mask and drain and `rate` for a K + V tile, a sixth more with a second CTA on its SM; what
+    //   does not fit (two CTAs an SM, clusters as the device has room for them) follows in waves.  Columns cost by the CTA, since a
+    //   softmax thread takes its key through all of them: sixteen pay only where CTAs are many or HBM bounds the launch ([1 x 64
+    //   heads on 4, 100 keys] 10.7 us in sixteen columns, 5.1 in four; [16 x 32 on 8, 4 rows, 8192 keys] 130 in four, 88 in sixteen).
+    //   A merge in the cluster costs 1 to 2 us, partials through memory and the combine kernel 7.5 and 0.34 a part.
+    //   HBM gives 7.65 TB/s, the dropout bits of a head and tile take 0.12.
+    struct Cost {
+        double fixed[4], rate[4];
+    };
+    static constexpr Cost kCost[2] = {{{3.0, 4.2, 6.1, 7.3}, {0.79, 0.84, 0.68, 1.06}},    // by columns 1, 4, 8, 16: D = 128
+                                      {{3.05, 4.2, 6.2, 7.7}, {0.69, 0.68, 0.65, 0.81}}};  // D = 64
+    static constexpr int kColumns[4] = {1, 4, 8, 16};
+    static constexpr double kMerge[5] = {0.0, 2.05, 1.15, 1.45, 1.0};  // 1, 2, 4, 8, 16 parts
+    const Cost& cost = kCost[a->head_dim <= 64];
+    const bool dropout = a->drop.threshold != 0ull;
+    const int queries = a->kv_group * a->seqlen_q, kv_units = units / a->kv_group;
+    const double hbm_us = static_cast<double>(kv_units) * n * kTile * a->head_dim * 4.0 / 7.65e6;
+    double best_us = 1e30;
+    for (int i = queries == 1 ? 0 : 1; i < 4; ++i) {
+        const int heads_per_cta = kColumns[i] / a->seqlen_q;
+        if (heads_per_cta < 1) continue;
+        const int subgroups = (a->kv_group + heads_per_cta - 1) / heads_per_cta;
+        const double rate = cost.rate[i] + (dropout ? 0.12 * std::min(heads_per_cta, a->kv_group) : 0.0);
+        // (with dropout the parts are the caller's splits, part of the streams' geometry)
+        for (int p = 0, parts = dropout ? splits : 1; dropout || (parts <= most && (p == 0 || parts <= n)); ++p, parts *= 2) {
+            const bool merged = parts == 2 || parts == 4 || parts == 8 || parts == 16;
+            if (merged && !dropout && room.fits(parts, 2) == 0) continue;
+            const long long ctas = static_cast<long long>(kv_units) * subgroups * parts;
+            const long long slots = merged && room.fits(parts, 2) > 0 ? static_cast<long long>(room.fits(parts, 2)) * parts : 2LL * sms;
+            const double chain = cost.fixed[i] + rate * ((n + parts - 1) / parts);
+            auto wave = [&](long long c) { return c > 0 ? chain * (1.0 + 0.166 * std::min(1.0, std::max(0.0, static_cast<double>(c) / sms - 1.0))) : 0.0; };
+            double us = static_cast<double>(ctas / slots) * wave(slots) + wave(ctas % slots);
+            if (merged) us += kMerge[parts == 2 ? 1 : parts == 4 ? 2 : parts == 8 ? 3 : 4] - (i > 0 ? 0.8 : 0.0);
+            else if (parts > 1) us += 7.5 + 0.34 * parts;
+            const double floor_us = 0.65 + hbm_us * (ctas <= slots ? 1.02 : 1.0);
+            us = std::max(us, floor_us) + 0.2 * std::min(us, floor_us);
+            if (us < best_us) {
+                best_us = us;
+                a->columns = kColumns[i];
+                a->subgroups = subgroups;
+                a->parts = parts;
+                a->merge = merged;
+            }
+            if (dropout) break;
+        }
+        if (kColumns[i] >= queries) break;  // (no use for more)
     }
-    // How many CTAs share a unit's keys: a model of the kernel's time, in us, fitted to sweeps over 8 to 1024 units
-    // x 1 to 256 tiles on B200.  Two CTAs fit an SM.  A K + V tile takes a CTA `full` when every SM has two (bound
-    // by HBM, 7.4 TB/s); with at most one CTA per SM it takes less as fewer SMs load at a time, down to `least`, the
-    // CTA's own chain of load, MMA, softmax, MMA.  A wave costs 3 us to start and drain, a merge in the cluster 1.2
-    // (16-CTA clusters are slow to place when they do not all fit at once), partials through memory and the combine
-    // kernel 8.  Measured, one CTA per unit against the choice: 8 K/V heads x 1000 keys 10.4 -> 6.3 us, x 32768 keys
-    // 226 -> 25; 128 units x 4097 keys 44.9 -> 44.6 (HBM-bound either way); 64 units x 8000 keys, 16 queries 77 -> 47.
-    a->by_split = 0;
-    const bool narrow = a->head_dim <= 64;
-    const double full = narrow ? 1.3 : 2.3, least = a->columns == 16 ? 1.15 : narrow ? 0.85 : 0.95;
-    int best = 1;
-    double best_t = 1e30;
-    for (int parts = 1; parts <= most && (parts == 1 || parts <= n); parts *= 2) {
-        const double ctas = static_cast<double>(cta_units) * parts, waves = std::floor(ctas / (2.0 * sms));
-        const double rest = ctas - waves * 2.0 * sms, even = static_cast<double>(n) / parts;
-        double t = waves * (full * even + 3.0);
-        if (rest > sms) t += full * even + 3.0;
-        else if (rest > 0) t += std::ceil(even) * std::max(least, 0.65 * full * rest / sms) + 3.0;
-        if (parts > 1) t += parts > kDecodeCluster ? 8.0 : (parts == 16 && ctas > sms) ? 7.0 : 1.2;
-        if (t < best_t) { best_t = t; best = parts; }
-    }
-    a->parts = best;
-    a->merge = best > 1 && best <= kDecodeCluster;
+    a->by_split = dropout && splits > 1;
 }
 
 cudaError_t launch_decode(const DecodeArgs& a_in, const CUtensorMap& tk, const CUtensorMap& tv, int units, bool bf16,

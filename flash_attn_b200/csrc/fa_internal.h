@@ -116,10 +116,10 @@ struct DecodeArgs {
 };
 constexpr int kDecodeCluster = 16;  // parts of a unit that one cluster merges (above 8: non-portable cluster size)
 constexpr int kDecodeParts = 64;    // parts at most
-// How many CTAs, at most `most`, share the keys of a unit (fills parts, merge, by_split, columns, subgroups and the
+// How many CTAs, at most `most`, share the keys of a unit and how many columns each has (fills parts, merge, by_split, columns, subgroups and the
 // tile ranges; the problem's fields are set).  `splits` is the resolved split count of the caller.  A plan with parts > 1
 // and merge == 0 writes partials: they need a workspace, and the combine kernel behind.
-void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms);
+void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms, const ClusterRoom& room);
 cudaError_t launch_decode(const DecodeArgs& a, const CUtensorMap& tk, const CUtensorMap& tv, int units, bool bf16,
                           cudaStream_t stream);
 

@@ -6,6 +6,7 @@ import torch
 
 import gpu_util
 import oracle_lib
+from plan_util import plan
 
 pytestmark = pytest.mark.gpu
 
@@ -91,7 +92,7 @@ def test_dropout_of_query_rows_and_heads_that_share_keys(H, Hk, Nq, nk, kw):
                                             p_dropout=0.25, drop_seed=7, **kw), f"{H}/{Hk} heads, {Nq} rows, {nk} keys {kw}")
 
 
-@pytest.mark.parametrize("tiles", [509, 512])  # a prime number of key tiles, and one that splits in many ways
+@pytest.mark.parametrize("tiles", [2039, 2048])  # a prime number of key tiles, and one that splits in many ways
 @pytest.mark.parametrize("d", [64, 60])        # 60: padded copies, which do need a workspace
 def test_a_plan_of_many_parts_does_without_their_workspace(tiles, d):
     """num_splits = 0 leaves the count to the library: with no room for the partials of its plan the parts are as many as a
@@ -101,6 +102,8 @@ def test_a_plan_of_many_parts_does_without_their_workspace(tiles, d):
     from flash_attn_b200 import _lib
     L = _lib.load()
     H, Hk, Nk = 4, 1, 128 * tiles
+    got = plan(1, H, 1, Nk, d, heads_k=Hk)
+    assert got.parts > 16 and not got.merged
     g = torch.Generator(device="cuda")
     g.manual_seed(9)
     q, k, v = (torch.randn((1, h, n, d), generator=g, device="cuda").bfloat16() for h, n in ((H, 1), (Hk, Nk), (Hk, Nk)))
@@ -127,3 +130,27 @@ def test_a_plan_of_many_parts_does_without_their_workspace(tiles, d):
     assert (lse - want_lse).abs().max() <= gpu_util.LSE_ABS
     p.num_splits = 32  # a count of the caller's: its workspace is asked for, as ever
     assert L.fa_fwd(ctypes.byref(p)) == -3
+
+
+@pytest.mark.parametrize("B,H,Hk,Nq,nk,d,kw,columns,parts", [
+    (1, 12, 2, 3, 69, 128, {}, 4, 1),                 # a head's three rows a CTA: six CTAs per K/V head
+    (2, 64, 8, 5, 1848, 128, {}, 8, 1),               # (window) five rows a CTA
+    (1, 32, 8, 8, 590, 128, {}, 8, 4),
+    (4, 28, 4, 2, 700, 64, {}, 4, 4),                 # sub-groups of two heads, one of one
+    (16, 32, 8, 4, 4100, 128, {}, 16, 2),             # sixteen where CTAs are many
+    (1, 4, 1, 1, 262000, 64, {}, 4, 64),              # more parts than a cluster holds: the combine kernel
+])
+def test_columns_and_parts_of_the_plan(B, H, Hk, Nq, nk, d, kw, columns, parts):
+    kw = dict(kw)
+    if nk == 1848:
+        kw["window"] = (200, 0)
+    got = plan(B, H, Nq, nk, d, heads_k=Hk, causal=True, q_pos0=nk - Nq, **kw)
+    assert (got.columns, got.parts) == (columns, parts)
+    import flash_attn_b200 as fa
+    torch.manual_seed(60)
+    q, k, v = (torch.randn(B, h, n, d, device="cuda", dtype=torch.bfloat16) for h, n in ((H, Nq), (Hk, nk), (Hk, nk)))
+    o, lse = fa.flash_attn_forward(q, k, v, causal=True, q_pos0=nk - Nq, num_splits=0, **kw)
+    torch.cuda.synchronize()
+    units = sorted({0, H // Hk - 1, H // Hk % (B * H), B * H // 2, B * H - 1})
+    gpu_util.assert_close(gpu_util.check_sampled_units(q, k, v, o, lse, units, lambda u: range(Nq), d ** -0.5, causal=True,
+                                                       q_pos0=nk - Nq, **kw), str((B, H, Nq, nk, d, kw)))

@@ -59,3 +59,16 @@ def test_the_clusters_of_a_split_are_resident_at_once(sms, clusters, Nq, per_sm)
 ])
 def test_part_counts(B, H, Hk, Nq, Nk, causal, parts):
     assert plan(B, H, Nq, Nk, 128, heads_k=Hk, causal=causal, q_pos0=Nk - Nq if causal else 0).parts in parts
+
+
+def test_decode_on_a_device_without_clusters():
+    got = [plan(1, 8, Nq, Nk, 128, heads_k=2, num_splits=s, clusters=(0, 148) + (0,) * 15)
+           for Nq in (1, 4, 8) for Nk in (100, 5000, 300000) for s in (0, 1)]
+    assert all(p.decode and not p.merged for p in got) and any(p.parts > 16 for p in got)
+
+
+@pytest.mark.parametrize("splits", [1, 3, 4, 16, 20])
+def test_decode_with_dropout_keeps_the_callers_splits(splits):
+    for B, H, Hk, Nq in ((1, 8, 8, 1), (2, 64, 8, 3), (16, 32, 8, 4)):
+        got = plan(B, H, Nq, 5000, 128, heads_k=Hk, p_dropout=0.1, num_splits=splits)
+        assert got.parts == splits and got.merged == (splits in (4, 16))
