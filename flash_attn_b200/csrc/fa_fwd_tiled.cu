@@ -1358,8 +1358,8 @@ bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causa
 // without stacking: what it takes is 1 % slower than the best on average.  Where it leaves more than a tenth, blocks do not
 // fit the device at once ([160 blocks, 67 tiles] 231 us unsplit, 203 in three parts and four waves).
 //   A CTA takes `base` to start and drain and `rate` for a KV tile.  The rate grows with the CTAs at work: by `crowd` up to one an
-//   SM (L2 and HBM; grouped queries share their K/V), by `over` for a second one on the SM (single query tiles only).
-//   A split pays `merge` + `merge_each` a part for staging, two cluster barriers and the merge (its distributed-shared-memory
+//   SM (L2 and HBM; less where grouped queries share their K/V), by `over` for a second one on the SM (single query tiles only).
+//   A split (or a staged launch of one part) pays `merge` + `merge_each` a part for staging, two cluster barriers and the merge (its distributed-shared-memory
 //   reads run at about 11 bytes a clock and SM), part counts that are no power of two a little more, few rows less.
 //   It is taken only where all its clusters are resident at once (ClusterRoom): a second wave waits for whole clusters to
 //   leave.  [16 blocks, 19 tiles] 34.0 unsplit, 20.6 / 20.5 / 22.2 / 40.3 in 4 / 5 / 6 / 7 parts (15 clusters of 7 fit),
@@ -1403,7 +1403,10 @@ int block_tiles(const FwdArgs& a, long long qb, bool pair) {
 Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged) {
     const bool pair = two_tiles(a);
     Cost c = kCost[pair][a.head_dim > 64];
-    if (pair && (a.kv_group > 1 || a.pack_rows > 0)) c.crowd = std::min(c.crowd, 0.1);
+    if (a.kv_group > 1 || a.pack_rows > 0) {
+        c.crowd = std::min(c.crowd, pair ? 0.1 : 0.6);
+        c.over = std::min(c.over, 0.2);
+    }
     if (a.alibi_slopes != nullptr && !a.is_causal && a.window_right != 0) c.rate *= 1.6;  // (a bias per element)
     const long long per_unit = pair ? (a.tr + 1) / 2 : a.tr;
     const long long blocks = a.units * per_unit, slots = pair ? sms : 2 * sms;
@@ -1424,18 +1427,16 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
     }
     const int tile_rows = pair ? 2 * kTile : kTile;
     const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
-    const double stage = staged ? 0.3 * c.merge * rows : 0.0;
-    Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, least >= 0.8 * n};
+    const double stage = staged ? (c.merge + c.merge_each) * rows : 0.0;
+    Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, least >= 0.8 * n || n - least <= 1};
     if (blocks > slots) {
         const double waves = static_cast<double>(blocks) / slots;
         if (!best.even) {  // blocks of different lengths: the longest first, shorter ones fill up
             best.us = std::max(best.us, waves * (launch_us(c, static_cast<double>(slots), sms, mean) + stage));
-        } else if (pair) {  // of about one length: wave after wave
+        } else {  // of about one length: wave after wave
             const long long rest = blocks % slots;
             best.us *= static_cast<double>(blocks / slots);
             if (rest > 0) best.us += launch_us(c, static_cast<double>(rest), sms, n) + stage;
-        } else {  // two CTAs an SM get out of step
-            best.us *= waves;
         }
     }
     for (int parts = 2; parts <= ClusterRoom::kMax && parts <= n; parts += parts < 8 ? 1 : 8) {
@@ -1508,9 +1509,9 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
     // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the query
     // blocks are of about one length (tiles across heads have the longest: [4 x 12 heads on 2, 1940 rows, 1241 keys, causal]
-    // 72 us stacked, 50 not), it saves a tenth of the query tiles, and the model says 7 % and half a microsecond of the time:
-    // below that the staged epilogue, slower than TMA stores, eats the gain ([64 heads on 8, 720 rows, 25871 keys], 184
-    // blocks instead of 192: 714 us against 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all
+    // 72 us stacked, 50 not), it saves query tiles, and the model says 3 % and two microseconds of the time: a
+    // staged epilogue takes as long as a merge ([64 heads on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us
+    // against 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all
     // of a head's positions; those past a row's own come first, and the row starts afresh behind them, but those before a
     // left window would come last and bring masked infinities and NaN with them: with one, only heads of a single tile are
     // stacked, whose rows walked all of these tiles anyway.)
@@ -1523,9 +1524,8 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
         b.tr = static_cast<int>((rows + kTile - 1) / kTile);
         b.units = a->units / heads;
         b.kv_group = 1;
-        const bool fewer = 10LL * b.tr <= 9LL * heads * a->tr;
-        const Split packed = split.even && fewer ? best_split(b, sms, room, true) : Split{1, 1e30, true};
-        if (packed.us < 0.93 * split.us - 0.5) {
+        const Split packed = split.even && b.tr < heads * a->tr ? best_split(b, sms, room, true) : Split{1, 1e30, true};
+        if (packed.us < 0.97 * split.us - 2.0) {
             *a = b;
             split = packed;
         }

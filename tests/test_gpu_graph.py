@@ -47,3 +47,30 @@ def test_capture_and_replay_matches_eager():
         torch.cuda.synchronize()
         for a, b in zip(got[0] + got[1], want_o + want_l):
             assert torch.equal(a, b), f"replay {trial} differs from the eager launch"
+
+
+def test_the_first_calls_of_a_process_may_be_captured():
+    """What is asked of the runtime once (function attributes, resident clusters) is asked inside the capture here."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+import flash_attn_b200 as fa
+torch.manual_seed(4)
+mk = lambda *shape: torch.randn(*shape, device="cuda").bfloat16()
+q, k, v = mk(1, 8, 256, 128), mk(1, 8, 2400, 128), mk(1, 8, 2400, 128)      # split over clusters
+q1 = mk(1, 8, 1, 128)                                                       # decode, split over clusters
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    o, _ = fa.flash_attn_forward(q, k, v)
+    o1, _ = fa.flash_attn_forward(q1, k, v)
+g.replay()
+torch.cuda.synchronize()
+assert torch.equal(o, fa.flash_attn_forward(q, k, v)[0]) and torch.equal(o1, fa.flash_attn_forward(q1, k, v)[0])
+print("captured")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
