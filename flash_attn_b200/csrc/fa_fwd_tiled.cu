@@ -967,14 +967,14 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 const float f = rescale ? factor : 1.0f;
                 // A row that has seen no key yet starts from zero, whatever the masked values left (0 * inf, 0 * NaN):
                 // where heads are stacked a query tile walks KV tiles past those of its rows.
-                const bool fresh = kStaged && rescale && m_ref == -INFINITY;
+                const uint32_t seen = kStaged && rescale && m_ref == -INFINITY ? 0u : 0xffffffffu;
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c) {
                     uint32_t orow[32];
                     tmem_ld32(tmem_o + lane_base + c * 32, orow);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) orow[i] = fresh ? 0u : __float_as_uint(__uint_as_float(orow[i]) * f);
+                    for (int i = 0; i < 32; ++i) orow[i] = __float_as_uint(__uint_as_float(orow[i] & seen) * f);
                     tmem_st32(tmem_o + lane_base + c * 32, orow);
                 }
             }
