@@ -726,10 +726,10 @@ void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms, const 
         const double rate = cost.rate[i] + (dropout ? 0.12 * std::min(heads_per_cta, a->kv_group) : 0.0);
         // (with dropout the parts are the caller's splits, part of the streams' geometry)
         for (int p = 0, parts = dropout ? splits : 1; dropout || (parts <= most && (p == 0 || parts <= n)); ++p, parts *= 2) {
-            const bool merged = parts == 2 || parts == 4 || parts == 8 || parts == 16;
-            if (merged && !dropout && room.fits(parts, 2) == 0) continue;
+            const bool cluster = parts == 2 || parts == 4 || parts == 8 || parts == 16, merged = cluster && room.fits(parts, 2) > 0;
+            if (cluster && !merged && !dropout) continue;
             const long long ctas = static_cast<long long>(kv_units) * subgroups * parts;
-            const long long slots = merged && room.fits(parts, 2) > 0 ? static_cast<long long>(room.fits(parts, 2)) * parts : 2LL * sms;
+            const long long slots = merged ? static_cast<long long>(room.fits(parts, 2)) * parts : 2LL * sms;
             const double chain = cost.fixed[i] + rate * ((n + parts - 1) / parts);
             auto wave = [&](long long c) { return c > 0 ? chain * (1.0 + 0.166 * std::min(1.0, std::max(0.0, static_cast<double>(c) / sms - 1.0))) : 0.0; };
             double us = static_cast<double>(ctas / slots) * wave(slots) + wave(ctas % slots);

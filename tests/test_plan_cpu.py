@@ -72,3 +72,5 @@ def test_decode_with_dropout_keeps_the_callers_splits(splits):
     for B, H, Hk, Nq in ((1, 8, 8, 1), (2, 64, 8, 3), (16, 32, 8, 4)):
         got = plan(B, H, Nq, 5000, 128, heads_k=Hk, p_dropout=0.1, num_splits=splits)
         assert got.parts == splits and got.merged == (splits in (4, 16))
+        alone = plan(B, H, Nq, 5000, 128, heads_k=Hk, p_dropout=0.1, num_splits=splits, clusters=(0, 148) + (0,) * 15)
+        assert alone.parts == splits and not alone.merged  # (the combine kernel)
