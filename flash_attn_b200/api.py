@@ -58,9 +58,13 @@ def flash_attn_forward(q, k, v, softmax_scale=None, causal=False, window=(-1, -1
 
     q [B,H,Nq,d], k/v [B,Hk,Nk,d] (Hk divides H; query head h reads K/V head
     h // (H // Hk)), fp16 or bf16, contiguous.  `window` = (left,
-    right) with -1 = unbounded; `alibi_slopes` fp32 [H]; `num_splits` 0 = the
-    reference heuristic, 1 = none, n = forced; `q_pos0`/`k_pos0` = global positions
-    of row/column 0 (for one block of a sharded sequence).  Returns (o, lse).
+    right) with -1 = unbounded; `alibi_slopes` fp32 [H]; `q_pos0`/`k_pos0` = global
+    positions of row/column 0 (for one block of a sharded sequence).  Returns (o, lse).
+
+    `num_splits`: with dropout it is part of the mask's geometry, 0 = the reference's
+    heuristic, 1 = none, n = n.  Without dropout the library shares the keys out as
+    suits the device whatever the number says; n > 1 only asks for a workspace that
+    holds n splits' partials (and bounds the parts of a call of up to eight rows).
 
     `accum` = (o_acc fp32 [B,H,Nq,d], lse_acc fp32 [B,H,Nq]): the launch merges its
     result into this running pair in its epilogue (key blocks that arrive one launch

@@ -228,7 +228,8 @@ int planned_parts(const fa_fwd_params* p, int splits, int sms) {
     return d.merge ? 1 : d.parts;
 }
 // head_dim that is not a multiple of 8: Q/K/V are copied to a pitch of d8 = ceil8(head_dim)
-// elements (zero columns), the kernels run on the padded problem, O is copied back.
+// elements (zero columns) and the kernels run on the padded problem.  They write O with its own pitch; only the unsplit
+// dropout kernels for more than eight rows leave a padded O, which is re-pitched (its room is always part of the size).
 struct PadPlan {
     int d8;
     size_t q_bytes, kv_bytes, o_bytes, total;

@@ -22,7 +22,10 @@
 // tiles per thread), hence kernels for 1, 4, 8 and 16 columns, no mask arithmetic on chunks that no mask
 // touches, warp maxima by redux, and the running maxima kept one column per lane: [16 x 32 query heads on 8
 // K/V heads, 4097 keys] 56.3 -> 44.6 us (6.0 TB/s), of which 6 us are start and drain; [8 x 32 on 8, 4 rows,
-// 8000 keys] 90 -> 47 us (16 columns instead of two CTAs per K/V head).
+// 8000 keys] 90 -> 47 us (16 columns, four parts, instead of two CTAs per K/V head).  In the mask pass, the dropout draws and
+// the epilogue a division or a Philox block per column and tile is what a launch of few tiles spends its time on: slopes, rows
+// and draws are worked out once per column, head or tile ([64 heads on 4, 100 keys, 16 columns] 10.8 -> 9.7 us without the
+// divisions; [2 x 4 heads, 8 rows, 2971 keys, dropout] 97 -> 28 with one Philox block per head and tile).
 //
 // The parts of a unit (plan_decode) are the CTAs of one cluster: each leaves its un-normalised O, max and sum
 // in its own shared memory, and the CTAs share out the columns and merge them through distributed shared
@@ -59,7 +62,7 @@ constexpr int kDThreads = 192;
 constexpr int kDTmemCols = 256;            // S^T: 2 buffers x up to 4 tiles x 16 columns; O^T: 16 columns at 128
 
 // kH = columns in use of the 16 (queries that share the CTA's K/V): 1, 4, 8 or 16.  The work of the softmax
-// warps goes with kH, so the smallest that holds the queries is taken.  D = 64 or 128 (head_dim rounded up).
+// warps goes with kH (plan_decode weighs it against reading K/V once).  D = 64 or 128 (head_dim rounded up).
 template <int kH, int D>
 struct DCfg {
     // KV tiles per softmax chunk: with 16 columns two, which keeps P and the score registers at the size
@@ -208,8 +211,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant_
         mbar_init(bar_o_done, 1);
         mbar_fence_init();
     }
-    // kH = 1: one CTA per (query unit, part of its keys).  kH = 8: one CTA per (K/V unit, sub-group of up
-    // to eight of its query heads, part); `unit` is then the first query unit of the sub-group.
+    // kH = 1: one CTA per (query unit, part of its keys).  kH = 4, 8, 16: one CTA per (K/V unit, sub-group of its query
+    // heads whose rows fit kH columns, part); `unit` is then the first query unit of the sub-group.
     const int cta_unit = static_cast<int>(fast_div(a.div_parts, blockIdx.x));
     const int part = static_cast<int>(blockIdx.x) - cta_unit * a.parts;
     int unit, kv_unit, gh = 1;
@@ -700,7 +703,7 @@ void plan_decode(DecodeArgs* a, int units, int splits, int most, int sms, const 
     // How many columns a CTA has (query heads that share a K/V head are packed into one CTA, whole heads with their query rows;
     // what does not fit goes to further sub-groups, CTAs of their own that read the same K/V) and how many CTAs share a unit's
     // keys: the fastest by a model of the kernel's time, in us, fitted to 461 shapes of 8 to 512 K/V heads x 1 to 256 tiles, each
-    // swept over its columns and parts: what it takes is 0.2 % slower than the best on average, at most 8 %.
+    // swept over its columns and parts: what it takes is 0.3 % slower than the best on average, at most 14 %.
     //   A CTA takes `fixed` to start, mask and drain and `rate` for a K + V tile, a sixth more with a second CTA on its SM; what
     //   does not fit (two CTAs an SM, clusters as the device has room for them) follows in waves.  Columns cost by the CTA, since a
     //   softmax thread takes its key through all of them: sixteen pay only where CTAs are many or HBM bounds the launch ([1 x 64

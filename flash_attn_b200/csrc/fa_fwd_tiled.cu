@@ -1355,7 +1355,7 @@ bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causa
 
 // How many CTAs share the keys of a query block, and the time that takes (us).  The model is fitted to sweeps over 4 to 160
 // blocks x 4 to 67 KV tiles with every part count (D = 128 and 64, two query tiles a CTA and one) and over 81 grouped shapes with and
-// without stacking: what it takes is 1 % slower than the best on average.  Where it leaves more than a tenth, blocks do not
+// without stacking: what it takes is 0.5 % / 0.9 % slower than the best on average.  Where it leaves more than a tenth, blocks do not
 // fit the device at once ([160 blocks, 67 tiles] 231 us unsplit, 203 in three parts and four waves).
 //   A CTA takes `base` to start and drain and `rate` for a KV tile.  The rate grows with the CTAs at work: by `crowd` up to one an
 //   SM (L2 and HBM; less where grouped queries share their K/V), by `over` for a second one on the SM (single query tiles only).
@@ -1509,12 +1509,12 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
     // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the query
     // blocks are of about one length (tiles across heads have the longest: [4 x 12 heads on 2, 1940 rows, 1241 keys, causal]
-    // 72 us stacked, 50 not), it saves query tiles, and the model says 3 % and two microseconds of the time: a
-    // staged epilogue takes as long as a merge ([64 heads on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us
-    // against 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all
-    // of a head's positions; those past a row's own come first, and the row starts afresh behind them, but those before a
-    // left window would come last and bring masked infinities and NaN with them: with one, only heads of a single tile are
-    // stacked, whose rows walked all of these tiles anyway.)
+    // 72 us stacked, 50 not), it saves query tiles, and the model says 3 % and two microseconds of the time: a staged
+    // epilogue takes as long as a merge ([64 heads on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against
+    // 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all of a head's positions; those past a
+    // row's own come first, and the row starts afresh behind them, but those before a left window would come last and bring
+    // masked infinities and NaN with them: with one, only heads of a single tile are stacked, whose rows walked all of these
+    // tiles anyway.)
     const int heads = a->kv_group;
     const long long rows = static_cast<long long>(heads) * a->seqlen_q;
     if (heads > 1 && a->alibi_slopes == nullptr && rows <= 0x3fffffffLL && (a->window_left < 0 || a->seqlen_q <= kTile)) {

@@ -88,8 +88,9 @@ typedef struct fa_fwd_params {
     int* status;              /* device int or NULL.  Every wait inside the kernels is bounded (about 2 s of SM
                                  clocks); a wait that gives up stores a code here -- 100 + n from the tiled
                                  forward kernel, 200 + n from the decode kernel, n naming the wait -- and the
-                                 CTA drains and exits, leaving O and LSE undefined.  fa_fwd is asynchronous:
-                                 the caller clears the word before the launch and reads it after synchronising
+                                 CTA drains and exits, leaving O and LSE undefined (O is NaN in rows that
+                                 CTAs merge on chip: a part never passes for the whole).  fa_fwd is
+                                 asynchronous: the caller clears the word before the launch and reads it after synchronising
                                  the stream.  fa_fwd_host does both itself and returns FA_ERR_DEVICE_TIMEOUT. */
     void* stream;             /* cudaStream_t; NULL = default stream (the reference's)       */
     int heads_k;              /* K/V heads for grouped-query attention: K and V are
@@ -128,9 +129,10 @@ typedef struct fa_fwd_params {
  * Asynchronous on p->stream. */
 int fa_fwd(const fa_fwd_params* p);
 
-/* Bytes of workspace fa_fwd needs for p (0 when it neither keeps split partials nor pads head_dim).  With
+/* Bytes of workspace fa_fwd wants for p (0 when it neither keeps split partials nor pads head_dim).  With
  * num_splits = n > 1 the partials of n splits; with 0 those of the launch the library plans, which may merge
- * the parts on chip and keep none.
+ * the parts on chip and keep none.  Without dropout a call with num_splits = 0 also runs with no room for
+ * its partials (it is then cut into as many parts as merge on chip).
  * Replaces the cudaMalloc sizing of O_tmp/L/M at src/main.cu:160-162. */
 size_t fa_fwd_workspace_bytes(const fa_fwd_params* p);
 
