@@ -35,26 +35,26 @@ encode_tiled_fn get_encode_tiled() {
     return fn;
 }
 
-// [units, rows, d] 16-bit tensor, box = 64 elements x 128 rows x 1 unit, 128-byte
+// [units, rows, d] tensor of an FA_DTYPE_*, box = 128 bytes x 128 rows x 1 unit, 128-byte
 // swizzle; out-of-range rows and columns read as zero, which replaces the
 // reference's hand-written zero padding (include/utils.h:67-114).
-int make_tensor_map(CUtensorMap* m, bool bf16, const void* base, int d, long long rows, long long units,
+int make_tensor_map(CUtensorMap* m, int dtype, const void* base, int d, long long rows, long long units,
                     int box_rows = kTile) {
     // A tensor map is a pure function of these arguments, so the last few are kept per host thread:
     // a caller that runs the same buffers again (every layer of every step) skips the driver call.
     struct Entry {
         const void* base;
         long long rows, units;
-        int d, box_rows, bf16, valid;
+        int d, box_rows, dtype, valid;
         CUtensorMap map;
     };
-    constexpr int kEntries = 8;
+    constexpr int kEntries = 16;
     thread_local Entry cache[kEntries] = {};
     thread_local int next_victim = 0;
     for (int i = 0; i < kEntries; ++i) {
         const Entry& e = cache[i];
         if (e.valid && e.base == base && e.rows == rows && e.units == units && e.d == d && e.box_rows == box_rows &&
-            e.bf16 == static_cast<int>(bf16)) {
+            e.dtype == dtype) {
             *m = e.map;
             return FA_OK;
         }
@@ -62,16 +62,18 @@ int make_tensor_map(CUtensorMap* m, bool bf16, const void* base, int d, long lon
     encode_tiled_fn enc = get_encode_tiled();
     if (!enc) return FA_ERR_CUDA;
     cuuint64_t dims[3] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(units)};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(d) * 2, static_cast<cuuint64_t>(rows) * d * 2};
-    cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
+    const int bytes = dtype == FA_DTYPE_FP32 ? 4 : 2;
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(d) * bytes, static_cast<cuuint64_t>(rows) * d * bytes};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / bytes), static_cast<cuuint32_t>(box_rows), 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+    CUresult r = enc(m, dtype == FA_DTYPE_FP32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                        : dtype == FA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return FA_ERR_CUDA;
     Entry& e = cache[next_victim];
     next_victim = (next_victim + 1) % kEntries;
-    e.base = base; e.rows = rows; e.units = units; e.d = d; e.box_rows = box_rows; e.bf16 = bf16; e.map = *m; e.valid = 1;
+    e.base = base; e.rows = rows; e.units = units; e.d = d; e.box_rows = box_rows; e.dtype = dtype; e.map = *m; e.valid = 1;
     return FA_OK;
 }
 
@@ -292,19 +294,27 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
     const bool bf16 = p->dtype == FA_DTYPE_BF16;
     CUtensorMap tk, tv;
     const int units_k = p->batch * kv_heads(p);
-    if ((rc = make_tensor_map(&tk, bf16, p->k, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
-    if ((rc = make_tensor_map(&tv, bf16, p->v, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
+    if ((rc = make_tensor_map(&tk, p->dtype, p->k, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
+    if ((rc = make_tensor_map(&tv, p->dtype, p->v, p->head_dim, p->seqlen_k, units_k)) != FA_OK) return rc;
     if (decode) {
         // one to eight query rows per unit: the streaming kernel with keys on the tensor-memory lanes
         if (launch_decode(d, tk, tv, units, bf16, stream) != cudaSuccess) return FA_ERR_CUDA;
     } else {
         CUtensorMap tq;
-        if ((rc = make_tensor_map(&tq, bf16, p->q, p->head_dim, a.seqlen_q, a.units)) != FA_OK) return rc;
+        if ((rc = make_tensor_map(&tq, p->dtype, p->q, p->head_dim, a.seqlen_q, a.units)) != FA_OK) return rc;
         // 16-bit output of an unsplit launch is written by TMA stores, one 32-row box per warp
         CUtensorMap to = tq;
         a.o_tma = (!a.staged && a.num_splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
-        if (a.o_tma && (rc = make_tensor_map(&to, bf16, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
-        if (launch_fwd_tiled(a, tq, tk, tv, to, a.units, bf16, dropout, stream) != cudaSuccess) return FA_ERR_CUDA;
+        if (a.o_tma && (rc = make_tensor_map(&to, p->dtype, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
+        CUtensorMap tc = tq;
+        if (p->accum_o != nullptr) {
+            // the running result comes and goes by TMA too; the last block stores the output instead
+            const bool last = a.accum_final && p->o != nullptr;
+            if ((rc = make_tensor_map(&tc, FA_DTYPE_FP32, p->accum_o, p->head_dim, p->seqlen_q, units)) != FA_OK) return rc;
+            if ((rc = make_tensor_map(&to, last ? p->o_dtype : FA_DTYPE_FP32, last ? p->o : p->accum_o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK)
+                return rc;
+        }
+        if (launch_fwd_tiled(a, tq, tk, tv, to, tc, a.units, bf16, dropout, stream) != cudaSuccess) return FA_ERR_CUDA;
     }
     if (parts > 1) {
         CombineArgs c;

@@ -113,7 +113,8 @@ struct Cfg {
     static constexpr int kSmemK = NQ * kTileBytes;
     static constexpr int kSmemV = kSmemK + kStages * kTileBytes;
     static constexpr int kSmemBar = kSmemV + kStages * kTileBytes;
-    static constexpr int kNumBars = 1 + 2 * NQ + 4 * kStages;
+    static constexpr int kNumBars = 2 + 3 * NQ + 4 * kStages;
+    static_assert(kNumBars <= 32, "a lane initialises each");
     // dropout keep bits, written by a helper warp per query tile: [NQ][2 row halves][kKeepRing tiles] words
     static constexpr int kSmemKeep = kSmemBar + 8 * kNumBars + 16;
     static constexpr int kSmemBytes = kSmemKeep + NQ * kKeepRing * 2 * 4 + 1024;  // + alignment slack
@@ -436,11 +437,14 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
     }
 }
 
-template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged>
+// kRunning: the launch may merge into a running result.  Without dropout every unstaged kernel may (the code costs it nothing);
+// with dropout those that do not are kernels of their own: the schedule that ptxas finds for their softmax loop beside it takes
+// 3 % more ([8,16,2048,128] causal, p = 0.1: 171.5 us against 167.1 under the power cap).
+template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, bool kRunning>
 __global__ void __launch_bounds__(Cfg<D, NQ>::kThreads, NQ == 1 ? 2 : 1)
 fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
-                 const FwdArgs a) {
+                 const __grid_constant__ CUtensorMap tmap_c, const FwdArgs a) {
     using C = Cfg<D, NQ>;
     extern __shared__ uint8_t smem_raw[];
     // 128-byte-swizzled tiles need a 1024-byte aligned base
@@ -458,6 +462,8 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t bar_k_empty = bar_k_full + 8 * C::kStages;    // [kStages]
     const uint32_t bar_v_full = bar_k_empty + 8 * C::kStages;    // [kStages]
     const uint32_t bar_v_empty = bar_v_full + 8 * C::kStages;    // [kStages]
+    const uint32_t bar_qk_done = bar_v_empty + 8 * C::kStages;   // running result only: Q and the K ring are free
+    const uint32_t bar_carry = bar_qk_done + 8;                  // [NQ] carried rows have landed
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kSmemBar + 8 * C::kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + C::kSmemBar + 8 * C::kNumBars + 4);
     volatile uint32_t* keep_tab = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kSmemKeep);
@@ -680,15 +686,20 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t tmem_base = (n_union > 0) ? *tmem_slot : 0u;
 
     int fail = 0;
+    // Rows carried from launch to launch: they lie, 32 fp32 columns a box, in the Q buffer of their query tile and in a stage of the K ring.
+    const bool carry = kRunning && a.accum_o != nullptr && !a.accum_first;
+    auto carry_box = [&](int i, int b) {
+        return b < C::kBoxes ? sQ + i * C::kTileBytes + b * (kTile * 128) : sK + i * C::kTileBytes + (b - C::kBoxes) * (kTile * 128);
+    };
 
     // The helper warpgroup (producer, MMA issuer, two idle warps) hands most of its registers to
     // the softmax warpgroups, which hold a 128-column score row per thread.  Each register
     // regime covers one whole branch below.
     if (warp >= NQ * 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsHelper));
-        if (n_union > 0 && warp == C::kProducerWarp) {
+        if (warp == C::kProducerWarp) {
             // ======================= TMA producer ===================================
-            if (lane == 0) {
+            if (n_union > 0 && lane == 0) {
                 for (int t = prefilled; t < n_union; ++t) {
                     if (FA_TEST_SKIPS(t)) continue;
                     const int st = t % C::kStages;
@@ -706,6 +717,20 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
                     for (int b = 0; b < C::kBoxes; ++b)
                         tma_load_3d(sV + st * C::kTileBytes + b * (kTile * 128), &tmap_v, bar_v_full + 8 * st, b * 64, row, kv_unit);
+                }
+            }
+            if (kRunning && carry) {
+                // The carried rows start as soon as the last Q K^T has read the buffers that take them, about a tile and a half
+                // ahead of their use (a CTA without keys: Q has landed before the CTA-wide sync).
+                __syncwarp();
+                static_assert(2 * C::kBoxes * NQ <= 32, "a lane issues each box");
+                const bool free = n_union == 0 || __shfl_sync(0xffffffffu, lane == 0 && fail == 0 && mbar_wait(bar_qk_done, 0, abort_flag) ? 1 : 0, 0) != 0;
+                const int i = lane % NQ, b = lane / NQ;
+                if (free && b < 2 * C::kBoxes && qb * NQ + i < a.tr) {
+                    if (b == 0) mbar_expect_tx(bar_carry + 8 * i, 2 * C::kTileBytes);
+                    tma_load_3d(carry_box(i, b), &tmap_c, bar_carry + 8 * i, b * 32, (qb * NQ + i) * kTile, unit);
+                } else if (!free && fail == 0) {
+                    fail = 10;
                 }
             }
         } else if (n_union > 0 && warp == C::kMmaWarp) {
@@ -757,6 +782,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                         }
                     }
                     umma_commit(bar_k_empty);
+                    if (kRunning && n_union == 1) umma_commit(bar_qk_done);
                 }
                 for (int t = 0; t < n_union && fail == 0; ++t) {
                     const int tile = hi - 1 - t;
@@ -800,6 +826,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                     if (leader) {
                         umma_commit(bar_v_empty + 8 * st);
                         if (more) umma_commit(bar_k_empty + 8 * st1);
+                        if (kRunning && t + 2 == n_union) umma_commit(bar_qk_done);
                     }
                 }
             } while (false);
@@ -1099,7 +1126,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         //   lse' = log(e^lse_c + e^lse),  O' = e^(lse_c - lse') O_c + e^(lse - lse') O,
         // here in the epilogue, on the row each thread already holds, instead of in a pass of its own.
         float w_old = 0.0f;  // weight of the carried row
-        if (a.accum_o != nullptr) {
+        if (kRunning && a.accum_o != nullptr) {
             const long long arow = unit_ll * a.seqlen_q + row;
             float lse_c = -INFINITY;
             if (!a.accum_first && row_ok) lse_c = a.accum_lse[arow];
@@ -1157,6 +1184,67 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             FA_TR(97);
             if (lane == 0) tma_store_wait_read();
+        } else if (kRunning && a.accum_o != nullptr) {
+            // Read-modify-write of the carried row, 32 columns at a time, in the box that its TMA load has brought; each warp stores
+            // its 32 rows of a box.  The sequence's last block leaves the 16-bit output instead, over the boxes it has read.
+            // Bound by the latency of a CTA's end (one CTA an SM: nothing overlaps it): a thread that read and wrote its own row in
+            // memory waited four times for its loads.  [1,32,8192,128] x 8192 keys: first block 462 -> 450 us (causal), one in the
+            // middle 912 -> 863, the last 893 -> 855; [2,4,333,96] x 777 keys 21.7 -> 13.4.  Whole lines by coalesced loads
+            // from a staged copy, without the early TMA loads, measured 914.
+            const bool out16 = a.accum_final && a.o != nullptr && !a.o_is_fp32;
+            if ((carry || n_union > 0) && rb < a.tr && !mbar_wait_warp(carry ? bar_carry + 8 * qi : bar_qk_done, 0, abort_flag) && fail == 0) fail = 11;
+            const int y0 = rb * kTile + (warp & 3) * 32;
+#pragma unroll 1
+            for (int b = 0; b < (rb < a.tr ? D / 32 : 0); ++b) {  // (beyond the last query tile the buffers are not this group's)
+                uint32_t orow[32];
+                if (have_o) {
+                    tmem_ld32(tmem_o + lane_base + b * 32, orow);
+                    tmem_wait_ld();
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) orow[i] = 0u;
+                }
+                const uint32_t row_addr = carry_box(qi, b) + r * 128;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const uint32_t at = row_addr + static_cast<uint32_t>((i >> 2) ^ (r & 7)) * 16;
+                    float4 v4 = make_float4(__uint_as_float(orow[i]) * inv, __uint_as_float(orow[i + 1]) * inv,
+                                            __uint_as_float(orow[i + 2]) * inv, __uint_as_float(orow[i + 3]) * inv);
+                    if (w_old != 0.0f) {
+                        const float4 c4 = ld_shared_f32x4(at);
+                        v4.x = fmaf(w_old, c4.x, v4.x);
+                        v4.y = fmaf(w_old, c4.y, v4.y);
+                        v4.z = fmaf(w_old, c4.z, v4.z);
+                        v4.w = fmaf(w_old, c4.w, v4.w);
+                    }
+                    orow[i] = __float_as_uint(v4.x);
+                    orow[i + 1] = __float_as_uint(v4.y);
+                    orow[i + 2] = __float_as_uint(v4.z);
+                    orow[i + 3] = __float_as_uint(v4.w);
+                    if (!out16) st_shared_v4(at, orow[i], orow[i + 1], orow[i + 2], orow[i + 3]);
+                }
+                if (out16) {
+                    // columns 32 b .. 32 b + 31 are half of a 64-column box
+                    const uint32_t out_addr = carry_box(qi, b & ~1) + r * 128;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        const uint32_t chunk = static_cast<uint32_t>((b & 1) * 4 + (i >> 3)) ^ static_cast<uint32_t>(r & 7);
+                        st_shared_v4(out_addr + chunk * 16, pack2<kBf16>(__uint_as_float(orow[i]), __uint_as_float(orow[i + 1])),
+                                     pack2<kBf16>(__uint_as_float(orow[i + 2]), __uint_as_float(orow[i + 3])),
+                                     pack2<kBf16>(__uint_as_float(orow[i + 4]), __uint_as_float(orow[i + 5])),
+                                     pack2<kBf16>(__uint_as_float(orow[i + 6]), __uint_as_float(orow[i + 7])));
+                    }
+                    if ((b & 1) == 0) continue;
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                const int first = out16 ? b & ~1 : b;
+                if (lane == 0 && y0 < a.seqlen_q && first * 32 < a.head_dim) {
+                    tma_store_3d(&tmap_o, carry_box(qi, first) + (warp & 3) * (32 * 128), first * 32, y0, unit);
+                    tma_store_commit();
+                }
+            }
+            if (lane == 0) tma_store_wait_read();
         } else {
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -1170,54 +1258,6 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             if (!row_ok) continue;
             const int col0 = c * 32;
-            if (a.accum_o != nullptr) {
-                // merged row: read-modify-write of the carried fp32 row (each thread walks its own row;
-                // the two 16-byte halves of every 32-byte sector are touched by consecutive
-                // instructions), and on the sequence's last block the 16-bit output as well
-                float* acc = a.accum_o + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    if (col0 + i < a.head_dim) {
-                        float4 v4 = make_float4(__uint_as_float(orow[i]) * inv, __uint_as_float(orow[i + 1]) * inv,
-                                                __uint_as_float(orow[i + 2]) * inv, __uint_as_float(orow[i + 3]) * inv);
-                        if (w_old != 0.0f) {
-                            const float4 c4 = *reinterpret_cast<const float4*>(acc + col0 + i);
-                            v4.x = fmaf(w_old, c4.x, v4.x);
-                            v4.y = fmaf(w_old, c4.y, v4.y);
-                            v4.z = fmaf(w_old, c4.z, v4.z);
-                            v4.w = fmaf(w_old, c4.w, v4.w);
-                        }
-                        if (!a.accum_final || a.o == nullptr) *reinterpret_cast<float4*>(acc + col0 + i) = v4;
-                        orow[i] = __float_as_uint(v4.x);
-                        orow[i + 1] = __float_as_uint(v4.y);
-                        orow[i + 2] = __float_as_uint(v4.z);
-                        orow[i + 3] = __float_as_uint(v4.w);
-                    }
-                }
-                if (a.accum_final && a.o != nullptr) {
-                    if (a.o_is_fp32) {
-                        float* dst = static_cast<float*>(a.o) + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            if (col0 + i < a.head_dim)
-                                *reinterpret_cast<uint4*>(dst + col0 + i) = make_uint4(orow[i], orow[i + 1], orow[i + 2], orow[i + 3]);
-                    } else {
-                        uint16_t* dst = static_cast<uint16_t*>(a.o) + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            if (col0 + i < a.head_dim) {
-                                uint4 v4;
-                                v4.x = pack2<kBf16>(__uint_as_float(orow[i]), __uint_as_float(orow[i + 1]));
-                                v4.y = pack2<kBf16>(__uint_as_float(orow[i + 2]), __uint_as_float(orow[i + 3]));
-                                v4.z = pack2<kBf16>(__uint_as_float(orow[i + 4]), __uint_as_float(orow[i + 5]));
-                                v4.w = pack2<kBf16>(__uint_as_float(orow[i + 6]), __uint_as_float(orow[i + 7]));
-                                *reinterpret_cast<uint4*>(dst + col0 + i) = v4;
-                            }
-                        }
-                    }
-                }
-                continue;
-            }
             if (a.num_splits > 1 || a.o_is_fp32) {
                 float* dst = (a.num_splits > 1)
                                  ? a.o_partial + ((unit_ll * a.num_splits + split) * a.seqlen_q + row) * a.head_dim
@@ -1277,10 +1317,10 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
 }
 
-template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged>
+template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, bool kRunning>
 cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                       const CUtensorMap& to, int units, cudaStream_t stream) {
-    auto kern = fwd_tiled_kernel<D, NQ, kBf16, kAlibi, kDropout, kStaged>;
+                       const CUtensorMap& to, const CUtensorMap& tc, int units, cudaStream_t stream) {
+    auto kern = fwd_tiled_kernel<D, NQ, kBf16, kAlibi, kDropout, kStaged, kRunning>;
     constexpr int smem = (kAlibi && Cfg<D, NQ>::kBiasBoxes) ? Cfg<D, NQ>::kSmemBytesBias : Cfg<D, NQ>::kSmemBytes;
     static_assert(smem <= 232448, "beyond the 227 KB a CTA may have");
     static std::atomic<bool> configured[64];
@@ -1322,28 +1362,31 @@ cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, 
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         if (a.parts > 1) cfg.numAttrs = 2;
     }
-    return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, a);
+    return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, tc, a);
 }
 
 template <int D, int NQ, bool kBf16>
 cudaError_t launch_flags(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const CUtensorMap& to, int units, bool alibi, bool dropout, cudaStream_t stream) {
+                         const CUtensorMap& to, const CUtensorMap& tc, int units, bool alibi, bool dropout, cudaStream_t stream) {
     if (a.staged)  // (never with dropout)
-        return alibi ? launch_one<D, NQ, kBf16, true, false, true>(a, tq, tk, tv, to, units, stream)
-                     : launch_one<D, NQ, kBf16, false, false, true>(a, tq, tk, tv, to, units, stream);
+        return alibi ? launch_one<D, NQ, kBf16, true, false, true, false>(a, tq, tk, tv, to, tc, units, stream)
+                     : launch_one<D, NQ, kBf16, false, false, true, false>(a, tq, tk, tv, to, tc, units, stream);
+    if (dropout && a.accum_o != nullptr)
+        return alibi ? launch_one<D, NQ, kBf16, true, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
+                     : launch_one<D, NQ, kBf16, false, true, false, true>(a, tq, tk, tv, to, tc, units, stream);
     if (alibi) {
-        return dropout ? launch_one<D, NQ, kBf16, true, true, false>(a, tq, tk, tv, to, units, stream)
-                       : launch_one<D, NQ, kBf16, true, false, false>(a, tq, tk, tv, to, units, stream);
+        return dropout ? launch_one<D, NQ, kBf16, true, true, false, false>(a, tq, tk, tv, to, tc, units, stream)
+                       : launch_one<D, NQ, kBf16, true, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
     }
-    return dropout ? launch_one<D, NQ, kBf16, false, true, false>(a, tq, tk, tv, to, units, stream)
-                   : launch_one<D, NQ, kBf16, false, false, false>(a, tq, tk, tv, to, units, stream);
+    return dropout ? launch_one<D, NQ, kBf16, false, true, false, false>(a, tq, tk, tv, to, tc, units, stream)
+                   : launch_one<D, NQ, kBf16, false, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
 }
 
 template <int D, int NQ>
 cudaError_t launch_dtype(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const CUtensorMap& to, int units, bool bf16, bool alibi, bool dropout, cudaStream_t stream) {
-    return bf16 ? launch_flags<D, NQ, true>(a, tq, tk, tv, to, units, alibi, dropout, stream)
-                : launch_flags<D, NQ, false>(a, tq, tk, tv, to, units, alibi, dropout, stream);
+                         const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool alibi, bool dropout, cudaStream_t stream) {
+    return bf16 ? launch_flags<D, NQ, true>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream)
+                : launch_flags<D, NQ, false>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream);
 }
 
 // two query tiles per CTA once a unit has more than one; a single tile (decode-like
@@ -1466,7 +1509,7 @@ ClusterRoom cluster_room(int sms) {
     if (known && ready[dev].load(std::memory_order_acquire)) return kept[dev];
     ClusterRoom room = {};
     room.one_per_sm[1] = sms;
-    auto kern = fwd_tiled_kernel<128, 2, true, false, false, true>;  // (one CTA an SM)
+    auto kern = fwd_tiled_kernel<128, 2, true, false, false, true, false>;  // (one CTA an SM)
     constexpr int smem = Cfg<128, 2>::kSmemBytes;
     bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
               cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
@@ -1535,15 +1578,15 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
 }
 
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                             const CUtensorMap& to, int units, bool bf16, bool dropout, cudaStream_t stream) {
+                             const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream) {
     const bool alibi = a.alibi_slopes != nullptr;
     const bool pair = two_tiles(a);
     if (a.head_dim <= 64) {
-        return pair ? launch_dtype<64, 2>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream)
-                    : launch_dtype<64, 1>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream);
+        return pair ? launch_dtype<64, 2>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream)
+                    : launch_dtype<64, 1>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);
     }
-    return pair ? launch_dtype<128, 2>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream)
-                : launch_dtype<128, 1>(a, tq, tk, tv, to, units, bf16, alibi, dropout, stream);
+    return pair ? launch_dtype<128, 2>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream)
+                : launch_dtype<128, 1>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);
 }
 
 }  // namespace fa

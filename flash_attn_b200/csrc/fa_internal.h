@@ -79,10 +79,11 @@ ClusterRoom cluster_room(int sms);  // of the current device; none above one CTA
 // problem with the heads of a K/V head stacked: units, heads, kv_group, seqlen_q, tr, pack_rows).
 void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room);
 
-// Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O
-// (32-row boxes); it is read only when a.o_tma is set.
+// Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O, or of the running
+// result where the launch leaves that (32-row boxes); it is read only when a.o_tma or a.accum_o is set.  `tc` is the load
+// map of the running result, read only when a.accum_o is set and something is carried.
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                             const CUtensorMap& to, int units, bool bf16, bool dropout, cudaStream_t stream);
+                             const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream);
 
 // Device-side argument block of the decode kernel (seqlen_q <= 8).
 struct DecodeArgs {

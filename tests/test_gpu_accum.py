@@ -53,6 +53,47 @@ def test_blocks_merged_in_the_epilogue_match_the_oracle(case):
     assert torch.equal(acc[1], lse)
 
 
+@pytest.mark.parametrize("Nq,d,dtype,out_dtype,causal", [
+    (257, 96, "bfloat16", None, True),         # a CTA whose second query tile does not exist
+    (385, 128, "float16", torch.float32, False),
+    (129, 64, "float16", torch.float32, True),
+    (127, 8, "bfloat16", None, False),         # one query tile, one box of columns
+    (300, 40, "bfloat16", None, True),
+    (640, 128, "bfloat16", torch.float32, True),
+])
+def test_running_rows_at_the_edges_of_tiles_and_boxes(Nq, d, dtype, out_dtype, causal):
+    # the carried rows travel in boxes of 32 columns over Q's and K's buffers: remainders of rows and columns, single KV tiles,
+    # blocks that some query tiles do not see at all, rows before and behind the tensor that nobody may touch
+    import flash_attn_b200 as fa
+    B, H, blocks = 2, 3, (130, 100, 300)
+    Nk = sum(blocks)
+    qn, kn, vn = synth.qkv(62, B, H, Nq, Nk, d, dtype, 0.7)
+    q, k, v = (gpu_util.to_dev(x, dtype) for x in (qn, kn, vn))
+    room = torch.full((B * H * Nq * d + 2048,), 7.0, device="cuda")
+    acc = (room[1024:-1024].view(B, H, Nq, d), torch.full((B, H, Nq), float("nan"), device="cuda"))
+    acc[0].fill_(float("nan"))
+    pos = 0
+    for i, n in enumerate(blocks):
+        o, lse = fa.flash_attn_forward(q, k[:, :, pos:pos + n].contiguous(), v[:, :, pos:pos + n].contiguous(), causal=causal,
+                                       k_pos0=pos, accum=acc, accum_first=i == 0, accum_final=i + 1 == len(blocks), out_dtype=out_dtype)
+        pos += n
+        want_o, want_lse = oracle_lib.forward(qn, kn[:, :, :pos], vn[:, :, :pos], d ** -0.5, causal=causal)
+        got_o, got_lse = (acc[0], acc[1]) if o is None else (o, lse)
+        assert np.abs(got_o.float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
+        assert np.abs(got_lse.cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
+    assert torch.equal(room[:1024], torch.full_like(room[:1024], 7.0)) and torch.equal(room[-1024:], torch.full_like(room[:1024], 7.0))
+
+
+@pytest.mark.parametrize("Nq,d", [(100, 64), (300, 128)])
+def test_one_block_with_dropout_equals_the_plain_launch(Nq, d):
+    import flash_attn_b200 as fa
+    q, k, v = (gpu_util.to_dev(x, "bfloat16") for x in synth.qkv(63, 1, 4, Nq, 400, d, "bfloat16"))
+    acc = (torch.empty((1, 4, Nq, d), device="cuda"), torch.empty((1, 4, Nq), device="cuda"))
+    plain = fa.flash_attn_forward(q, k, v, p_dropout=0.3, seed=5)
+    run = fa.flash_attn_forward(q, k, v, p_dropout=0.3, seed=5, accum=acc, accum_first=True, accum_final=True)
+    assert torch.equal(plain[0], run[0]) and torch.equal(plain[1], run[1])
+
+
 def test_rows_that_see_nothing_in_a_block_keep_their_running_result():
     # causal with the second block wholly after the first 128 queries: those rows must come through unchanged
     import flash_attn_b200 as fa
