@@ -437,9 +437,9 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
     }
 }
 
-// kRunning: the launch may merge into a running result.  Without dropout every unstaged kernel may (the code costs it nothing);
-// with dropout those that do not are kernels of their own: the schedule that ptxas finds for their softmax loop beside it takes
-// 3 % more ([8,16,2048,128] causal, p = 0.1: 171.5 us against 167.1 under the power cap).
+// kRunning: the launch merges into a running result.  Those kernels are instances of their own: with that epilogue in every
+// kernel a short launch takes longer ([4,16,512,128] causal 11.4 us against 11.15) and ptxas finds the dropout kernels' softmax
+// loop another schedule ([8,16,2048,128] causal, p = 0.1: 171.5 us against 168 under the power cap).
 template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, bool kRunning>
 __global__ void __launch_bounds__(Cfg<D, NQ>::kThreads, NQ == 1 ? 2 : 1)
 fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -1371,15 +1371,20 @@ cudaError_t launch_flags(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
     if (a.staged)  // (never with dropout)
         return alibi ? launch_one<D, NQ, kBf16, true, false, true, false>(a, tq, tk, tv, to, tc, units, stream)
                      : launch_one<D, NQ, kBf16, false, false, true, false>(a, tq, tk, tv, to, tc, units, stream);
-    if (dropout && a.accum_o != nullptr)
-        return alibi ? launch_one<D, NQ, kBf16, true, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
-                     : launch_one<D, NQ, kBf16, false, true, false, true>(a, tq, tk, tv, to, tc, units, stream);
+    if (a.accum_o != nullptr) {
+        if (alibi) {
+            return dropout ? launch_one<D, NQ, kBf16, true, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
+                           : launch_one<D, NQ, kBf16, true, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+        }
+        return dropout ? launch_one<D, NQ, kBf16, false, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
+                       : launch_one<D, NQ, kBf16, false, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+    }
     if (alibi) {
         return dropout ? launch_one<D, NQ, kBf16, true, true, false, false>(a, tq, tk, tv, to, tc, units, stream)
-                       : launch_one<D, NQ, kBf16, true, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+                       : launch_one<D, NQ, kBf16, true, false, false, false>(a, tq, tk, tv, to, tc, units, stream);
     }
     return dropout ? launch_one<D, NQ, kBf16, false, true, false, false>(a, tq, tk, tv, to, tc, units, stream)
-                   : launch_one<D, NQ, kBf16, false, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+                   : launch_one<D, NQ, kBf16, false, false, false, false>(a, tq, tk, tv, to, tc, units, stream);
 }
 
 template <int D, int NQ>
