@@ -157,6 +157,24 @@ int resolve_splits(const fa_fwd_params* p, int sms) {
     return std::max(1, std::min(s, tc));
 }
 
+// Units whose CTAs are interleaved in launch order.  Query blocks of one length (no mask that shortens the first ones by more
+// than a fifth) go unit by unit, which keeps neighbouring CTAs on the same K/V tiles in L2: [1,32,8192,128] against 8192 keys
+// before it 837 us in groups of 16, 812 unit by unit.  Causal blocks go heaviest first over groups of 16 units, near a
+// longest-job-first schedule ([8,16,2048,128] 142 us, 148 unit by unit; 8192 rows 435 and 473), or of fewer where a
+// group's K/V would pass 48 MB (L2 holds 126 MB in two halves): [1,32,16384,128] 1684 us in groups of 16, 1655 / 1651 / 1672 of
+// 8 / 4 / 2, [1,16,32768,128] 3276 against 3242 / 3217 / 3215.  (Powers of two: groups of 6 leave one of 2 behind and take 1729.)
+int unit_group(const fa_fwd_params* p, int kv_group) {
+    if (!p->is_causal || p->window_left >= 0) return 1;
+    const long long nk = p->seqlen_k, start = p->q_pos0 - p->k_pos0;
+    auto visible = [&](long long row) { return std::max(0LL, std::min(nk, start + row + 1)); };
+    const long long first = visible(std::min(p->seqlen_q, 2 * kTile) - 1), last = visible(p->seqlen_q - 1);
+    if (5 * first >= 4 * last) return 1;
+    const double unit_bytes = 4.0 * static_cast<double>(last) * p->head_dim / kv_group;
+    int units = 16;
+    while (units > 1 && units * unit_bytes > 48.0 * 1048576.0) units /= 2;
+    return units;
+}
+
 void fill_args(const fa_fwd_params* p, int splits, FwdArgs* a) {
     std::memset(a, 0, sizeof(*a));
     a->o = p->o;
@@ -166,9 +184,7 @@ void fill_args(const fa_fwd_params* p, int splits, FwdArgs* a) {
     a->heads = p->heads;
     a->units = p->batch * p->heads;
     a->kv_group = p->heads / kv_heads(p);
-    // query blocks of very different cost (causal, no left window): heaviest-first over groups of
-    // 16 units; otherwise unit-major, which keeps neighbouring CTAs on the same K/V tiles in L2
-    a->unit_group = (p->is_causal && p->window_left < 0) ? 16 : 1;
+    a->unit_group = unit_group(p, a->kv_group);
     a->seqlen_q = p->seqlen_q;
     a->seqlen_k = p->seqlen_k;
     a->head_dim = p->head_dim;
