@@ -3,6 +3,7 @@
 There is no fallback: if the library is missing or fails to load, importing the
 compute entry points raises."""
 import ctypes
+import functools
 import os
 import struct
 
@@ -169,6 +170,8 @@ def load():
     L.fa_strerror.restype = ctypes.c_char_p
     L.fa_version.argtypes = []
     L.fa_version.restype = ctypes.c_int
+    from . import _call  # the call path on torch tensors (csrc/fa_torch.cpp), bound to this library's entry points
+    L.forward = functools.partial(_call.forward, *(ctypes.cast(f, ctypes.c_void_p).value for f in (L.fa_fwd, L.fa_fwd_workspace_bytes)))
     _lib = L
     return L
 

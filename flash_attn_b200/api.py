@@ -72,59 +72,13 @@ def flash_attn_forward(q, k, v, softmax_scale=None, causal=False, window=(-1, -1
     `accum_final` the last one, and only that call writes and returns (o, lse) --
     the others return (None, None).
     """
-    L = _lib.load()
-    if not q.is_cuda:
-        raise ValueError("flash_attn_forward needs CUDA tensors (use flash_attn_forward_host for host buffers)")
-    B, H, Nq, d = q.shape
-    device = q.device
-    writes_output = accum is None or accum_final
-    if out is None and writes_output:
-        out = torch.empty((B, H, Nq, d), device=device, dtype=out_dtype or q.dtype)
-    lse = torch.empty((B, H, Nq), device=device, dtype=torch.float32) if (return_lse and writes_output) else None
-    if alibi_slopes is not None:
-        alibi_slopes = alibi_slopes.to(device=device, dtype=torch.float32).contiguous()
-    if not writes_output:
-        out = None
-    o = out if out is not None else q
-    _check(q, k, v, o)
-    accum_ptrs, flags = (0, 0), 0
-    if accum is not None:
-        o_acc, lse_acc = accum
-        if o_acc.dtype != torch.float32 or lse_acc.dtype != torch.float32 or not o_acc.is_contiguous() or \
-                not lse_acc.is_contiguous() or o_acc.shape != (B, H, Nq, d) or lse_acc.shape != (B, H, Nq):
-            raise ValueError("accum = (fp32 [B,H,Nq,d], fp32 [B,H,Nq]), contiguous")
-        accum_ptrs = (o_acc.data_ptr(), lse_acc.data_ptr())
-        flags = (_lib.FA_ACCUM_FIRST if accum_first else 0) | (_lib.FA_ACCUM_FINAL if accum_final else 0)
-    # A short call is bound by this function, not by its kernel, so the parameter block is packed in one go (thirty-odd
-    # attribute stores of a ctypes structure took 4 us), the device is only switched when it is another one, and the
-    # workspace is only asked for where one can be needed.  One call of [1,4,256,256,64] took 18.5 us
-    # and takes 13.6, with num_splits = 0 23.4 and 14.8, of which the two allocations are 5 and the native call 4.
-    head = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if out is not None else 0,
-            lse.data_ptr() if lse is not None else 0, _DT[q.dtype], _DT[o.dtype], B, H, Nq, k.shape[2], d,
-            float(softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(d)), int(bool(causal)),
-            int(window[0]), int(window[1]), alibi_slopes.data_ptr() if alibi_slopes is not None else 0,
-            float(p_dropout), int(seed), int(offset), int(unit0), int(num_splits), int(q_pos0), int(k_pos0))
-    tail = (k.shape[1],) + accum_ptrs + (flags, int(launch_index))
-    status_ptr = status.data_ptr() if status is not None else 0
-
-    def launch():
-        nonlocal workspace
-        ws = (0, 0)
-        if num_splits != 1 or d % 8 != 0:
-            need = L.fa_fwd_workspace_bytes(_lib.pack_params(*head, 0, 0, status_ptr, 0, *tail))
-            if need:
-                if workspace is None or workspace.numel() * workspace.element_size() < need:
-                    workspace = torch.empty(need, device=device, dtype=torch.uint8)
-                ws = (workspace.data_ptr(), workspace.numel() * workspace.element_size())
-        stream = torch._C._cuda_getCurrentRawStream(device.index)
-        _lib.check(L.fa_fwd(_lib.pack_params(*head, *ws, status_ptr, stream, *tail)), "fa_fwd")
-
-    if device.index == torch.cuda.current_device():
-        launch()
-    else:
-        with torch.cuda.device(device):
-            launch()
-    return out, lse
+    # (the whole call is native: see csrc/fa_torch.cpp)
+    done = _lib.load().forward(q, k, v, softmax_scale, causal, window, alibi_slopes, p_dropout, seed, offset, num_splits, out,
+                               out_dtype, return_lse, q_pos0, k_pos0, unit0, workspace, status, accum, accum_first,
+                               accum_final, launch_index)
+    if type(done) is int:
+        _lib.check(done, "fa_fwd")
+    return done
 
 
 def flash_attn_forward_host(q, k, v, softmax_scale=None, causal=False, window=(-1, -1), alibi_slopes=None,

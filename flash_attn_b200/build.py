@@ -1,4 +1,4 @@
-"""Builds libfa_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libfa_b200.so (the C-ABI library, nvcc for sm_100a) and _call.so (its call path on torch tensors) in-tree.
 
     python -m flash_attn_b200.build [--force] [--verbose]
 
@@ -30,7 +30,29 @@ def needs_build():
     return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in SOURCES + HEADERS)
 
 
+CALL = os.path.join(PKG, "_call.so")
+
+
+def build_call(force=False):
+    """Builds _call.so (csrc/fa_torch.cpp: flash_attn_forward on torch tensors) against the installed torch."""
+    src = os.path.join(CSRC, "fa_torch.cpp")
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(PKG, "..", "include", "fa_b200.h")))
+    if not force and os.path.exists(CALL) and os.path.getmtime(CALL) >= newest:
+        return CALL
+    import sysconfig
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc_path()))
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           "-isystem", os.path.join(tdir, "include"), "-isystem", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+                           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"), src, "-o", CALL,
+                           "-L", os.path.join(tdir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    return CALL
+
+
 def build(force=False, verbose=False):
+    build_call(force)
     if not force and not needs_build():
         return LIB
     objs = []
