@@ -276,11 +276,13 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
     DecodeArgs d;
     const bool dropout = p->p_dropout > 0.0f;
     int parts = splits;  // partial results per unit
-    if (!decode && !dropout) {
-        // how the keys are shared out is the library's business; the parts of a query block merge on chip
-        a.num_splits = parts = 1;
-        a.tiles_per_split = a.tc;
-        plan_tiled(&a, sms, cluster_room(sms));
+    if (!decode) {
+        if (!dropout) {
+            // how the keys are shared out is the library's business; the parts of a query block merge on chip
+            a.num_splits = parts = 1;
+            a.tiles_per_split = a.tc;
+        }
+        plan_tiled(&a, sms, cluster_room(sms), dropout);
     }
     if (decode) {
         fill_decode_args(p, a, &d);
@@ -425,7 +427,7 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd
         return FA_OK;
     }
     a.o_dim = p->head_dim;
-    plan_tiled(&a, num_sms, room);
+    plan_tiled(&a, num_sms, room, false);
     plan->parts = a.parts;
     plan->merged = a.parts > 1;
     plan->staged = a.staged;

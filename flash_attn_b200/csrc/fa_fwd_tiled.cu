@@ -1426,6 +1426,7 @@ double launch_us(const Cost& c, double ctas, int sms, double tiles) {
 struct Split {
     int parts;
     double us;
+    bool pair;  // two query tiles a CTA
     bool even;  // the query blocks are of about one length
 };
 // KV tiles that query block `qb` (two query tiles if `pair`) walks, as kv_tile_range has it.
@@ -1448,14 +1449,13 @@ int block_tiles(const FwdArgs& a, long long qb, bool pair) {
     return std::max(hi - lo, 0);
 }
 
-Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged) {
-    const bool pair = two_tiles(a);
+Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged, int most_parts, bool pair) {
     Cost c = kCost[pair][a.head_dim > 64];
     if (a.kv_group > 1 || a.pack_rows > 0) {
         c.crowd = std::min(c.crowd, pair ? 0.1 : 0.6);
         c.over = std::min(c.over, 0.2);
     }
-    if (a.alibi_slopes != nullptr && !a.is_causal && a.window_right != 0) c.rate *= 1.6;  // (a bias per element)
+    if (a.alibi_slopes != nullptr) c.rate *= !a.is_causal && a.window_right != 0 ? 1.6 : pair ? 1.0 : 1.15;  // (a bias per element; per pair of columns)
     const long long per_unit = pair ? (a.tr + 1) / 2 : a.tr;
     const long long blocks = a.units * per_unit, slots = pair ? sms : 2 * sms;
     // KV tiles of a unit's query blocks, on at most nine of them.  (The masks and not the length of K decide: a prompt written
@@ -1476,7 +1476,7 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
     const int tile_rows = pair ? 2 * kTile : kTile;
     const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
     const double stage = staged ? (c.merge + c.merge_each) * rows : 0.0;
-    Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, least >= 0.8 * n || n - least <= 1};
+    Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, pair, least >= 0.8 * n || n - least <= 1};
     if (blocks > slots) {
         const double waves = static_cast<double>(blocks) / slots;
         if (!best.even) {  // blocks of different lengths: the longest first, shorter ones fill up
@@ -1487,14 +1487,30 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
             if (rest > 0) best.us += launch_us(c, static_cast<double>(rest), sms, n) + stage;
         }
     }
-    for (int parts = 2; parts <= ClusterRoom::kMax && parts <= n; parts += parts < 8 ? 1 : 8) {
+    for (int parts = 2; parts <= most_parts && parts <= n; parts += parts < 8 ? 1 : 8) {
         if (blocks > room.fits(parts, pair ? 1 : 2)) continue;
         const double merge = c.merge * ((parts & (parts - 1)) ? 1.15 : 1.0) + c.merge_each * std::min(parts, 10);
         const double us = launch_us(c, static_cast<double>(blocks * parts), sms, (n + parts - 1) / parts) + merge * rows +
                           (parts == 16 ? 1.5 : 0.0);
-        if (us < best.us * (best.parts == 1 ? 0.96 : 1.0)) best = {parts, us, best.even};
+        if (us < best.us * (best.parts == 1 ? 0.96 : 1.0)) best = {parts, us, pair, best.even};
     }
     return best;
+}
+
+// Two query tiles a CTA, or one where the launch leaves SMs idle: a tile alone takes 2400 cycles for a KV tile (D = 64; 2700 at
+// D = 128), two that share an SM 3100, but a tile each to more CTAs than SMs costs the K/V reuse and, at D = 128, waits for a
+// ring of one stage.  us in two tiles / in one: [1,4,256,256,64] 5.94 / 4.81, [1,32,384,384,64] 7.99 / 6.98, [1,16,512,512,128]
+// 10.55 / 9.63, [1,32,512,512,128] 10.8 / 11.0 (128 CTAs of one tile), [1,64,512,512,128] 11.5 / 12.2 (256), but
+// [1,96,384,384,128] 17.2 / 10.6: 192 blocks of two tiles, of which 148 fit, against 288 tiles of which all fit.  The margins: under
+// a causal mask the model does not see that a pair's diagonal step has one tile only ([1,32,384,384,128] 8.7 / 9.0), nor what a
+// staged epilogue costs a single tile.  Over 300 random calls of up to 300 query tiles: 0.95 of two tiles always.
+Split best_cut(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged, int most_parts) {
+    const Split one = best_split(a, sms, room, staged, most_parts, false);
+    if (!two_tiles(a)) return one;
+    const Split two = best_split(a, sms, room, staged, most_parts, true);
+    const long long ctas = static_cast<long long>(a.units) * a.tr * one.parts;
+    const double margin = ctas > 2 * sms ? 0.0 : ctas > sms || a.is_causal || staged ? 0.8 : 0.93;
+    return one.us < margin * two.us ? one : two;
 }
 
 }  // namespace
@@ -1548,12 +1564,16 @@ ClusterRoom cluster_room(int sms) {
     return room;
 }
 
-void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
+void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room, bool dropout) {
     a->parts = 1;
     a->pack_rows = 0;
-    a->staged = a->o_dim != a->head_dim;
-    if (a->accum_o != nullptr) return;  // (a running pair is merged by the unstaged epilogue, each query tile as it finishes)
-    Split split = best_split(*a, sms, room, a->staged != 0);
+    // With dropout the caller's splits are part of the result; a running pair is merged by the unstaged epilogue, each query tile
+    // as it finishes.
+    const bool unsplit = dropout || a->accum_o != nullptr;
+    a->staged = !dropout && a->o_dim != a->head_dim;
+    Split split = best_cut(*a, sms, room, a->staged != 0, unsplit ? 1 : ClusterRoom::kMax);
+    a->pair = a->num_splits > 1 ? two_tiles(*a) : split.pair;
+    if (unsplit) return;
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
     // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the query
     // blocks are of about one length (tiles across heads have the longest: [4 x 12 heads on 2, 1940 rows, 1241 keys, causal]
@@ -1572,20 +1592,21 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room) {
         b.tr = static_cast<int>((rows + kTile - 1) / kTile);
         b.units = a->units / heads;
         b.kv_group = 1;
-        const Split packed = split.even && b.tr < heads * a->tr ? best_split(b, sms, room, true) : Split{1, 1e30, true};
+        const Split packed = split.even && b.tr < heads * a->tr ? best_cut(b, sms, room, true, ClusterRoom::kMax) : Split{1, 1e30, true, true};
         if (packed.us < 0.97 * split.us - 2.0) {
             *a = b;
             split = packed;
         }
     }
     a->parts = split.parts;
+    a->pair = split.pair;
     a->staged = a->staged || a->parts > 1 || a->pack_rows > 0;
 }
 
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream) {
     const bool alibi = a.alibi_slopes != nullptr;
-    const bool pair = two_tiles(a);
+    const bool pair = a.pair != 0;
     if (a.head_dim <= 64) {
         return pair ? launch_dtype<64, 2>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream)
                     : launch_dtype<64, 1>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);

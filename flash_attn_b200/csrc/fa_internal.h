@@ -45,6 +45,7 @@ struct FwdArgs {
     int kv_group;           // query units per K/V unit (grouped-query attention); K/V unit = unit / kv_group
     int seqlen_q, seqlen_k, head_dim;
     int tr, tc;             // query / key tiles
+    int pair;               // query tiles of a CTA: two, or one
     int num_splits, tiles_per_split;
     float scale_log2;       // softmax_scale * log2(e)
     int is_causal, window_left, window_right;
@@ -75,9 +76,9 @@ struct ClusterRoom {
 };
 ClusterRoom cluster_room(int sms);  // of the current device; none above one CTA where the runtime does not say
 
-// Decides how a launch without dropout is cut (fills staged, parts and, for short grouped queries, restates the
-// problem with the heads of a K/V head stacked: units, heads, kv_group, seqlen_q, tr, pack_rows).
-void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room);
+// Decides how a launch is cut: pair and, without dropout, staged, parts and, for short grouped queries, a problem
+// restated with the heads of a K/V head stacked (units, heads, kv_group, seqlen_q, tr, pack_rows).
+void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room, bool dropout);
 
 // Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O, or of the running
 // result where the launch leaves that (32-row boxes); it is read only when a.o_tma or a.accum_o is set.  `tc` is the load
