@@ -325,7 +325,7 @@ __device__ __forceinline__ void issue_qk_bias(uint32_t d_tmem, uint32_t qa_lo, u
 }
 
 // The end of a staged launch: the CTAs of a cluster hold, for the same NQ * 128 query rows, the un-normalised
-// rows, maxima and sums over their own keys (one CTA, parts = 1: all keys).  Each CTA finishes an equal share of the
+// rows, maxima and sums over their own keys.  Each CTA finishes an equal share of the
 // rows from all of them, O = sum_j 2^(m_j - m) O_j / l, l = sum_j 2^(m_j - m) l_j
 // (src/flash_forward_splitkv.h:359-397), and writes them a row or two per warp instruction.
 template <int D, int NQ, bool kBf16>
@@ -383,7 +383,8 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
             for (int u = 0; u < kUnroll; ++u) {
                 const int row = r_lo + k0 + u * kStep;
                 const uint32_t addr = base + row * (D * 4) + (chunk ^ (row & 7)) * 16;
-                v[u] = own ? ld_shared_f32x4_if(addr, k0 + u * kStep < n_rows) : ld_cluster_f32x4_if(addr, k0 + u * kStep < n_rows);
+                const bool take = k0 + u * kStep < n_rows && col < a.o_dim;  // (of a padded head no more than its own columns)
+                v[u] = own ? ld_shared_f32x4_if(addr, take) : ld_cluster_f32x4_if(addr, take);
             }
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
@@ -1083,9 +1084,10 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
         FA_TR(96);
         if constexpr (kStaged) {
-            // un-normalised rows, maxima and sums go to shared memory (the ring is free once the MMAs of both
-            // query tiles have completed, the Q tiles too); merge_rows below finishes them
-            asm volatile("bar.sync 5, %0;" ::"n"(NQ * 128) : "memory");
+            // A split leaves un-normalised rows, maxima and sums in shared memory (the ring is free once the MMAs of both
+            // query tiles have completed, the Q tiles too); merge_rows below finishes them.  Unsplit, each warp finishes its own.
+            if (a.parts > 1) asm volatile("bar.sync 5, %0;" ::"n"(NQ * 128) : "memory");
+            else if (!have_o && rb < a.tr) (void)mbar_wait_warp(bar_q_full, 0, abort_flag);  // (Q has landed where the rows are staged)
             // A wait of this CTA gave up (the flag was set by whoever waited, before the barrier above): none of its rows
             // may pass for the part of a softmax, so every row sum is NaN, which the merge carries to O (and to
             // LSE = -inf); and the copies still in flight land first, since they write where the rows are staged.
@@ -1094,6 +1096,66 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 const long long t0 = clock64();
                 while (clock64() - t0 < 200000) { }
             }
+            if (a.parts == 1) {
+                // Rows of any pitch, sixteen at a time through this warp's part of the query tile's Q buffer: they are consecutive in
+                // memory, so neighbouring lanes write neighbouring elements (or 16-byte chunks, where the pitch allows).
+                // Bound by latency; no barrier, so each warp leaves as it is done.  Kernels of a call with fp32 output, against
+                // merge_rows for one part: [2,8,500,500,31] causal 14.4 -> 12.8 us, [4,8,1000,1000,20] 26.4 -> 24.0.
+                const uint32_t rows16 = sQ + qi * C::kTileBytes + (warp & 3) * (32 * D * 2);
+                const float inv = gave_up ? __int_as_float(0x7fc00000) : l_sum == 0.0f ? 0.0f : 1.0f / l_sum;
+                auto scaled = [&](uint32_t x) { return inv == 0.0f ? 0u : __float_as_uint(__uint_as_float(x) * inv); };  // (a row without keys is 0, whatever masked values left)
+                if (a.lse != nullptr && row < a.seqlen_q)
+                    a.lse[static_cast<long long>(unit) * a.seqlen_q + row] = !gave_up && l_sum > 0.0f ? m_ref * kLn2 + __logf(l_sum) : -INFINITY;
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    const int first = rb * kTile + (warp & 3) * 32 + h * 16;
+                    const int n_rows = min(16, a.seqlen_q - first);
+                    if (n_rows <= 0) break;
+#pragma unroll 1
+                    for (int c = 0; c < D / 32; ++c) {
+                        uint32_t orow[32];
+                        if (have_o) {
+                            tmem_ld32(tmem_o + lane_base + c * 32, orow);
+                            tmem_wait_ld();
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) orow[i] = 0u;
+                        }
+                        if ((lane >> 4) == h) {
+#pragma unroll
+                            for (int i = 0; i < 32; i += 4) {
+                                const uint32_t chunk = static_cast<uint32_t>((c * 32 + i) >> 2) ^ static_cast<uint32_t>(lane & 7);
+                                st_shared_v4(rows16 + (lane & 15) * (D * 4) + chunk * 16, scaled(orow[i]), scaled(orow[i + 1]), scaled(orow[i + 2]), scaled(orow[i + 3]));
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    const long long at0 = (static_cast<long long>(unit) * a.seqlen_q + first) * a.o_dim;
+                    if (a.o_dim % 8 == 0) {
+                        constexpr int kLanes = D / 4, kPerWarp = 32 / kLanes;
+                        const int chunk = lane % kLanes;
+#pragma unroll 4
+                        for (int k = lane / kLanes; k < 16; k += kPerWarp) {
+                            if (k >= n_rows || chunk * 4 >= a.o_dim) continue;
+                            const float4 o = ld_shared_f32x4(rows16 + k * (D * 4) + static_cast<uint32_t>(chunk ^ (k & 7)) * 16);
+                            const long long at = at0 + k * a.o_dim + chunk * 4;
+                            if (a.o_is_fp32) *reinterpret_cast<float4*>(static_cast<float*>(a.o) + at) = o;
+                            else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.o) + at) = make_uint2(pack2<kBf16>(o.x, o.y), pack2<kBf16>(o.z, o.w));
+                        }
+                    } else {
+                        const uint32_t n = static_cast<uint32_t>(n_rows * a.o_dim);
+                        const uint8_t* src = smem_gen + (rows16 - smem_base);
+#pragma unroll 4
+                        for (uint32_t e = lane; e < n; e += 32) {
+                            const uint32_t k = fast_div(a.div_o_dim, e), col = e - k * a.o_dim;
+                            const float x = *reinterpret_cast<const float*>(src + k * (D * 4) + ((col >> 2) ^ (k & 7)) * 16 + (col & 3) * 4);
+                            if (a.o_is_fp32) static_cast<float*>(a.o)[at0 + e] = x;
+                            else static_cast<uint16_t*>(a.o)[at0 + e] = static_cast<uint16_t>(pack2<kBf16>(x, 0.0f));
+                        }
+                    }
+                    __syncwarp();
+                }
+            } else {
             const uint32_t stage = sK + (qi * kTile + r) * (D * 4);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -1113,6 +1175,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             *reinterpret_cast<float2*>(smem_gen + C::kSmemQ + (qi * kTile + r) * 8) =
                 make_float2(have_o ? m_ref : -INFINITY, gave_up ? __int_as_float(0x7fc00000) : have_o ? l_sum : 0.0f);
+            }
         } else {
         float inv = 0.0f;
         if (l_sum > 0.0f) inv = (kDropout ? a.drop.inv_keep : 1.0f) / l_sum;
@@ -1290,12 +1353,13 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
 
     if constexpr (kStaged) {
-        __syncwarp();
-        if (a.parts > 1) cluster_sync();
-        else __syncthreads();
-        if (warp < NQ * 4) merge_rows<D, NQ, kBf16>(a, smem_gen, smem_base, part, unit, qb);
-        __syncwarp();
-        if (a.parts > 1) cluster_sync();  // the peers' shared memory stays until everyone has read it
+        if (a.parts > 1) {
+            __syncwarp();
+            cluster_sync();
+            if (warp < NQ * 4) merge_rows<D, NQ, kBf16>(a, smem_gen, smem_base, part, unit, qb);
+            __syncwarp();
+            cluster_sync();  // the peers' shared memory stays until everyone has read it
+        }
     }
 
     // ---- teardown ------------------------------------------------------------------
@@ -1357,6 +1421,7 @@ cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, 
     if (kStaged) {
         a.div_parts = make_fastdiv(static_cast<uint32_t>(a.parts));
         a.div_pack = make_fastdiv(static_cast<uint32_t>(a.pack_rows));
+        a.div_o_dim = make_fastdiv(static_cast<uint32_t>(a.o_dim));
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = static_cast<unsigned>(a.parts);
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
@@ -1407,7 +1472,7 @@ bool two_tiles(const FwdArgs& a) { return a.tr > 2 || (a.tr == 2 && (!a.is_causa
 // fit the device at once ([160 blocks, 67 tiles] 231 us unsplit, 203 in three parts and four waves).
 //   A CTA takes `base` to start and drain and `rate` for a KV tile.  The rate grows with the CTAs at work: by `crowd` up to one an
 //   SM (L2 and HBM; less where grouped queries share their K/V), by `over` for a second one on the SM (single query tiles only).
-//   A split (or a staged launch of one part) pays `merge` + `merge_each` a part for staging, two cluster barriers and the merge (its distributed-shared-memory
+//   A split pays `merge` + `merge_each` a part for staging, two cluster barriers and the merge (its distributed-shared-memory
 //   reads run at about 11 bytes a clock and SM), part counts that are no power of two a little more, few rows less.
 //   It is taken only where all its clusters are resident at once (ClusterRoom): a second wave waits for whole clusters to
 //   leave.  [16 blocks, 19 tiles] 34.0 unsplit, 20.6 / 20.5 / 22.2 / 40.3 in 4 / 5 / 6 / 7 parts (15 clusters of 7 fit),
@@ -1475,7 +1540,7 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
     }
     const int tile_rows = pair ? 2 * kTile : kTile;
     const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
-    const double stage = staged ? (c.merge + c.merge_each) * rows : 0.0;
+    const double stage = staged ? 0.4 : 0.0;
     Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, pair, least >= 0.8 * n || n - least <= 1};
     if (blocks > slots) {
         const double waves = static_cast<double>(blocks) / slots;
@@ -1502,14 +1567,13 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
 // ring of one stage.  us in two tiles / in one: [1,4,256,256,64] 5.94 / 4.81, [1,32,384,384,64] 7.99 / 6.98, [1,16,512,512,128]
 // 10.55 / 9.63, [1,32,512,512,128] 10.8 / 11.0 (128 CTAs of one tile), [1,64,512,512,128] 11.5 / 12.2 (256), but
 // [1,96,384,384,128] 17.2 / 10.6: 192 blocks of two tiles, of which 148 fit, against 288 tiles of which all fit.  The margins: under
-// a causal mask the model does not see that a pair's diagonal step has one tile only ([1,32,384,384,128] 8.7 / 9.0), nor what a
-// staged epilogue costs a single tile.  Over 300 random calls of up to 300 query tiles: 0.95 of two tiles always.
+// a causal mask the model does not see that a pair's diagonal step has one tile only ([1,32,384,384,128] 8.7 / 9.0).  Over 300 random calls of up to 300 query tiles: 0.95 of two tiles always.
 Split best_cut(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged, int most_parts) {
     const Split one = best_split(a, sms, room, staged, most_parts, false);
     if (!two_tiles(a)) return one;
     const Split two = best_split(a, sms, room, staged, most_parts, true);
     const long long ctas = static_cast<long long>(a.units) * a.tr * one.parts;
-    const double margin = ctas > 2 * sms ? 0.0 : ctas > sms || a.is_causal || staged ? 0.8 : 0.93;
+    const double margin = ctas > 2 * sms ? 0.0 : ctas > sms || a.is_causal ? 0.8 : 0.93;
     return one.us < margin * two.us ? one : two;
 }
 

@@ -63,7 +63,7 @@ struct FwdArgs {
     int o_dim;              // columns (and row pitch) of O: head_dim, or less when Q, K, V are padded copies
     // launch order of the CTAs (filled by launch_fwd_tiled): divisors of the block index
     FastDiv div_group_ctas, div_gsize, div_last_gsize, div_splits, div_kv_group;
-    FastDiv div_parts, div_pack;
+    FastDiv div_parts, div_pack, div_o_dim;
     DropoutParams drop;
 };
 
