@@ -27,6 +27,8 @@ def _check(q, k, v, o):
     dt = q.dtype
     if (dt is not torch.float16 and dt is not torch.bfloat16) or k.dtype is not dt or v.dtype is not dt:
         raise ValueError("q, k, v must share dtype float16 or bfloat16")
+    if o.numel() < q.numel():
+        raise ValueError("out must hold [batch, heads, seqlen, head_dim]")
 
 
 def _params(q, k, v, o, lse, softmax_scale, causal, window, alibi_slopes, p_dropout, seed, offset, unit0, num_splits,
@@ -96,6 +98,8 @@ def flash_attn_forward_host(q, k, v, softmax_scale=None, causal=False, window=(-
     lse = torch.empty((B, H, Nq), dtype=torch.float32, pin_memory=True) if return_lse else None
     if alibi_slopes is not None:
         alibi_slopes = alibi_slopes.to(device="cpu", dtype=torch.float32).contiguous()
+        if alibi_slopes.numel() < H:
+            raise ValueError("alibi_slopes must hold a slope for each head")
     p = _params(q, k, v, out, lse, softmax_scale, causal, window, alibi_slopes, p_dropout, seed, offset, 0,
                 num_splits, 0, 0)
     with torch.cuda.device(device if device is not None else torch.cuda.current_device()):

@@ -6,6 +6,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -70,6 +71,21 @@ int dtype_of(const at::Tensor& t) {
 }
 bool same(at::IntArrayRef a, at::IntArrayRef b) { return a == b; }
 
+// Kernels follow a pointer as it is, so memory that `device` does not reach is refused here.  A tensor on the device itself costs a
+// comparison; pinned and managed host memory and an enabled peer's memory are reached too, which the runtime is asked about.
+bool reaches(const c10::Device& device, const void* memory) {
+    const c10::cuda::OptionalCUDAGuard guard(device);
+    cudaPointerAttributes at;
+    const bool known = cudaPointerGetAttributes(&at, memory) == cudaSuccess;
+    if (!known) (void)cudaGetLastError();
+    return known && at.devicePointer != nullptr;
+}
+void need_reach(const c10::Device& device, const at::Tensor& t, const char* name) {
+    if (t.device() == device || t.numel() == 0 || reaches(device, t.data_ptr())) return;
+    PyErr_Format(PyExc_ValueError, "%s must be on q's device, or in memory that this device reaches", name);
+    throw python_error_set();
+}
+
 enum Arg {
     kFwd, kWorkspaceFn, kQ, kK, kV, kScale, kCausal, kWindow, kSlopes, kDropout, kSeed, kOffset, kSplits, kOut, kOutDtype,
     kReturnLse, kQPos0, kKPos0, kUnit0, kWorkspace, kStatus, kAccum, kAccumFirst, kAccumFinal, kLaunchIndex, kArgs
@@ -103,7 +119,10 @@ PyObject* forward_impl(PyObject* const* args) {
         if (truth_of(args[kReturnLse])) lse = at::empty({B, H, Nq}, q.options().dtype(at::kFloat).layout(at::kStrided).requires_grad(false));
     }
     at::Tensor slopes;
-    if (args[kSlopes] != Py_None) slopes = tensor_of(args[kSlopes], "alibi_slopes").to(device, at::kFloat).contiguous();
+    if (args[kSlopes] != Py_None) {
+        slopes = tensor_of(args[kSlopes], "alibi_slopes").to(device, at::kFloat).contiguous();
+        if (slopes.numel() < H) value_error("alibi_slopes must hold a slope for each head");
+    }
     const at::Tensor& o = out.defined() ? out : q;
     if (k.dim() < 3) value_error("k and v must be [batch, heads_k, seqlen_k, head_dim] with heads a multiple of heads_k");
     const int64_t Hk = k.size(1), Nk = k.size(2);
@@ -115,6 +134,11 @@ PyObject* forward_impl(PyObject* const* args) {
     const at::ScalarType type = q.scalar_type();
     if ((type != at::kHalf && type != at::kBFloat16) || k.scalar_type() != type || v.scalar_type() != type)
         value_error("q, k, v must share dtype float16 or bfloat16");
+    // (an output of another shape is filled as [batch, heads, seqlen, head_dim] rows one behind the other: it has to hold them)
+    if (o.numel() < q.numel()) value_error("out must hold [batch, heads, seqlen, head_dim]");
+    need_reach(device, k, "k");
+    need_reach(device, v, "v");
+    need_reach(device, o, "out");
 
     fa_fwd_params p;
     std::memset(&p, 0, sizeof p);
@@ -137,6 +161,8 @@ PyObject* forward_impl(PyObject* const* args) {
         if (!tensors || o_acc.scalar_type() != at::kFloat || lse_acc.scalar_type() != at::kFloat || !o_acc.is_contiguous() ||
             !lse_acc.is_contiguous() || !same(o_acc.sizes(), rows) || !same(lse_acc.sizes(), at::IntArrayRef(rows, 3)))
             value_error("accum = (fp32 [B,H,Nq,d], fp32 [B,H,Nq]), contiguous");
+        need_reach(device, o_acc, "accum");
+        need_reach(device, lse_acc, "accum");
         p.accum_o = static_cast<float*>(o_acc.data_ptr());
         p.accum_lse = static_cast<float*>(lse_acc.data_ptr());
         p.accum_flags = (truth_of(args[kAccumFirst]) ? FA_ACCUM_FIRST : 0) | (accum_final ? FA_ACCUM_FINAL : 0);
@@ -187,7 +213,13 @@ PyObject* forward_impl(PyObject* const* args) {
     p.num_splits = int_of(args[kSplits]);
     p.q_pos0 = static_cast<int64_t>(bits_of(args[kQPos0]));
     p.k_pos0 = static_cast<int64_t>(bits_of(args[kKPos0]));
-    if (args[kStatus] != Py_None) p.status = static_cast<int*>(tensor_of(args[kStatus], "status").data_ptr());
+    if (args[kStatus] != Py_None) {
+        const at::Tensor& status = tensor_of(args[kStatus], "status");
+        if (status.nbytes() < sizeof(int) || reinterpret_cast<uintptr_t>(status.data_ptr()) % sizeof(int) != 0)
+            value_error("status must hold an aligned 32-bit word");
+        need_reach(device, status, "status");
+        p.status = static_cast<int*>(status.data_ptr());
+    }
 
     const c10::cuda::OptionalCUDAGuard guard(device);  // (nothing where the device is the current one)
     at::Tensor workspace;
@@ -195,8 +227,11 @@ PyObject* forward_impl(PyObject* const* args) {
         const size_t need = workspace_bytes(&p);
         if (need != 0) {
             if (args[kWorkspace] != Py_None) workspace = tensor_of(args[kWorkspace], "workspace");
-            if (!workspace.defined() || workspace.nbytes() < need)
+            // (of a tensor that is not contiguous the byte count says nothing about the memory behind its first element)
+            if (!workspace.defined() || workspace.nbytes() < need || !workspace.is_contiguous())
                 workspace = at::empty({static_cast<int64_t>(need)}, at::TensorOptions().device(device).dtype(at::kByte));
+            else
+                need_reach(device, workspace, "workspace");
             p.workspace = workspace.data_ptr();
             p.workspace_bytes = workspace.nbytes();
         }

@@ -85,3 +85,52 @@ def test_what_was_refused_stays_refused(change, error):
     q, k, v = _qkv()
     with pytest.raises(error):
         fa.flash_attn_forward(**{**dict(q=q, k=k, v=v), **change(q, k, v)})
+
+
+# what lies outside a tensor, or in memory that the device does not reach, must not come to a kernel: nothing is launched here
+@pytest.mark.parametrize("change", [
+    lambda q, k, v: dict(out=torch.empty(q.numel() - 1, device="cuda", dtype=q.dtype)),
+    lambda q, k, v: dict(out=torch.empty(q[:, :2].shape, device="cuda", dtype=q.dtype)),
+    lambda q, k, v: dict(out=torch.empty(q.shape, dtype=q.dtype)),
+    lambda q, k, v: dict(k=k.cpu()),
+    lambda q, k, v: dict(v=v.cpu()),
+    lambda q, k, v: dict(alibi_slopes=torch.ones(3)),
+    lambda q, k, v: dict(status=torch.zeros(0, device="cuda", dtype=torch.int32)),
+    lambda q, k, v: dict(status=torch.zeros(1, device="cuda", dtype=torch.int16)),
+    lambda q, k, v: dict(status=torch.zeros(8, device="cuda", dtype=torch.int8)[1:]),
+    lambda q, k, v: dict(status=torch.zeros(1, dtype=torch.int32)),
+    lambda q, k, v: dict(num_splits=2, workspace=torch.empty(1 << 24, dtype=torch.uint8)),
+    lambda q, k, v: dict(accum=(torch.empty(q.shape), torch.empty(q.shape[:3], device="cuda")), accum_first=True),
+    lambda q, k, v: dict(accum=(torch.empty(q.shape, device="cuda"), torch.empty(q.shape[:3])), accum_first=True),
+])
+def test_memory_that_a_kernel_may_not_touch_is_refused(change):
+    import flash_attn_b200 as fa
+    q, k, v = _qkv()
+    with pytest.raises(ValueError):
+        fa.flash_attn_forward(**{**dict(q=q, k=k, v=v), **change(q, k, v)})
+
+
+def test_memory_of_another_shape_or_place_that_serves_is_taken():
+    import flash_attn_b200 as fa
+    q, k, v = _qkv()
+    want = fa.flash_attn_forward(q, k, v)[0]
+    flat = torch.full((q.numel() + 8,), 7.0, device="cuda", dtype=q.dtype)
+    assert fa.flash_attn_forward(q, k, v, out=flat)[0] is flat
+    assert torch.equal(flat[:-8].view_as(q), want) and bool((flat[-8:] == 7.0).all())
+    status = torch.zeros(1, dtype=torch.int32).pin_memory()
+    assert torch.equal(fa.flash_attn_forward(q, k, v, status=status)[0], want)
+    slopes = torch.full((4,), 0.25)
+    assert torch.equal(*(fa.flash_attn_forward(q, k, v, alibi_slopes=x)[0] for x in (slopes, torch.cat([slopes, slopes]))))
+    split = fa.flash_attn_forward(q, k, v, num_splits=2)[0]
+    for room in (torch.empty(1, device="cuda").expand(1 << 22), torch.empty(4)):  # (no room: the call takes its own)
+        assert torch.equal(fa.flash_attn_forward(q, k, v, num_splits=2, workspace=room)[0], split)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+
+
+def test_host_buffers_too_small_for_the_call_are_refused():
+    import flash_attn_b200 as fa
+    q, k, v = (x.cpu() for x in _qkv())
+    for bad in (dict(out=torch.empty(q.numel() - 1, dtype=q.dtype)), dict(alibi_slopes=torch.ones(3))):
+        with pytest.raises(ValueError):
+            fa.flash_attn_forward_host(q, k, v, **bad)
