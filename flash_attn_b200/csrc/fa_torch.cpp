@@ -191,8 +191,14 @@ PyObject* forward_impl(PyObject* const* args) {
     }
     p.is_causal = truth_of(args[kCausal]) ? 1 : 0;
     for (int i = 0; i < 2; ++i) {
-        PyObject* x = PyTuple_CheckExact(args[kWindow]) && PyTuple_GET_SIZE(args[kWindow]) > i
-                          ? Py_NewRef(PyTuple_GET_ITEM(args[kWindow], i)) : PySequence_GetItem(args[kWindow], i);
+        PyObject* x;
+        if (PyTuple_CheckExact(args[kWindow]) && PyTuple_GET_SIZE(args[kWindow]) > i) {
+            x = Py_NewRef(PyTuple_GET_ITEM(args[kWindow], i));
+        } else {  // window[i] of whatever has items (a tensor is no sequence)
+            PyObject* at = PyLong_FromLong(i);
+            x = at ? PyObject_GetItem(args[kWindow], at) : nullptr;
+            Py_XDECREF(at);
+        }
         if (!x) throw python_error_set();
         int w;
         try {

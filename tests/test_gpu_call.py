@@ -34,6 +34,8 @@ def _by_ctypes(q, k, v, o, lse, **kw):
     (64, dict(), dict()),
     (64, dict(softmax_scale=np.float64(0.25), causal=1, window=[np.int64(50), 0], q_pos0=np.int32(200)),
      dict(softmax_scale=0.25, is_causal=1, window_left=50, window_right=0, q_pos0=200)),
+    (64, dict(causal=True, window=torch.tensor([50, -1])), dict(is_causal=1, window_left=50)),
+    (64, dict(window={0: 20, 1: 30}), dict(window_left=20, window_right=30)),
     (128, dict(p_dropout=0.25, seed=-3, offset=2 ** 64 + 8, launch_index=1), dict(p_dropout=0.25, seed=2 ** 64 - 3, offset=8, launch_index=1)),
     (128, dict(p_dropout=0.5, seed=7, num_splits=2, unit0=5), dict(p_dropout=0.5, seed=7, num_splits=2, unit0=5)),
     (50, dict(out_dtype=torch.float32, num_splits=0), dict(num_splits=0)),
