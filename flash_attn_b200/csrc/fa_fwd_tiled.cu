@@ -58,15 +58,16 @@ extern "C" int fa_trace_read(long long* host_out) {
 #define FA_TR(ev) do { } while (0)
 #endif
 
-// Test build only (-DFA_TEST_SHORT_WAIT): the producer can be told to leave out the loads of one KV
-// tile, so that a consumer's bounded wait runs out and the give-up path (status word, drain, TMEM
-// release, clean exit) can be checked on a GPU without faulting or hanging anything.
+// Test build only (-DFA_TEST_SHORT_WAIT): the producer can be told to leave out the loads of a KV tile and of all
+// behind it, so that a consumer's bounded wait runs out and the give-up path (status word, drain, TMEM
+// release, clean exit) can be checked on a GPU without faulting or hanging anything.  (Not of one tile alone: in a ring of one
+// stage the wait that belongs to the tile after it would pass at once, and the stage's barrier would be armed twice in a phase.)
 #ifdef FA_TEST_SHORT_WAIT
 __device__ int fa_test_skip_tile = -1;
 extern "C" int fa_test_skip_kv_tile(int t) {
     return static_cast<int>(cudaMemcpyToSymbol(fa_test_skip_tile, &t, sizeof(int)));
 }
-#define FA_TEST_SKIPS(t) (fa_test_skip_tile == (t))
+#define FA_TEST_SKIPS(t) (fa_test_skip_tile >= 0 && (t) >= fa_test_skip_tile)
 #else
 #define FA_TEST_SKIPS(t) false
 #endif
@@ -1193,9 +1194,13 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             const long long arow = unit_ll * a.seqlen_q + row;
             float lse_c = -INFINITY;
             if (!a.accum_first && row_ok) lse_c = a.accum_lse[arow];
+            // The buffers of the carried rows, before anything of this launch's is written: if a wait gave up, here or before, neither
+            // the rows nor their sums may pass for a running result, so both become NaN, which later launches carry on.
+            if ((carry || n_union > 0) && rb < a.tr && !mbar_wait_warp(carry ? bar_carry + 8 * qi : bar_qk_done, 0, abort_flag) && fail == 0) fail = 11;
+            if (fail != 0) lse_c = __int_as_float(0x7fc00000);
             const float m = fmaxf(lse_c, lse_val);
             float lse_new = -INFINITY, w_new = 0.0f;
-            if (m != -INFINITY) {
+            if (m != -INFINITY || lse_c != lse_c) {
                 const float e_old = __expf(lse_c - m), e_new = __expf(lse_val - m);
                 const float sum = e_old + e_new;
                 w_old = e_old / sum;
@@ -1255,10 +1260,15 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             // middle 912 -> 863, the last 893 -> 855; [2,4,333,96] x 777 keys 21.7 -> 13.4.  Whole lines by coalesced loads
             // from a staged copy, without the early TMA loads, measured 914.
             const bool out16 = a.accum_final && a.o != nullptr && !a.o_is_fp32;
-            if ((carry || n_union > 0) && rb < a.tr && !mbar_wait_warp(carry ? bar_carry + 8 * qi : bar_qk_done, 0, abort_flag) && fail == 0) fail = 11;
+            if (fail != 0 && row_ok) {  // (straight to memory: copies may still be on their way to the buffers)
+                const bool last = a.accum_final && a.o != nullptr;
+                uint8_t* dst = static_cast<uint8_t*>(last ? a.o : static_cast<void*>(a.accum_o)) + (unit_ll * a.seqlen_q + row) * a.head_dim * (out16 ? 2 : 4);
+                for (int i = 0; i < a.head_dim * (out16 ? 2 : 4); i += 16)
+                    *reinterpret_cast<uint4*>(dst + i) = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);  // (NaN in all three types)
+            }
             const int y0 = rb * kTile + (warp & 3) * 32;
 #pragma unroll 1
-            for (int b = 0; b < (rb < a.tr ? D / 32 : 0); ++b) {  // (beyond the last query tile the buffers are not this group's)
+            for (int b = 0; b < (rb < a.tr && fail == 0 ? D / 32 : 0); ++b) {  // (beyond the last query tile the buffers are not this group's)
                 uint32_t orow[32];
                 if (have_o) {
                     tmem_ld32(tmem_o + lane_base + b * 32, orow);

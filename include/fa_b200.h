@@ -89,7 +89,8 @@ typedef struct fa_fwd_params {
                                  clocks); a wait that gives up stores a code here -- 100 + n from the tiled
                                  forward kernel, 200 + n from the decode kernel, n naming the wait -- and the
                                  CTA drains and exits, leaving O and LSE undefined (O is NaN in rows that
-                                 CTAs merge on chip: a part never passes for the whole).  fa_fwd is
+                                 CTAs merge on chip: a part never passes for the whole; of a running result
+                                 both are NaN, and later launches keep them so).  fa_fwd is
                                  asynchronous: the caller clears the word before the launch and reads it after synchronising
                                  the stream.  fa_fwd_host does both itself and returns FA_ERR_DEVICE_TIMEOUT. */
     void* stream;             /* cudaStream_t; NULL = default stream (the reference's)       */

@@ -1,6 +1,6 @@
 """The give-up path of the kernels' bounded waits, exercised on a GPU without faulting, trapping or
 hanging anything: a test build of the library (-DFA_TEST_SHORT_WAIT: waits give up after about 2 ms)
-whose TMA producer is told to leave out the loads of one KV tile.  The MMA warp's wait for that tile
+whose TMA producer is told to leave out the loads of a KV tile and of those behind it.  The MMA warp's wait for that tile
 runs out, the kernel records 100 + n in the status word, drains, frees its tensor memory and returns;
 the host-buffer entry point turns the word into FA_ERR_DEVICE_TIMEOUT; the next ordinary launch on
 the same device and context is correct."""
@@ -132,3 +132,62 @@ def test_a_part_that_gave_up_leaves_no_plausible_row(test_lib, skip, H, Hk, Nq, 
     want_o, want_lse = oracle_lib.forward(qh, np.repeat(kh, H // Hk, 1), np.repeat(vh, H // Hk, 1), d ** -0.5)
     assert np.abs(o.float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
     assert np.abs(lse.cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
+
+
+@pytest.mark.parametrize("H,Nq,d,skip,causal,out_dtype", [
+    (160, 256, 128, 1, False, torch.bfloat16),  # (two query tiles a CTA)
+    (120, 300, 64, 0, True, torch.float32),     # (a CTA whose second query tile does not exist; the first tile of the walk)
+    (3, 300, 128, 1, False, torch.float32),     # (one query tile a CTA, a ring of one stage)
+])
+def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip, causal, out_dtype):
+    """The block before it is complete, and so are the ones behind it: neither may make its rows look like a result."""
+    from flash_attn_b200 import _lib
+    L = test_lib
+    Nk = 500
+    qh, kh, vh = synth.qkv(42, 1, 3, Nq, 4 * Nk, d, "bfloat16")  # (the oracle's heads, again and again)
+    q, k, v = (gpu_util.to_dev(x, "bfloat16")[:, torch.arange(H) % 3].contiguous() for x in (qh, kh, vh))
+    acc = (torch.empty((1, H, Nq, d), device="cuda"), torch.empty((1, H, Nq), device="cuda"))
+    o = torch.zeros((1, H, Nq, d), device="cuda", dtype=out_dtype)
+    lse = torch.zeros((1, H, Nq), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def block(i, first, final):
+        kb, vb = (x[:, :, i * Nk:(i + 1) * Nk].contiguous() for x in (k, v))
+        p = _params(q, kb, vb, o, lse, status)
+        p.o_dtype = _lib.FA_DTYPE_FP32 if out_dtype is torch.float32 else _lib.FA_DTYPE_BF16
+        p.is_causal, p.q_pos0, p.k_pos0 = int(causal), 3 * Nk, i * Nk  # (with a causal mask no query sees the fourth block's end)
+        p.accum_o, p.accum_lse = acc[0].data_ptr(), acc[1].data_ptr()
+        p.accum_flags = (_lib.FA_ACCUM_FIRST if first else 0) | (_lib.FA_ACCUM_FINAL if final else 0)
+        assert L.fa_fwd(ctypes.byref(p)) == 0
+        torch.cuda.synchronize()
+
+    def gives_up(i, first, final):
+        status.zero_()
+        try:
+            assert L.fa_test_skip_kv_tile(skip) == 0
+            block(i, first, final)
+        finally:
+            assert L.fa_test_skip_kv_tile(-1) == 0
+        assert 100 < int(status.item()) < 200
+
+    for first in (False, True):  # a block in the middle, the first one, and what the launches behind it make of the pair
+        if not first:
+            block(0, True, False)
+            assert torch.isfinite(acc[0]).all() and torch.isfinite(acc[1]).all()
+        gives_up(1, first, False)
+        assert torch.isnan(acc[0]).all() and torch.isnan(acc[1]).all()
+        status.zero_()
+        block(2, False, False)
+        assert torch.isnan(acc[0]).all() and torch.isnan(acc[1]).all()
+        block(3, False, True)
+        assert torch.isnan(o).all() and torch.isnan(lse).all() and int(status.item()) == 0
+    block(0, True, False)
+    gives_up(1, False, True)  # the last block
+    assert torch.isnan(o).all() and torch.isnan(lse).all() and torch.isnan(acc[1]).all()
+    status.zero_()
+    for i in range(4):
+        block(i, i == 0, i == 3)
+    want_o, want_lse = oracle_lib.forward(qh, kh, vh, d ** -0.5, causal=causal, q_pos0=3 * Nk)
+    assert int(status.item()) == 0
+    assert np.abs(o[:, :3].float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
+    assert np.abs(lse[:, :3].cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
