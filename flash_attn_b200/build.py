@@ -14,6 +14,11 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libfa_b200.so")
 SOURCES = ["fa_api.cu", "fa_fwd_tiled.cu", "fa_decode.cu", "fa_aux.cu", "fa_static_scratch.cu", "fa_ring.cu"]
 HEADERS = ["fa_internal.h", "sm100_ptx.cuh", "philox.cuh", os.path.join("..", "..", "include", "fa_b200.h")]
+# units of compilation (source, object, flags), longest first: the tiled kernels once for each head dimension and number of query
+# tiles a CTA (in one unit they take ptxas two minutes)
+UNITS = [("fa_fwd_tiled.cu", f"fa_fwd_tiled_{d}_{nq}.o", [f"-DFA_TILED_D={d}", f"-DFA_TILED_NQ={nq}"])
+         for d, nq in ((128, 2), (64, 2), (128, 1), (64, 1))]
+UNITS += [(f, f.replace(".cu", ".o"), []) for f in SOURCES if f != "fa_fwd_tiled.cu"]
 
 
 def nvcc_path():
@@ -23,11 +28,40 @@ def nvcc_path():
     raise RuntimeError("nvcc not found: the CUDA library cannot be built")
 
 
-def needs_build():
-    if not os.path.exists(LIB):
+def needs_build(lib=LIB):
+    if not os.path.exists(lib):
         return True
-    t = os.path.getmtime(LIB)
+    t = os.path.getmtime(lib)
     return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in SOURCES + HEADERS)
+
+
+def _compile(lib, build_dir, flags, verbose=False):
+    os.makedirs(build_dir, exist_ok=True)
+    common = [nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+              "--compress-mode=size", "-Xcompiler", "-fPIC", "-Xptxas", "-v" if verbose else "-warn-spills"] + flags
+    objs, procs = [], []
+    for src, obj, defines in UNITS:
+        objs.append(os.path.join(build_dir, obj))
+        procs.append((src, subprocess.Popen(common + defines + ["-c", os.path.join(CSRC, src), "-o", objs[-1]],
+                                            stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    failed = []
+    for src, pr in procs:
+        out, _ = pr.communicate()
+        if verbose or pr.returncode != 0:
+            sys.stderr.write(out)
+        if pr.returncode != 0:
+            failed.append(src)
+    if failed:
+        raise RuntimeError(f"nvcc failed on {', '.join(failed)}")
+    subprocess.check_call([nvcc_path(), "-shared", "-o", lib + ".new"] + objs + ["-Xcompiler", "-fPIC", "-ldl"])
+    os.replace(lib + ".new", lib)
+
+
+def build(force=False, verbose=False):
+    build_call(force)
+    if force or needs_build():
+        _compile(LIB, os.path.join(PKG, "build"), [], verbose)
+    return LIB
 
 
 CALL = os.path.join(PKG, "_call.so")
@@ -51,57 +85,15 @@ def build_call(force=False):
     return CALL
 
 
-def build(force=False, verbose=False):
-    build_call(force)
-    if not force and not needs_build():
-        return LIB
-    objs = []
-    build_dir = os.path.join(PKG, "build")
-    os.makedirs(build_dir, exist_ok=True)
-    common = [nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-Xptxas", "-v" if verbose else "-warn-spills"]
-    procs = []
-    for src in SOURCES:
-        obj = os.path.join(build_dir, src.replace(".cu", ".o"))
-        objs.append(obj)
-        procs.append((src, subprocess.Popen(common + ["-c", os.path.join(CSRC, src), "-o", obj],
-                                            stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    for src, pr in procs:
-        out, _ = pr.communicate()
-        if verbose or pr.returncode != 0:
-            sys.stderr.write(out)
-        if pr.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src}")
-    subprocess.check_call([nvcc_path(), "-shared", "-o", LIB] + objs + ["-Xcompiler", "-fPIC", "-ldl"])
-    return LIB
-
-
 TEST_LIB = os.path.join(PKG, "libfa_b200_shortwait.so")
 
 
 def build_test_variant(force=False):
     """Builds libfa_b200_shortwait.so, the library compiled with -DFA_TEST_SHORT_WAIT: bounded waits give
-    up after about 2 ms and the producer of the tiled kernel can be told to leave one KV tile out
+    up after about 2 ms and the producer of the tiled kernel can be told to leave KV tiles out
     (fa_test_skip_kv_tile).  Used only by the GPU test of the give-up path."""
-    if not force and os.path.exists(TEST_LIB) and not any(
-            os.path.getmtime(os.path.join(CSRC, f)) > os.path.getmtime(TEST_LIB) for f in SOURCES + HEADERS):
-        return TEST_LIB
-    build_dir = os.path.join(PKG, "build", "shortwait")
-    os.makedirs(build_dir, exist_ok=True)
-    common = [nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-DFA_TEST_SHORT_WAIT", "-Xcompiler", "-fPIC", "-Xptxas", "-warn-spills"]
-    procs, objs = [], []
-    for src in SOURCES:
-        obj = os.path.join(build_dir, src.replace(".cu", ".o"))
-        objs.append(obj)
-        procs.append((src, subprocess.Popen(common + ["-c", os.path.join(CSRC, src), "-o", obj],
-                                            stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    for src, pr in procs:
-        out, _ = pr.communicate()
-        if pr.returncode != 0:
-            sys.stderr.write(out)
-            raise RuntimeError(f"nvcc failed on {src} (test variant)")
-    subprocess.check_call([nvcc_path(), "-shared", "-o", TEST_LIB] + objs + ["-Xcompiler", "-fPIC", "-ldl"])
+    if force or needs_build(TEST_LIB):
+        _compile(TEST_LIB, os.path.join(PKG, "build", "shortwait"), ["-DFA_TEST_SHORT_WAIT"])
     return TEST_LIB
 
 

@@ -36,6 +36,15 @@
 #include "fa_internal.h"
 #include "sm100_ptx.cuh"
 
+// ptxas takes about half a minute for the kernels of one head dimension and number of query tiles a CTA, so this file is compiled
+// once for each of the four, side by side; the plan and the dispatch are in one of them.
+#ifndef FA_TILED_D
+#error "compiled with FA_TILED_D = 64 or 128 and FA_TILED_NQ = 1 or 2"
+#endif
+#define FA_TILED_MAIN (FA_TILED_D == 128 && FA_TILED_NQ == 2)
+#define FA_TILED_JOIN(name, d, nq) name##_##d##_##nq
+#define FA_TILED_NAME(name, d, nq) FA_TILED_JOIN(name, d, nq)
+
 // Optional timeline tracing for kernel development (compiled out unless FA_TRACE is
 // defined): lane 0 of every warp of CTA FA_TRACE_CTA records (event, clock) pairs.
 #ifdef FA_TRACE
@@ -43,7 +52,7 @@
 #define FA_TRACE_CTA 0
 #endif
 __device__ long long fa_trace_buf[16 * 512];
-extern "C" int fa_trace_read(long long* host_out) {
+extern "C" int FA_TILED_NAME(fa_trace_read, FA_TILED_D, FA_TILED_NQ)(long long* host_out) {
     return static_cast<int>(cudaMemcpyFromSymbol(host_out, fa_trace_buf, sizeof(long long) * 16 * 512));
 }
 #define FA_TR(ev)                                                                              \
@@ -64,9 +73,20 @@ extern "C" int fa_trace_read(long long* host_out) {
 // stage the wait that belongs to the tile after it would pass at once, and the stage's barrier would be armed twice in a phase.)
 #ifdef FA_TEST_SHORT_WAIT
 __device__ int fa_test_skip_tile = -1;
-extern "C" int fa_test_skip_kv_tile(int t) {
+extern "C" int FA_TILED_NAME(fa_test_skip_kv_tile, FA_TILED_D, FA_TILED_NQ)(int t) {
     return static_cast<int>(cudaMemcpyToSymbol(fa_test_skip_tile, &t, sizeof(int)));
 }
+#if FA_TILED_MAIN
+extern "C" {
+int fa_test_skip_kv_tile_64_1(int t);
+int fa_test_skip_kv_tile_64_2(int t);
+int fa_test_skip_kv_tile_128_1(int t);
+}
+extern "C" int fa_test_skip_kv_tile(int t) {
+    const int rc[4] = {fa_test_skip_kv_tile_64_1(t), fa_test_skip_kv_tile_64_2(t), fa_test_skip_kv_tile_128_1(t), fa_test_skip_kv_tile_128_2(t)};
+    return rc[0] ? rc[0] : rc[1] ? rc[1] : rc[2] ? rc[2] : rc[3];
+}
+#endif
 #define FA_TEST_SKIPS(t) (fa_test_skip_tile >= 0 && (t) >= fa_test_skip_tile)
 #else
 #define FA_TEST_SKIPS(t) false
@@ -315,7 +335,7 @@ __device__ __forceinline__ void issue_pv_rest(uint32_t d_tmem, uint32_t a_tmem, 
 }
 
 // One more k-step of S = Q K^T over the bias boxes (accumulating).
-__device__ __forceinline__ void issue_qk_bias(uint32_t d_tmem, uint32_t qa_lo, uint32_t kb_lo, uint32_t desc_hi, uint32_t idesc) {
+[[maybe_unused]] __device__ __forceinline__ void issue_qk_bias(uint32_t d_tmem, uint32_t qa_lo, uint32_t kb_lo, uint32_t desc_hi, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p1;\n\t.reg .b64 da, db;\n\t"
         "setp.eq.b32 p1, 0, 0;\n\t"
@@ -1462,12 +1482,17 @@ cudaError_t launch_flags(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
                    : launch_one<D, NQ, kBf16, false, false, false, false>(a, tq, tk, tv, to, tc, units, stream);
 }
 
-template <int D, int NQ>
-cudaError_t launch_dtype(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                         const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool alibi, bool dropout, cudaStream_t stream) {
-    return bf16 ? launch_flags<D, NQ, true>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream)
-                : launch_flags<D, NQ, false>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream);
+}  // namespace
+
+cudaError_t FA_TILED_NAME(launch_tiled, FA_TILED_D, FA_TILED_NQ)(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                                                                 const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool alibi,
+                                                                 bool dropout, cudaStream_t stream) {
+    return bf16 ? launch_flags<FA_TILED_D, FA_TILED_NQ, true>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream)
+                : launch_flags<FA_TILED_D, FA_TILED_NQ, false>(a, tq, tk, tv, to, tc, units, alibi, dropout, stream);
 }
+
+#if FA_TILED_MAIN
+namespace {
 
 // two query tiles per CTA once a unit has more than one; a single tile (decode-like
 // shapes) keeps two independent CTAs per SM instead
@@ -1681,12 +1706,9 @@ cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUte
                              const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream) {
     const bool alibi = a.alibi_slopes != nullptr;
     const bool pair = a.pair != 0;
-    if (a.head_dim <= 64) {
-        return pair ? launch_dtype<64, 2>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream)
-                    : launch_dtype<64, 1>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);
-    }
-    return pair ? launch_dtype<128, 2>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream)
-                : launch_dtype<128, 1>(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);
+    const auto launch = a.head_dim <= 64 ? (pair ? launch_tiled_64_2 : launch_tiled_64_1) : pair ? launch_tiled_128_2 : launch_tiled_128_1;
+    return launch(a, tq, tk, tv, to, tc, units, bf16, alibi, dropout, stream);
 }
+#endif
 
 }  // namespace fa

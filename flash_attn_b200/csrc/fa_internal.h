@@ -86,6 +86,11 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room, bool dropout);
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream);
 
+// ... for one head dimension and number of query tiles a CTA (each a unit of compilation of fa_fwd_tiled.cu).
+typedef cudaError_t launch_tiled_fn(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                                    const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool alibi, bool dropout, cudaStream_t stream);
+launch_tiled_fn launch_tiled_64_1, launch_tiled_64_2, launch_tiled_128_1, launch_tiled_128_2;
+
 // Device-side argument block of the decode kernel (seqlen_q <= 8).
 struct DecodeArgs {
     const void* q;          // [units, seqlen_q, d]
