@@ -170,10 +170,28 @@ def load():
     L.fa_strerror.restype = ctypes.c_char_p
     L.fa_version.argtypes = []
     L.fa_version.restype = ctypes.c_int
-    from . import _call  # the call path on torch tensors (csrc/fa_torch.cpp), bound to this library's entry points
-    L.forward = functools.partial(_call.forward, *(ctypes.cast(f, ctypes.c_void_p).value for f in (L.fa_fwd, L.fa_fwd_workspace_bytes)))
     _lib = L
     return L
+
+
+forward = None  # the call path on torch tensors, once load_call has run
+
+
+def load_call():
+    """The call path on torch tensors (csrc/fa_torch.cpp), bound to the library's entry points.  Only flash_attn_forward needs
+    it: a module that is missing or was built for another torch leaves the C entry points usable."""
+    global forward
+    L = load()
+    import torch
+    built = "build it with `python -m flash_attn_b200.build`"
+    try:
+        from . import _call
+    except ImportError as e:
+        raise ImportError(f"the call path on torch tensors cannot be loaded ({e}): {built}") from e
+    if _call.built_for != torch.__version__:
+        raise ImportError(f"the call path was built for torch {_call.built_for}, this is {torch.__version__}: {built}")
+    forward = functools.partial(_call.forward, *(ctypes.cast(f, ctypes.c_void_p).value for f in (L.fa_fwd, L.fa_fwd_workspace_bytes)))
+    return forward
 
 
 def strerror(code):

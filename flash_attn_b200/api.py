@@ -75,9 +75,9 @@ def flash_attn_forward(q, k, v, softmax_scale=None, causal=False, window=(-1, -1
     the others return (None, None).
     """
     # (the whole call is native: see csrc/fa_torch.cpp)
-    done = _lib.load().forward(q, k, v, softmax_scale, causal, window, alibi_slopes, p_dropout, seed, offset, num_splits, out,
-                               out_dtype, return_lse, q_pos0, k_pos0, unit0, workspace, status, accum, accum_first,
-                               accum_final, launch_index)
+    forward = _lib.forward or _lib.load_call()
+    done = forward(q, k, v, softmax_scale, causal, window, alibi_slopes, p_dropout, seed, offset, num_splits, out, out_dtype,
+                   return_lse, q_pos0, k_pos0, unit0, workspace, status, accum, accum_first, accum_final, launch_index)
     if type(done) is int:
         _lib.check(done, "fa_fwd")
     return done

@@ -1,4 +1,4 @@
-"""Builds libfa_b200.so (the C-ABI library, nvcc for sm_100a) and _call.so (its call path on torch tensors) in-tree.
+"""Builds libfa_b200.so (the C-ABI library, nvcc for sm_100a) and _call.<ABI>.so (its call path on torch tensors) in-tree.
 
     python -m flash_attn_b200.build [--force] [--verbose]
 
@@ -8,6 +8,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -57,32 +58,50 @@ def _compile(lib, build_dir, flags, verbose=False):
     os.replace(lib + ".new", lib)
 
 
-def build(force=False, verbose=False):
-    build_call(force)
-    if force or needs_build():
-        _compile(LIB, os.path.join(PKG, "build"), [], verbose)
-    return LIB
+# The call path is C++ against this Python and this torch: the file's name carries the one's ABI tag, and what it was built
+# from (torch's version and the compiler's arguments) is kept beside the objects and in the module (_call.built_for).
+CALL = os.path.join(PKG, "_call" + sysconfig.get_config_var("EXT_SUFFIX"))
+CALL_SOURCE = os.path.join(CSRC, "fa_torch.cpp")
 
 
-CALL = os.path.join(PKG, "_call.so")
-
-
-def build_call(force=False):
-    """Builds _call.so (csrc/fa_torch.cpp: flash_attn_forward on torch tensors) against the installed torch."""
-    src = os.path.join(CSRC, "fa_torch.cpp")
-    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(PKG, "..", "include", "fa_b200.h")))
-    if not force and os.path.exists(CALL) and os.path.getmtime(CALL) >= newest:
-        return CALL
-    import sysconfig
+def _call_command():
     import torch
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(nvcc_path()))
-    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
-                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-                           "-isystem", os.path.join(tdir, "include"), "-isystem", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
-                           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"), src, "-o", CALL,
-                           "-L", os.path.join(tdir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f'-DFA_BUILT_FOR="{torch.__version__}"',
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-isystem", os.path.join(tdir, "include"), "-isystem", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+            "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"), CALL_SOURCE,
+            "-L", os.path.join(tdir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
+def needs_build_call():
+    stamp = os.path.join(PKG, "build", os.path.basename(CALL) + ".txt")
+    if not os.path.exists(CALL) or not os.path.exists(stamp):
+        return True
+    newest = max(os.path.getmtime(CALL_SOURCE), os.path.getmtime(os.path.join(PKG, "..", "include", "fa_b200.h")))
+    with open(stamp) as f:
+        return os.path.getmtime(CALL) < newest or f.read() != "\n".join(_call_command())
+
+
+def build_call(force=False):
+    """Builds the module of csrc/fa_torch.cpp (flash_attn_forward on torch tensors) against the installed torch."""
+    if force or needs_build_call():
+        os.makedirs(os.path.join(PKG, "build"), exist_ok=True)
+        command = _call_command()
+        subprocess.check_call(command + ["-o", CALL + ".new"])
+        os.replace(CALL + ".new", CALL)
+        with open(os.path.join(PKG, "build", os.path.basename(CALL) + ".txt"), "w") as f:
+            f.write("\n".join(command))
     return CALL
+
+
+def build(force=False, verbose=False):
+    """The library first: it and the C callers need neither torch nor Python."""
+    if force or needs_build():
+        _compile(LIB, os.path.join(PKG, "build"), [], verbose)
+    build_call(force)
+    return LIB
 
 
 TEST_LIB = os.path.join(PKG, "libfa_b200_shortwait.so")

@@ -280,4 +280,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_call", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__call() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__call() {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", FA_BUILT_FOR) != 0) {  // (torch's version: other versions have other classes)
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}
