@@ -134,20 +134,27 @@ struct Cfg {
     static constexpr int kSmemK = NQ * kTileBytes;
     static constexpr int kSmemV = kSmemK + kStages * kTileBytes;
     static constexpr int kSmemBar = kSmemV + kStages * kTileBytes;
-    static constexpr int kNumBars = 2 + 3 * NQ + 4 * kStages;
+    static constexpr int kNumBars = 1 + 2 * NQ + 4 * kStages;
     static_assert(kNumBars <= 32, "a lane initialises each");
     // dropout keep bits, written by a helper warp per query tile: [NQ][2 row halves][kKeepRing tiles] words
     static constexpr int kSmemKeep = kSmemBar + 8 * kNumBars + 16;
-    static constexpr int kSmemBytes = kSmemKeep + NQ * kKeepRing * 2 * 4 + 1024;  // + alignment slack
+    static constexpr int kSmemRun = kSmemKeep + NQ * kKeepRing * 2 * 4;  // barriers of a launch that merges into a running result
+    static constexpr int kSmemEnd = kSmemRun + 8 * (1 + NQ);
+    static constexpr int kSmemBytes = kSmemEnd + 1024;  // + alignment slack
     static constexpr int kKeepWarp0 = NQ * 4 + 2;  // the helper warp of query tile i is kKeepWarp0 + i
     // ALiBi whose bias is linear in the key position (every visible key at or before the query) is added by
     // the tensor core: one more K = 16 step per Q K^T over two extra 64-column boxes, [1 1 0 ...] for every
     // query row and [hi lo 0 ...] of slope * column / scale for every key row of a tile (two 16-bit terms
     // carry the bias to 2^-17 relative).  Two-tile CTAs only: a single-tile CTA shares its SM.
     static constexpr bool kBiasBoxes = NQ == 2;
-    static constexpr int kSmemBiasQ = (kSmemKeep + NQ * kKeepRing * 2 * 4 + 1023) / 1024 * 1024;
+    static constexpr int kSmemBiasQ = (kSmemEnd + 1023) / 1024 * 1024;
     static constexpr int kSmemBiasK = kSmemBiasQ + kTile * 128;
     static constexpr int kSmemBytesBias = kSmemBiasK + kTile * 128 + 1024;  // dynamic shared memory of the ALiBi kernels
+};
+
+// What the kernels that merge into a running result are launched with: the load map of that result too.
+struct alignas(64) RunningArgs : FwdArgs {
+    CUtensorMap tmap_c;
 };
 
 struct TileRange {
@@ -466,7 +473,7 @@ template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, b
 __global__ void __launch_bounds__(Cfg<D, NQ>::kThreads, NQ == 1 ? 2 : 1)
 fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
-                 const __grid_constant__ CUtensorMap tmap_c, const FwdArgs a) {
+                 const __grid_constant__ std::conditional_t<kRunning, RunningArgs, FwdArgs> a) {
     using C = Cfg<D, NQ>;
     extern __shared__ uint8_t smem_raw[];
     // 128-byte-swizzled tiles need a 1024-byte aligned base
@@ -484,7 +491,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t bar_k_empty = bar_k_full + 8 * C::kStages;    // [kStages]
     const uint32_t bar_v_full = bar_k_empty + 8 * C::kStages;    // [kStages]
     const uint32_t bar_v_empty = bar_v_full + 8 * C::kStages;    // [kStages]
-    const uint32_t bar_qk_done = bar_v_empty + 8 * C::kStages;   // running result only: Q and the K ring are free
+    const uint32_t bar_qk_done = smem_base + C::kSmemRun;        // running result only: Q and the K ring are free
     const uint32_t bar_carry = bar_qk_done + 8;                  // [NQ] carried rows have landed
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kSmemBar + 8 * C::kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + C::kSmemBar + 8 * C::kNumBars + 4);
@@ -507,6 +514,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // the maps are kernel parameters, not memory of the kernel in front.
     if (warp == C::kProducerWarp) {
         if (lane < C::kNumBars) mbar_init(bar0 + 8 * lane, 1);
+        if (kRunning && lane < 1 + NQ) mbar_init(bar_qk_done + 8 * lane, 1);
         if (lane == 0) {
             *abort_flag = 0;
             tma_prefetch_desc(&tmap_q);
@@ -709,7 +717,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
     int fail = 0;
     // Rows carried from launch to launch: they lie, 32 fp32 columns a box, in the Q buffer of their query tile and in a stage of the K ring.
-    const bool carry = kRunning && a.accum_o != nullptr && !a.accum_first;
+    const bool carry = kRunning && !a.accum_first;
     auto carry_box = [&](int i, int b) {
         return b < C::kBoxes ? sQ + i * C::kTileBytes + b * (kTile * 128) : sK + i * C::kTileBytes + (b - C::kBoxes) * (kTile * 128);
     };
@@ -719,9 +727,9 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // regime covers one whole branch below.
     if (warp >= NQ * 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsHelper));
-        if (warp == C::kProducerWarp) {
+        if ((kRunning || n_union > 0) && warp == C::kProducerWarp) {
             // ======================= TMA producer ===================================
-            if (n_union > 0 && lane == 0) {
+            if ((!kRunning || n_union > 0) && lane == 0) {
                 for (int t = prefilled; t < n_union; ++t) {
                     if (FA_TEST_SKIPS(t)) continue;
                     const int st = t % C::kStages;
@@ -741,7 +749,8 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                         tma_load_3d(sV + st * C::kTileBytes + b * (kTile * 128), &tmap_v, bar_v_full + 8 * st, b * 64, row, kv_unit);
                 }
             }
-            if (kRunning && carry) {
+            if constexpr (kRunning) {
+            if (carry) {
                 // The carried rows start as soon as the last Q K^T has read the buffers that take them, about a tile and a half
                 // ahead of their use (a CTA without keys: Q has landed before the CTA-wide sync).
                 __syncwarp();
@@ -750,10 +759,11 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 const int i = lane % NQ, b = lane / NQ;
                 if (free && b < 2 * C::kBoxes && qb * NQ + i < a.tr) {
                     if (b == 0) mbar_expect_tx(bar_carry + 8 * i, 2 * C::kTileBytes);
-                    tma_load_3d(carry_box(i, b), &tmap_c, bar_carry + 8 * i, b * 32, (qb * NQ + i) * kTile, unit);
+                    tma_load_3d(carry_box(i, b), &a.tmap_c, bar_carry + 8 * i, b * 32, (qb * NQ + i) * kTile, unit);
                 } else if (!free && fail == 0) {
                     fail = 10;
                 }
+            }
             }
         } else if (n_union > 0 && warp == C::kMmaWarp) {
             // ======================= MMA issuer =====================================
@@ -1210,7 +1220,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         //   lse' = log(e^lse_c + e^lse),  O' = e^(lse_c - lse') O_c + e^(lse - lse') O,
         // here in the epilogue, on the row each thread already holds, instead of in a pass of its own.
         float w_old = 0.0f;  // weight of the carried row
-        if (kRunning && a.accum_o != nullptr) {
+        if constexpr (kRunning) {
             const long long arow = unit_ll * a.seqlen_q + row;
             float lse_c = -INFINITY;
             if (!a.accum_first && row_ok) lse_c = a.accum_lse[arow];
@@ -1237,7 +1247,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         } else if (a.lse != nullptr && row_ok) {
             a.lse[unit_ll * a.seqlen_q + row] = lse_val;
         }
-        if (a.o_tma && have_o) {
+        if (!kRunning && a.o_tma && have_o) {
             // 16-bit output of an unsplit launch: the rows are staged in this query tile's Q buffer
             // (free once the last Q K^T has completed, which o_full implies) in the 128-byte-swizzled
             // box layout, and each warp hands its 32 rows to the TMA unit, which writes whole lines
@@ -1272,7 +1282,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             FA_TR(97);
             if (lane == 0) tma_store_wait_read();
-        } else if (kRunning && a.accum_o != nullptr) {
+        } else if constexpr (kRunning) {
             // Read-modify-write of the carried row, 32 columns at a time, in the box that its TMA load has brought; each warp stores
             // its 32 rows of a box.  The sequence's last block leaves the 16-bit output instead, over the boxes it has read.
             // Bound by the latency of a CTA's end (one CTA an SM: nothing overlaps it): a thread that read and wrote its own row in
@@ -1412,8 +1422,11 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 }
 
 template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, bool kRunning>
-cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                       const CUtensorMap& to, const CUtensorMap& tc, int units, cudaStream_t stream) {
+cudaError_t launch_one(const FwdArgs& args, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                       const CUtensorMap& to, [[maybe_unused]] const CUtensorMap& tc, int units, cudaStream_t stream) {
+    std::conditional_t<kRunning, RunningArgs, FwdArgs> a;
+    static_cast<FwdArgs&>(a) = args;
+    if constexpr (kRunning) a.tmap_c = tc;
     auto kern = fwd_tiled_kernel<D, NQ, kBf16, kAlibi, kDropout, kStaged, kRunning>;
     constexpr int smem = (kAlibi && Cfg<D, NQ>::kBiasBoxes) ? Cfg<D, NQ>::kSmemBytesBias : Cfg<D, NQ>::kSmemBytes;
     static_assert(smem <= 232448, "beyond the 227 KB a CTA may have");
@@ -1457,7 +1470,7 @@ cudaError_t launch_one(FwdArgs a, const CUtensorMap& tq, const CUtensorMap& tk, 
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         if (a.parts > 1) cfg.numAttrs = 2;
     }
-    return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, tc, a);
+    return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, a);
 }
 
 template <int D, int NQ, bool kBf16>
