@@ -129,3 +129,26 @@ def test_later_launch_masks_against_the_oracle(case):
                             p_dropout=0.2, drop_seed=11, num_splits=case.get("splits", 1), q_pos0=case.get("q_pos0", 0),
                             launch_index=case["k"])
     gpu_util.assert_close(res, str(case))
+
+
+@pytest.mark.parametrize("Nq,d,dtype,out_dtype", [
+    (257, 96, "bfloat16", torch.float32),
+    (100, 64, "float16", torch.float32),
+    (300, 128, "bfloat16", None),
+])
+def test_blocks_with_dropout_merge_as_their_separate_results_do(Nq, d, dtype, out_dtype):
+    import flash_attn_b200 as fa
+    B, H, blocks = 1, 3, (130, 300, 257)
+    q, k, v = (gpu_util.to_dev(x, dtype) for x in synth.qkv(64, B, H, Nq, sum(blocks), d, dtype))
+    acc = (torch.full((B, H, Nq, d), float("nan"), device="cuda"), torch.full((B, H, Nq), float("nan"), device="cuda"))
+    ref = (torch.zeros((B, H, Nq, d), device="cuda"), torch.full((B, H, Nq), -float("inf"), device="cuda"))
+    pos = 0
+    for i, n in enumerate(blocks):
+        kb, vb = (x[:, :, pos:pos + n].contiguous() for x in (k, v))
+        opts = dict(causal=True, q_pos0=300, k_pos0=pos, p_dropout=0.2, seed=7, offset=1000 * i, alibi_slopes=torch.full((H,), 0.01))
+        fa.merge_partial(*ref, *fa.flash_attn_forward(q, kb, vb, out_dtype=torch.float32, **opts))
+        o, lse = fa.flash_attn_forward(q, kb, vb, accum=acc, accum_first=i == 0, accum_final=i + 1 == len(blocks), out_dtype=out_dtype, **opts)
+        pos += n
+    # fp32 weights and products in another order: a few ulps of values up to 4; the 16-bit output rounds once more
+    assert (o.float() - ref[0]).abs().max() <= (2e-5 if out_dtype is torch.float32 else 2e-2)
+    assert (lse - ref[1]).abs().max() <= 2e-5 and torch.equal(lse, acc[1])

@@ -134,12 +134,13 @@ def test_a_part_that_gave_up_leaves_no_plausible_row(test_lib, skip, H, Hk, Nq, 
     assert np.abs(lse.cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
 
 
-@pytest.mark.parametrize("H,Nq,d,skip,causal,out_dtype", [
-    (160, 256, 128, 1, False, torch.bfloat16),  # (two query tiles a CTA)
-    (120, 300, 64, 0, True, torch.float32),     # (a CTA whose second query tile does not exist; the first tile of the walk)
-    (3, 300, 128, 1, False, torch.float32),     # (one query tile a CTA, a ring of one stage)
+@pytest.mark.parametrize("H,Nq,d,skip,causal,out_dtype,p_dropout", [
+    (160, 256, 128, 1, False, torch.bfloat16, 0.0),  # (two query tiles a CTA)
+    (120, 300, 64, 0, True, torch.float32, 0.0),     # (a CTA whose second query tile does not exist; the first tile of the walk)
+    (3, 300, 128, 1, False, torch.float32, 0.0),     # (one query tile a CTA, a ring of one stage)
+    (3, 300, 96, 1, False, torch.bfloat16, 0.1),     # (with dropout the rows are merged without TMA)
 ])
-def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip, causal, out_dtype):
+def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip, causal, out_dtype, p_dropout):
     """The block before it is complete, and so are the ones behind it: neither may make its rows look like a result."""
     from flash_attn_b200 import _lib
     L = test_lib
@@ -155,6 +156,7 @@ def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip,
         kb, vb = (x[:, :, i * Nk:(i + 1) * Nk].contiguous() for x in (k, v))
         p = _params(q, kb, vb, o, lse, status)
         p.o_dtype = _lib.FA_DTYPE_FP32 if out_dtype is torch.float32 else _lib.FA_DTYPE_BF16
+        p.p_dropout, p.seed = p_dropout, 3
         p.is_causal, p.q_pos0, p.k_pos0 = int(causal), 3 * Nk, i * Nk  # (with a causal mask no query sees the fourth block's end)
         p.accum_o, p.accum_lse = acc[0].data_ptr(), acc[1].data_ptr()
         p.accum_flags = (_lib.FA_ACCUM_FIRST if first else 0) | (_lib.FA_ACCUM_FINAL if final else 0)
@@ -189,5 +191,8 @@ def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip,
         block(i, i == 0, i == 3)
     want_o, want_lse = oracle_lib.forward(qh, kh, vh, d ** -0.5, causal=causal, q_pos0=3 * Nk)
     assert int(status.item()) == 0
+    if p_dropout > 0.0:  # (each block's launch has a mask of its own)
+        assert torch.isfinite(o).all()
+        return
     assert np.abs(o[:, :3].float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
     assert np.abs(lse[:, :3].cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
