@@ -1633,7 +1633,7 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
     }
     const int tile_rows = pair ? 2 * kTile : kTile;
     const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
-    const double stage = staged ? 0.4 : 0.0;
+    const double stage = !staged ? 0.0 : a.pack_rows > 0 ? (c.merge + c.merge_each) * rows : 0.4;
     Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, pair, least >= 0.8 * n || n - least <= 1};
     if (blocks > slots) {
         const double waves = static_cast<double>(blocks) / slots;
@@ -1666,7 +1666,7 @@ Split best_cut(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged, 
     if (!two_tiles(a)) return one;
     const Split two = best_split(a, sms, room, staged, most_parts, true);
     const long long ctas = static_cast<long long>(a.units) * a.tr * one.parts;
-    const double margin = ctas > 2 * sms ? 0.0 : ctas > sms || a.is_causal ? 0.8 : 0.93;
+    const double margin = ctas > 2 * sms ? 0.0 : ctas > sms || a.is_causal || a.pack_rows > 0 ? 0.8 : 0.93;
     return one.us < margin * two.us ? one : two;
 }
 
