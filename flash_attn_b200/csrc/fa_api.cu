@@ -157,25 +157,27 @@ int resolve_splits(const fa_fwd_params* p, int sms) {
     return std::max(1, std::min(s, tc));
 }
 
-// Units whose CTAs are interleaved in launch order.  Query blocks of one length (no mask that shortens the first ones by more
-// than a fifth) go unit by unit, which keeps neighbouring CTAs on the same K/V tiles in L2: [1,32,8192,128] against 8192 keys
-// before it 837 us in groups of 16, 812 unit by unit.  Causal blocks go heaviest first over groups of 16 units, near a
-// longest-job-first schedule ([8,16,2048,128] 142 us, 148 unit by unit; 8192 rows 435 and 473), or of fewer where a
-// group's K/V would pass 48 MB (L2 holds 126 MB in two halves): [1,32,16384,128] 1684 us in groups of 16, 1655 / 1651 / 1672 of
+// Units whose CTAs are interleaved in launch order.  Query blocks of one length, to a twentieth, go unit by unit, which keeps
+// neighbouring CTAs on the same K/V tiles in L2: [1,32,8192,128] against 8192 keys before it 837 us in groups of 16, 812 unit by
+// unit, [1,64,1024,128] at the end of 16384 keys 457 and 446.  Others go heaviest first over groups of 16 units, near
+// a longest-job-first schedule ([8,16,2048,128] causal 142 us, 148 unit by unit; 8192 rows 435 and 473; 2048 rows at the end of
+// 16384 keys, whose blocks differ by a tenth, 431 and 472).  The groups are smaller where one of 16 is more than the CTAs in flight and its
+// K/V would pass 48 MB (L2 holds 126 MB in two halves): [1,32,16384,128] 1684 us in groups of 16, 1655 / 1651 / 1672 of
 // 8 / 4 / 2, [1,16,32768,128] 3276 against 3242 / 3217 / 3215.  (Powers of two: groups of 6 leave one of 2 behind and take 1729.)
-int unit_group(const fa_fwd_params* p, int kv_group) {
+int unit_group(const fa_fwd_params* p, int kv_group, int sms) {
     if (!p->is_causal || p->window_left >= 0) return 1;
     const long long nk = p->seqlen_k, start = p->q_pos0 - p->k_pos0;
     auto visible = [&](long long row) { return std::max(0LL, std::min(nk, start + row + 1)); };
     const long long first = visible(std::min(p->seqlen_q, 2 * kTile) - 1), last = visible(p->seqlen_q - 1);
-    if (5 * first >= 4 * last) return 1;
+    if (20 * first >= 19 * last) return 1;
+    const long long blocks = (p->seqlen_q + 2 * kTile - 1) / (2 * kTile);
     const double unit_bytes = 4.0 * static_cast<double>(last) * p->head_dim / kv_group;
-    int units = 16;
-    while (units > 1 && units * unit_bytes > 48.0 * 1048576.0) units /= 2;
+    int units = kUnitGroup;
+    while (units > 1 && units * blocks > sms && units * unit_bytes > 48.0 * 1048576.0) units /= 2;
     return units;
 }
 
-void fill_args(const fa_fwd_params* p, int splits, FwdArgs* a) {
+void fill_args(const fa_fwd_params* p, int splits, int sms, FwdArgs* a) {
     std::memset(a, 0, sizeof(*a));
     a->o = p->o;
     a->lse = p->lse;
@@ -184,7 +186,7 @@ void fill_args(const fa_fwd_params* p, int splits, FwdArgs* a) {
     a->heads = p->heads;
     a->units = p->batch * p->heads;
     a->kv_group = p->heads / kv_heads(p);
-    a->unit_group = unit_group(p, a->kv_group);
+    a->unit_group = unit_group(p, a->kv_group, sms);
     a->seqlen_q = p->seqlen_q;
     a->seqlen_k = p->seqlen_k;
     a->head_dim = p->head_dim;
@@ -240,7 +242,7 @@ int planned_parts(const fa_fwd_params* p, int splits, int sms) {
     if (p->seqlen_q > 8 || p->accum_o != nullptr) return p->p_dropout > 0.0f ? splits : 1;
     FwdArgs a;
     DecodeArgs d;
-    fill_args(p, splits, &a);
+    fill_args(p, splits, sms, &a);
     fill_decode_args(p, a, &d);
     plan_decode(&d, p->batch * p->heads, splits, most_parts(p, splits), sms, cluster_room(sms));
     return d.merge ? 1 : d.parts;
@@ -270,7 +272,7 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
     const int units = p->batch * p->heads;
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
     FwdArgs a;
-    fill_args(p, splits, &a);
+    fill_args(p, splits, sms, &a);
     a.o_dim = o_dim;
     const bool decode = p->seqlen_q <= 8 && p->accum_o == nullptr;
     DecodeArgs d;
@@ -410,7 +412,7 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd
     fa_fwd_params q = *p;
     q.head_dim = (p->head_dim + 7) / 8 * 8;
     FwdArgs a;
-    fill_args(&q, splits, &a);
+    fill_args(&q, splits, num_sms, &a);
     std::memset(plan, 0, sizeof(*plan));
     if (p->seqlen_q <= 8 && p->accum_o == nullptr) {
         DecodeArgs d;
@@ -498,7 +500,7 @@ int fa_dropout_mask(const fa_fwd_params* p, uint8_t* keep) {
     int sms = 148, major = 10;
     if (p->num_splits == 0 && (rc = sm_count_of_current_device(&sms, &major)) != FA_OK) return rc;
     FwdArgs a;
-    fill_args(p, resolve_splits(p, sms), &a);
+    fill_args(p, resolve_splits(p, sms), sms, &a);
     if (!(p->p_dropout > 0.0f)) a.drop.threshold = 0ull;
     if (launch_dropout_mask(a, keep, static_cast<long long>(p->batch) * p->heads,
                             static_cast<cudaStream_t>(p->stream)) != cudaSuccess)

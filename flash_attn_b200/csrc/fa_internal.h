@@ -67,6 +67,8 @@ struct FwdArgs {
     DropoutParams drop;
 };
 
+constexpr int kUnitGroup = 16;  // units whose CTAs are interleaved in launch order where query blocks differ in length, at most
+
 // Clusters that the device holds at once.  A cluster lies within a GPC, and GPCs differ in their SMs from device to device: a
 // B200 with 148 SMs holds 74 clusters of 2 CTAs at one CTA an SM, 45 of 3, 33 of 4, 26 of 5, 22 of 6, 15 of 7 or 8, 7 of 16.
 struct ClusterRoom {
