@@ -99,10 +99,15 @@ namespace {
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: rescale O only when the max grew by > 2^8
 // Which column pairs take the polynomial exp2: one pair of every four (a quarter of the elements), bit
 // 4*(g%2) + q = pair q of an even / odd group of eight columns.  The position decides how the cubic's FMAs
-// interleave with the MUFU results around them; measured over all sixteen placements, pair 0 everywhere is
-// the fastest without dropout and pairs 0 / 1 of even / odd groups with it (up to 2 % between placements).
-constexpr uint32_t kPolyMaskPlain = 0x11u;
-constexpr uint32_t kPolyMaskDropout = 0x21u;
+// interleave with the MUFU results around them, and which is the best changes with the code around the loop (up to 5 % between the
+// sixteen placements), so it is measured per kernel.  D = 128 without ALiBi, with the running result in instances of its own: pair 3
+// everywhere (pair 0, the best before: [28 heads on 4, 849, 11656 keys] 151.6 us against 149.2, [1,32,2048,16384] 440.0 against
+// 433.9, [1,32,8192,128] causal 434.8 against 431.6).  The others as they were: pair 0, with dropout pairs 0 / 1 of
+// even / odd groups.
+constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, [[maybe_unused]] bool masked) {
+    if (d == 128 && !alibi) return dropout ? 0x21u : 0x88u;
+    return dropout ? 0x21u : 0x11u;
+}
 constexpr int kKeepChunk = 2;              // KV tiles whose dropout keep bits are handed over at a time (one Philox pass)
 constexpr int kKeepRing = 2 * kKeepChunk;  // tiles the keep-bit table holds
 constexpr float kLog2e = 1.4426950408889634f;
@@ -1053,8 +1058,8 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             // polynomial needs finite arguments: on tiles with masked (-inf) scores its results for those
             // elements are replaced by 0 (MUFU gives 0 by itself).
             auto exp_tile = [&](auto guard_tag) {
-                constexpr uint32_t kPolyMask = kDropout ? kPolyMaskDropout : kPolyMaskPlain;
                 constexpr bool kGuard = decltype(guard_tag)::value;  // the tile has masked (-inf) scores
+                constexpr uint32_t kPolyMask = poly_mask(D, kAlibi, kDropout, kGuard);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {  // quarters of 32 columns
                     uint32_t pr[16];
