@@ -104,7 +104,7 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units: rescale O only when th
 // everywhere (pair 0, the best before: [28 heads on 4, 849, 11656 keys] 151.6 us against 149.2, [1,32,2048,16384] 440.0 against
 // 433.9, [1,32,8192,128] causal 434.8 against 431.6).  The others as they were: pair 0, with dropout pairs 0 / 1 of
 // even / odd groups.
-constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, [[maybe_unused]] bool masked) {
+__host__ __device__ constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, [[maybe_unused]] bool masked) {
     if (d == 128 && !alibi) return dropout ? 0x21u : 0x88u;
     return dropout ? 0x21u : 0x11u;
 }
