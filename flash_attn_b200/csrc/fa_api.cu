@@ -327,7 +327,7 @@ int run_fwd(const fa_fwd_params* p, int o_dim, int splits, int sms) {
         a.o_tma = (!a.staged && a.num_splits == 1 && p->o_dtype != FA_DTYPE_FP32 && p->accum_o == nullptr) ? 1 : 0;
         if (a.o_tma && (rc = make_tensor_map(&to, p->dtype, p->o, p->head_dim, p->seqlen_q, units, 32)) != FA_OK) return rc;
         CUtensorMap tc = tq;
-        if (p->accum_o != nullptr && !dropout) {
+        if (p->accum_o != nullptr) {
             // the running result comes and goes by TMA too; the last block stores the output instead
             const bool last = a.accum_final && p->o != nullptr;
             if ((rc = make_tensor_map(&tc, FA_DTYPE_FP32, p->accum_o, p->head_dim, p->seqlen_q, units)) != FA_OK) return rc;

@@ -102,10 +102,12 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units: rescale O only when th
 // interleave with the MUFU results around them, and which is the best changes with the code around the loop (up to 5 % between the
 // sixteen placements), so it is measured per kernel.  D = 128 without ALiBi, with the running result in instances of its own: pair 3
 // everywhere (pair 0, the best before: [28 heads on 4, 849, 11656 keys] 151.6 us against 149.2, [1,32,2048,16384] 440.0 against
-// 433.9, [1,32,8192,128] causal 434.8 against 431.6).  The others as they were: pair 0, with dropout pairs 0 / 1 of
+// 433.9, [1,32,8192,128] causal 434.8 against 431.6); with dropout pairs 3 / 1 of even / odd groups on full tiles and none on masked
+// ones, which then need no guard (pairs 0 / 1 on all: [8,16,2048,128] causal, p = 0.1 144.5 us against 142.9, [2,16,1024,128] x 8192 keys
+// 117.3 against 116.7; of masked tiles with pairs 3 / 1 too 144.2).  The others as they were: pair 0, with dropout pairs 0 / 1 of
 // even / odd groups.
-__host__ __device__ constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, [[maybe_unused]] bool masked) {
-    if (d == 128 && !alibi) return dropout ? 0x21u : 0x88u;
+__host__ __device__ constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, bool masked) {
+    if (d == 128 && !alibi) return dropout ? (masked ? 0u : 0x28u) : 0x88u;
     return dropout ? 0x21u : 0x11u;
 }
 constexpr int kKeepChunk = 2;              // KV tiles whose dropout keep bits are handed over at a time (one Philox pass)
@@ -472,10 +474,9 @@ __device__ __forceinline__ void merge_rows(const FwdArgs& a, uint8_t* smem_gen, 
 }
 
 // kRunning: the launch merges into a running result whose rows come and go by TMA.  Those kernels are instances of their own: with
-// that epilogue, its barriers and its map in every kernel a short launch takes longer ([4,16,512,128] causal 11.53 us against 11.22).
-// With dropout the running result is read and written a row a thread by the ordinary kernels instead: without that code behind it
-// the softmax loop comes out of ptxas slower on masked tiles ([8,16,2048,128] causal, p = 0.1: 142.8 us against 141.7, with the
-// TMA epilogue 145), and launches that merge nothing are what dropout is used for.
+// that epilogue, its barriers and its map in every kernel a short launch takes longer ([4,16,512,128] causal 11.53 us against 11.22)
+// and ptxas finds the dropout kernels' softmax loop another schedule ([8,16,2048,128] causal, p = 0.1: 171.5 us against 168 under
+// the power cap).
 template <int D, int NQ, bool kBf16, bool kAlibi, bool kDropout, bool kStaged, bool kRunning>
 __global__ void __launch_bounds__(Cfg<D, NQ>::kThreads, NQ == 1 ? 2 : 1)
 fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -1227,13 +1228,13 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         //   lse' = log(e^lse_c + e^lse),  O' = e^(lse_c - lse') O_c + e^(lse - lse') O,
         // here in the epilogue, on the row each thread already holds, instead of in a pass of its own.
         float w_old = 0.0f;  // weight of the carried row
-        if (kRunning || (kDropout && a.accum_o != nullptr)) {
+        if constexpr (kRunning) {
             const long long arow = unit_ll * a.seqlen_q + row;
             float lse_c = -INFINITY;
             if (!a.accum_first && row_ok) lse_c = a.accum_lse[arow];
             // The buffers of the carried rows, before anything of this launch's is written: if a wait gave up, here or before, neither
             // the rows nor their sums may pass for a running result, so both become NaN, which later launches carry on.
-            if (kRunning && (carry || n_union > 0) && rb < a.tr && !mbar_wait_warp(carry ? bar_carry + 8 * qi : bar_qk_done, 0, abort_flag) && fail == 0) fail = 11;
+            if ((carry || n_union > 0) && rb < a.tr && !mbar_wait_warp(carry ? bar_carry + 8 * qi : bar_qk_done, 0, abort_flag) && fail == 0) fail = 11;
             if (fail != 0) lse_c = __int_as_float(0x7fc00000);
             const float m = fmaxf(lse_c, lse_val);
             float lse_new = -INFINITY, w_new = 0.0f;
@@ -1368,54 +1369,6 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             if (!row_ok) continue;
             const int col0 = c * 32;
-            if (kDropout && a.accum_o != nullptr) {
-                // the running result: read-modify-write of the carried fp32 row (each thread walks its own row;
-                // the two 16-byte halves of every 32-byte sector are touched by consecutive
-                // instructions), and on the sequence's last block the output instead
-                float* acc = a.accum_o + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    if (col0 + i < a.head_dim) {
-                        float4 v4 = make_float4(__uint_as_float(orow[i]) * inv, __uint_as_float(orow[i + 1]) * inv,
-                                                __uint_as_float(orow[i + 2]) * inv, __uint_as_float(orow[i + 3]) * inv);
-                        if (w_old != 0.0f) {
-                            const float4 c4 = *reinterpret_cast<const float4*>(acc + col0 + i);
-                            v4.x = fmaf(w_old, c4.x, v4.x);
-                            v4.y = fmaf(w_old, c4.y, v4.y);
-                            v4.z = fmaf(w_old, c4.z, v4.z);
-                            v4.w = fmaf(w_old, c4.w, v4.w);
-                        }
-                        if (!a.accum_final || a.o == nullptr) *reinterpret_cast<float4*>(acc + col0 + i) = v4;
-                        orow[i] = __float_as_uint(v4.x);
-                        orow[i + 1] = __float_as_uint(v4.y);
-                        orow[i + 2] = __float_as_uint(v4.z);
-                        orow[i + 3] = __float_as_uint(v4.w);
-                    }
-                }
-                if (a.accum_final && a.o != nullptr) {
-                    if (a.o_is_fp32) {
-                        float* dst = static_cast<float*>(a.o) + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            if (col0 + i < a.head_dim)
-                                *reinterpret_cast<uint4*>(dst + col0 + i) = make_uint4(orow[i], orow[i + 1], orow[i + 2], orow[i + 3]);
-                    } else {
-                        uint16_t* dst = static_cast<uint16_t*>(a.o) + (unit_ll * a.seqlen_q + row) * a.head_dim;
-#pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            if (col0 + i < a.head_dim) {
-                                uint4 v4;
-                                v4.x = pack2<kBf16>(__uint_as_float(orow[i]), __uint_as_float(orow[i + 1]));
-                                v4.y = pack2<kBf16>(__uint_as_float(orow[i + 2]), __uint_as_float(orow[i + 3]));
-                                v4.z = pack2<kBf16>(__uint_as_float(orow[i + 4]), __uint_as_float(orow[i + 5]));
-                                v4.w = pack2<kBf16>(__uint_as_float(orow[i + 6]), __uint_as_float(orow[i + 7]));
-                                *reinterpret_cast<uint4*>(dst + col0 + i) = v4;
-                            }
-                        }
-                    }
-                }
-                continue;
-            }
             if (a.num_splits > 1 || a.o_is_fp32) {
                 float* dst = (a.num_splits > 1)
                                  ? a.o_partial + ((unit_ll * a.num_splits + split) * a.seqlen_q + row) * a.head_dim
@@ -1534,9 +1487,14 @@ cudaError_t launch_flags(const FwdArgs& a, const CUtensorMap& tq, const CUtensor
     if (a.staged)  // (never with dropout)
         return alibi ? launch_one<D, NQ, kBf16, true, false, true, false>(a, tq, tk, tv, to, tc, units, stream)
                      : launch_one<D, NQ, kBf16, false, false, true, false>(a, tq, tk, tv, to, tc, units, stream);
-    if (a.accum_o != nullptr && !dropout)
-        return alibi ? launch_one<D, NQ, kBf16, true, false, false, true>(a, tq, tk, tv, to, tc, units, stream)
-                     : launch_one<D, NQ, kBf16, false, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+    if (a.accum_o != nullptr) {
+        if (alibi) {
+            return dropout ? launch_one<D, NQ, kBf16, true, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
+                           : launch_one<D, NQ, kBf16, true, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+        }
+        return dropout ? launch_one<D, NQ, kBf16, false, true, false, true>(a, tq, tk, tv, to, tc, units, stream)
+                       : launch_one<D, NQ, kBf16, false, false, false, true>(a, tq, tk, tv, to, tc, units, stream);
+    }
     if (alibi) {
         return dropout ? launch_one<D, NQ, kBf16, true, true, false, false>(a, tq, tk, tv, to, tc, units, stream)
                        : launch_one<D, NQ, kBf16, true, false, false, false>(a, tq, tk, tv, to, tc, units, stream);

@@ -83,8 +83,8 @@ ClusterRoom cluster_room(int sms);  // of the current device; none above one CTA
 void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room, bool dropout);
 
 // Launchers implemented in the .cu files; all return a cudaError_t.  `to` is the store map of O, or of the running
-// result where the launch leaves that (32-row boxes); it is read only when a.o_tma or, without dropout, a.accum_o is set.  `tc` is
-// the load map of the running result, read only when that is so and something is carried.
+// result where the launch leaves that (32-row boxes); it is read only when a.o_tma or a.accum_o is set.  `tc` is the load
+// map of the running result, read only when a.accum_o is set and something is carried.
 cudaError_t launch_fwd_tiled(const FwdArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const CUtensorMap& to, const CUtensorMap& tc, int units, bool bf16, bool dropout, cudaStream_t stream);
 

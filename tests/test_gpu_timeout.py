@@ -138,7 +138,7 @@ def test_a_part_that_gave_up_leaves_no_plausible_row(test_lib, skip, H, Hk, Nq, 
     (160, 256, 128, 1, False, torch.bfloat16, 0.0),  # (two query tiles a CTA)
     (120, 300, 64, 0, True, torch.float32, 0.0),     # (a CTA whose second query tile does not exist; the first tile of the walk)
     (3, 300, 128, 1, False, torch.float32, 0.0),     # (one query tile a CTA, a ring of one stage)
-    (3, 300, 96, 1, False, torch.bfloat16, 0.1),     # (with dropout the rows are merged without TMA)
+    (3, 300, 96, 1, False, torch.bfloat16, 0.1),
 ])
 def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip, causal, out_dtype, p_dropout):
     """The block before it is complete, and so are the ones behind it: neither may make its rows look like a result."""
