@@ -5,7 +5,6 @@ compute entry points raises."""
 import ctypes
 import functools
 import os
-import struct
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libfa_b200.so")
@@ -45,29 +44,6 @@ class FwdParams(ctypes.Structure):
         ("accum_o", ctypes.c_void_p), ("accum_lse", ctypes.c_void_p), ("accum_flags", ctypes.c_int),
         ("launch_index", ctypes.c_uint64),
     ]
-
-
-# The same block packed in one call: the fields in order, in C's own sizes and alignment (the trailing 0Q rounds the
-# size up to the structure's alignment as C does).
-_PACK = struct.Struct("@5P7if3iPf3Qi2qPN2Pi2PiQ0Q")
-assert _PACK.size == ctypes.sizeof(FwdParams)
-
-
-def pack_params(*values):
-    """A FwdParams (by reference) with `values` in field order.  Values that a field cannot hold are converted as
-    ctypes converts them."""
-    try:
-        return _PACK.pack(*values)
-    except (struct.error, OverflowError):
-        return bytes(FwdParams(*values))
-
-
-class _ParamsArg:
-    """Argument type of a `const fa_fwd_params*`: a packed block or a reference to a FwdParams."""
-
-    @classmethod
-    def from_param(cls, x):
-        return ctypes.c_char_p.from_param(x) if type(x) is bytes else ctypes.POINTER(FwdParams).from_param(x)
 
 
 class FwdPlan(ctypes.Structure):
@@ -125,7 +101,7 @@ def load():
         raise ImportError(f"{LIB_PATH} is missing: build it with `python -m flash_attn_b200.build`; "
                           "there is no non-CUDA fallback")
     L = ctypes.CDLL(LIB_PATH)
-    pp = _ParamsArg
+    pp = ctypes.POINTER(FwdParams)
     L.fa_fwd.argtypes = [pp]
     L.fa_fwd.restype = ctypes.c_int
     L.fa_fwd_host.argtypes = [pp]

@@ -40,8 +40,9 @@ encode_tiled_fn get_encode_tiled() {
 // reference's hand-written zero padding (include/utils.h:67-114).
 int make_tensor_map(CUtensorMap* m, int dtype, const void* base, int d, long long rows, long long units,
                     int box_rows = kTile) {
-    // A tensor map is a pure function of these arguments, so the last few are kept per host thread:
-    // a caller that runs the same buffers again (every layer of every step) skips the driver call.
+    // A tensor map is a pure function of these arguments, so the last sixteen are kept per host thread: a caller that runs the same
+    // buffers again skips the driver call.  (A decode call has two, a tiled one three or four, a block of a running result five;
+    // replaced in turn, so a program that takes more buffers than that in turn encodes a map for each.)
     struct Entry {
         const void* base;
         long long rows, units;
@@ -424,14 +425,16 @@ int fa_fwd_plan(const fa_fwd_params* p, int num_sms, const int* clusters, fa_fwd
         plan->columns = d.columns;
         return FA_OK;
     }
-    if (p->p_dropout > 0.0f) {
-        plan->parts = splits;
-        return FA_OK;
+    const bool dropout = p->p_dropout > 0.0f;
+    if (!dropout) {
+        a.num_splits = 1;
+        a.tiles_per_split = a.tc;
     }
     a.o_dim = p->head_dim;
-    plan_tiled(&a, num_sms, room, false);
-    plan->parts = a.parts;
+    plan_tiled(&a, num_sms, room, dropout);
+    plan->parts = dropout ? splits : a.parts;
     plan->merged = a.parts > 1;
+    plan->columns = a.pair ? 2 * kTile : kTile;
     plan->staged = a.staged;
     plan->stacked_rows = a.pack_rows;
     return FA_OK;

@@ -1596,7 +1596,7 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
     }
     const int tile_rows = pair ? 2 * kTile : kTile;
     const double rows = std::min(1.0, 0.35 + 0.85 * std::min(a.seqlen_q, tile_rows) / tile_rows);  // (how full the blocks are)
-    const double stage = !staged ? 0.0 : a.pack_rows > 0 ? (c.merge + c.merge_each) * rows : 0.4;
+    const double stage = !staged ? 0.0 : a.pack_rows > 0 ? (c.merge + c.merge_each) * rows : 0.4;  // (stacked heads: see plan_tiled)
     Split best = {1, launch_us(c, static_cast<double>(std::min(blocks, slots)), sms, n) + stage, pair, least >= 0.8 * n || n - least <= 1};
     if (blocks > slots) {
         const double waves = static_cast<double>(blocks) / slots;
@@ -1623,7 +1623,8 @@ Split best_split(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged
 // ring of one stage.  us in two tiles / in one: [1,4,256,256,64] 5.94 / 4.81, [1,32,384,384,64] 7.99 / 6.98, [1,16,512,512,128]
 // 10.55 / 9.63, [1,32,512,512,128] 10.8 / 11.0 (128 CTAs of one tile), [1,64,512,512,128] 11.5 / 12.2 (256), but
 // [1,96,384,384,128] 17.2 / 10.6: 192 blocks of two tiles, of which 148 fit, against 288 tiles of which all fit.  The margins: under
-// a causal mask the model does not see that a pair's diagonal step has one tile only ([1,32,384,384,128] 8.7 / 9.0).  Over 300 random calls of up to 300 query tiles: 0.95 of two tiles always.
+// a causal mask the model does not see that a pair's diagonal step has one tile only ([1,32,384,384,128] 8.7 / 9.0).  Over 300 random calls of up to 300 query tiles: 0.95 of
+// two tiles always; over 40 padded ones (odd head dimensions, unsplit epilogue) 0.91 of the time before both.
 Split best_cut(const FwdArgs& a, int sms, const ClusterRoom& room, bool staged, int most_parts) {
     const Split one = best_split(a, sms, room, staged, most_parts, false);
     if (!two_tiles(a)) return one;
@@ -1697,9 +1698,10 @@ void plan_tiled(FwdArgs* a, int sms, const ClusterRoom& room, bool dropout) {
     // Grouped queries: the heads that share a K/V head are consecutive rows of Q, O and LSE, so they stack into one
     // unit of heads * seqlen_q rows without a copy: a remainder tile per unit instead of one per head.  Taken where the query
     // blocks are of about one length (tiles across heads have the longest: [4 x 12 heads on 2, 1940 rows, 1241 keys, causal]
-    // 72 us stacked, 50 not), it saves query tiles, and the model says 3 % and two microseconds of the time: a staged
-    // epilogue takes as long as a merge ([64 heads on 8, 720 rows, 25871 keys], 184 blocks instead of 192: 714 us against
-    // 699).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all of a head's positions; those past a
+    // 72 us stacked, 50 not), it saves query tiles, and the model says 3 % and two microseconds of the time, with a stacked
+    // launch charged what a merge costs, although an unsplit one has none: charged its epilogue's 0.4 us, heads were stacked where that
+    // loses ([13 x 16 heads on 4, 215 rows, 780 keys, causal] 34.6 us, 43.5 stacked, [16 x 28 on 4, 438 rows, 829 keys] 106 and
+    // 124, [64 heads on 8, 720 rows, 25871 keys], 184 blocks instead of 192, 699 and 714).  (ALiBi slopes go by head.  A tile across heads walks the KV tiles of all of a head's positions; those past a
     // row's own come first, and the row starts afresh behind them, but those before a left window would come last and bring
     // masked infinities and NaN with them: with one, only heads of a single tile are stacked, whose rows walked all of these
     // tiles anyway.)

@@ -1,7 +1,8 @@
 // The call path of flash_attn_forward on torch tensors: checks, output allocation, parameter block, stream and launch in
 // one native function.  Successor of the host side of the reference's main() (src/main.cu:109-205) for callers whose memory
 // torch owns.  A short call is bound by the host: [1,4,256,256,64] took 15.0 us a call through ctypes (two allocations through
-// Python 5, argument handling 5, the library 4) and takes 6.3, of which the kernel is 5.9; a decode step over 1000 keys 16.6 and 6.9.
+// Python 5, argument handling 5, the library 4) and takes 6.1, of which the kernel is 4.8; a decode step over 1000 keys 16.4 and 6.6, of
+// which the kernel is 5.1.  (On buffers seen before: a new one costs a tensor map each.)
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>

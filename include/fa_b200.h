@@ -149,7 +149,7 @@ typedef struct fa_fwd_plan_info {
     int decode;               /* 1: the kernel for seqlen_q <= 8, 0: the tiled kernel */
     int parts;                /* CTAs that share the keys of a query block (decode: of a unit) */
     int merged;               /* the parts are one cluster and merge on chip (0 with parts > 1: the combine kernel) */
-    int columns;              /* decode: query columns of a CTA */
+    int columns;              /* query rows of a CTA: decode 1, 4, 8 or 16 (columns of its tiles), else 128 or 256 */
     int staged;               /* tiled: finished rows leave through shared memory */
     int stacked_rows;         /* tiled: the heads of a K/V head are stacked into one unit, this many rows each; 0 = not */
 } fa_fwd_plan_info;

@@ -145,6 +145,7 @@ def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip,
     from flash_attn_b200 import _lib
     L = test_lib
     Nk = 500
+    assert plan(1, H, Nq, Nk, d, causal=causal, q_pos0=3 * Nk, p_dropout=p_dropout, num_splits=1, accum=True).columns == (128 if H == 3 else 256)
     qh, kh, vh = synth.qkv(42, 1, 3, Nq, 4 * Nk, d, "bfloat16")  # (the oracle's heads, again and again)
     q, k, v = (gpu_util.to_dev(x, "bfloat16")[:, torch.arange(H) % 3].contiguous() for x in (qh, kh, vh))
     acc = (torch.empty((1, H, Nq, d), device="cuda"), torch.empty((1, H, Nq), device="cuda"))
@@ -196,3 +197,41 @@ def test_a_block_that_gave_up_leaves_no_running_result(test_lib, H, Nq, d, skip,
         return
     assert np.abs(o[:, :3].float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
     assert np.abs(lse[:, :3].cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
+
+
+@pytest.mark.parametrize("H,Hk,Nq,Nk,d,causal", [
+    (4, 4, 300, 300, 31, False),     # padded rows
+    (300, 300, 200, 300, 31, False),  # ... in CTAs of two query tiles
+    (512, 64, 48, 546, 128, True),   # stacked heads
+])
+def test_an_unsplit_staged_launch_that_gave_up_leaves_no_plausible_row(test_lib, H, Hk, Nq, Nk, d, causal):
+    """Each warp finishes its own rows behind its own waits; those that ran out make them NaN."""
+    L = test_lib
+    got = plan(1, H, Nq, Nk, d, heads_k=Hk, causal=causal, q_pos0=Nk - Nq if causal else 0)
+    assert got.parts == 1 and got.staged and bool(got.stacked_rows) == (Hk < H)
+    qh, kh, vh = synth.qkv(43, 1, 4, Nq, Nk, d, "bfloat16")
+    q = gpu_util.to_dev(qh, "bfloat16")[:, torch.arange(H) % 4].contiguous()
+    k, v = (gpu_util.to_dev(x, "bfloat16")[:, torch.arange(Hk) % 4].contiguous() for x in (kh, vh))
+    o = torch.zeros_like(q)
+    lse = torch.zeros((1, H, Nq), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = _params(q, k, v, o, lse, status)
+    p.heads_k, p.num_splits, p.is_causal, p.q_pos0 = Hk, 0, int(causal), Nk - Nq if causal else 0
+    need = L.fa_fwd_workspace_bytes(ctypes.byref(p))
+    ws = torch.empty(max(need, 16), device="cuda", dtype=torch.uint8)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    try:
+        assert L.fa_test_skip_kv_tile(1) == 0
+        assert L.fa_fwd(ctypes.byref(p)) == 0
+        torch.cuda.synchronize()
+        assert 100 < int(status.item()) < 200
+        assert torch.isnan(o).all() and not torch.isfinite(lse).any()
+    finally:
+        assert L.fa_test_skip_kv_tile(-1) == 0
+    status.zero_()
+    assert L.fa_fwd(ctypes.byref(p)) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and torch.isfinite(o).all()
+    want_o, want_lse = oracle_lib.forward(qh[:, :1], kh[:, :1], vh[:, :1], d ** -0.5, causal=causal, q_pos0=Nk - Nq if causal else 0)
+    assert np.abs(o[:, :1].float().cpu().numpy() - want_o).max() <= gpu_util.O_MAX_ABS
+    assert np.abs(lse[:, :1].cpu().numpy() - want_lse).max() <= gpu_util.LSE_ABS
