@@ -104,11 +104,12 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units: rescale O only when th
 // everywhere (pair 0, the best before: [28 heads on 4, 849, 11656 keys] 151.6 us against 149.2, [1,32,2048,16384] 440.0 against
 // 433.9, [1,32,8192,128] causal 434.8 against 431.6); with dropout pairs 3 / 1 of even / odd groups on full tiles and none on masked
 // ones, which then need no guard (pairs 0 / 1 on all: [8,16,2048,128] causal, p = 0.1 144.5 us against 142.9, [2,16,1024,128] x 8192 keys
-// 117.3 against 116.7; of masked tiles with pairs 3 / 1 too 144.2).  The others as they were: pair 0, with dropout pairs 0 / 1 of
-// even / odd groups.
-__host__ __device__ constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, bool masked) {
+// 117.3 against 116.7; of masked tiles with pairs 3 / 1 too 144.2).  D = 64 pairs 0 / 3 of even / odd groups where not staged (before
+// them pair 0, with dropout 0 / 1: [3,32,3862,64] with ALiBi and a window 192.2 us against 190.3, [4,16,2048,64] causal, p = 0.1 63.4
+// against 63.1, [4,16,4096,64] causal 206.5 against 200.9).  The others as they were: pair 0, with dropout pairs 0 / 1.
+__host__ __device__ constexpr uint32_t poly_mask(int d, bool alibi, bool dropout, bool staged, bool masked) {
     if (d == 128 && !alibi) return dropout ? (masked ? 0u : 0x28u) : 0x88u;
-    return dropout ? 0x21u : 0x11u;
+    return d == 64 && !staged ? 0x81u : dropout ? 0x21u : 0x11u;
 }
 constexpr int kKeepChunk = 2;              // KV tiles whose dropout keep bits are handed over at a time (one Philox pass)
 constexpr int kKeepRing = 2 * kKeepChunk;  // tiles the keep-bit table holds
@@ -1060,7 +1061,7 @@ fwd_tiled_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             // elements are replaced by 0 (MUFU gives 0 by itself).
             auto exp_tile = [&](auto guard_tag) {
                 constexpr bool kGuard = decltype(guard_tag)::value;  // the tile has masked (-inf) scores
-                constexpr uint32_t kPolyMask = poly_mask(D, kAlibi, kDropout, kGuard);
+                constexpr uint32_t kPolyMask = poly_mask(D, kAlibi, kDropout, kStaged, kGuard);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {  // quarters of 32 columns
                     uint32_t pr[16];
